@@ -463,12 +463,12 @@ int wcg_batch_autotune(wcg_batch* b, const double* dt, const int* candidates, in
 
 /* Launch schedule of a context's pressure solve (no reference counterpart).
  * Performance only: every schedule gives bit-identical results.
- *   sweep_cluster    CTAs per thread-block cluster along c in the MIC(0)
- *                    sweeps: 0 chosen per solve from the patches along c
- *                    (the default), 1 plain, or 2, 3, 4, 8, 9, 16 (used when
- *                    the box has more than half that many patches along c);
- *   sweep_cluster_a  CTAs along a as well (2-D clusters): 1, 4 (with
- *                    sweep_cluster 1..4) or 8 (with sweep_cluster 1..2);
+ *   sweep_cluster    0 (the default), 1, 2, 3, 4, 8, 9 or 16, and
+ *   sweep_cluster_a  1, 4 (with sweep_cluster 1..4) or 8 (with sweep_cluster
+ *                    1..2): the extents of the thread-block clusters that
+ *                    the MIC(0) sweeps once ran in.  Accepted and returned;
+ *                    the sweeps run one CTA per patch, which is faster than
+ *                    every cluster shape was, whatever they say;
  *   pcg_batch        PCG iterations launched per convergence check on the
  *                    host (1..64; default 8). */
 typedef struct wcg_schedule {

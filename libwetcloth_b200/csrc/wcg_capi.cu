@@ -301,16 +301,13 @@ int wcg_create(const wcg_params* params, wcg_ctx** out) {
   // the PCG's SpMV: row-parallel (default) or patch-streamed (performance
   // knob; the dot products' partial sums are grouped differently)
   if (const char* v = getenv("WCG_SPMV")) ctx->c.spmv_rows = !strcmp(v, "stream") ? 0 : 1;
-  // CTAs per thread-block cluster along c in the MIC(0) sweeps (1, 2, 3, 4,
-  // 8, 9 or 16; performance knob, identical results).  Default 0: chosen per
-  // solve from the patches along c (pl_setup).
+  // cluster extents of the launch schedule (wcg_schedule): held for
+  // wcg_get_schedule, without effect on the sweeps
   ctx->c.sweep_cluster = 0;
   if (const char* v = getenv("WCG_SWEEP_CLUSTER")) {
     const int k = atoi(v);
     ctx->c.sweep_cluster = (k == 2 || k == 3 || k == 4 || k == 8 || k == 9 || k == 16) ? k : 1;
   }
-  // and along a: 2-D clusters of CC x CA CTAs (CA 4 or 8 with CC 1, 2 or 4;
-  // CA 8 with CC 1 or 2), a-face neighbours through shared memory as well
   if (const char* v = getenv("WCG_SWEEP_CLUSTER_A")) {
     const int k = atoi(v), cc = ctx->c.sweep_cluster;
     const bool ok = (k == 4 && cc <= 4) || (k == 8 && cc <= 2);

@@ -253,11 +253,10 @@ struct Context {
   DevBuf pl64;                   // kNumPl64Fields * pl_cap doubles
   DevBuf pl_edge;                // tagged edge words
   DevBuf pl_order;               // patches in wave order (int32)
-  DevBuf pl_corder;              // cluster columns in wave order (sweep_cluster > 1)
-  DevBuf pl_corder2;             // 2-D cluster tiles in wave order (sweep_cluster_a > 1)
-  int sweep_cluster = 1;         // CTAs per cluster along c in the MIC(0) sweeps
-  int sweep_cluster_a = 1;       // ... and along a (2-D clusters: 4 or 8)
-  int pl_cc = 1;                 // the c-extent the current solve uses (<= patches along c)
+  // cluster extents of the launch schedule, kept for wcg_get_schedule (the
+  // sweeps run one CTA per patch whatever they say)
+  int sweep_cluster = 1;
+  int sweep_cluster_a = 1;
   int spmv_rows = 1;             // 0: the patch-streamed SpMV instead of the row-parallel one
   int pcg_batch = 8;             // PCG iterations launched per host convergence check
   DevBuf pl_part;                // per-patch partials (double)
@@ -268,10 +267,6 @@ struct Context {
   TermSet term{};                // terminator shapes (the params' box, or wcg_set_terminators)
   int stale_patch = -1;          // failure-path test: a patch whose waits cannot succeed
   std::vector<int> pl_order_h;
-  // host copies of pl_corder / pl_corder2 and the (nPA, nPC, CC, CA) they
-  // were built for: re-uploaded only when that changes
-  std::vector<int> pl_corder_h, pl_corder2_h;
-  long long pl_corder_key = -1, pl_corder2_key = -1;
 
   // multigrid-PCG: dense levels (d, ax, ay, az, x, b per cell; masks) and the
   // level-0 PCG vectors

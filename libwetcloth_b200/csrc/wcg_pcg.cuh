@@ -488,10 +488,39 @@ __global__ void __launch_bounds__(kRedThreads)
 // (k_red_*) or the last block of the kernel that wrote the partials
 // (last_block).  Partials are summed thread-strided, then by the block tree,
 // so both forms give the same bits.
+// The tree of block_sum / block_max over kRedThreads values in shared memory,
+// for blocks of at least kRedThreads threads (the first kRedThreads add).
+template <typename T>
+__device__ inline T tree_sum(T* sm) {
+  __syncthreads();
+  for (int o = kRedThreads >> 1; o > 0; o >>= 1) {
+    if (threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
+    __syncthreads();
+  }
+  const T r = sm[0];
+  __syncthreads();
+  return r;
+}
+template <typename T>
+__device__ inline T tree_max(T* sm) {
+  __syncthreads();
+  for (int o = kRedThreads >> 1; o > 0; o >>= 1) {
+    if (threadIdx.x < o)
+      sm[threadIdx.x] = sm[threadIdx.x] > sm[threadIdx.x + o] ? sm[threadIdx.x] : sm[threadIdx.x + o];
+    __syncthreads();
+  }
+  const T r = sm[0];
+  __syncthreads();
+  return r;
+}
+
 __device__ inline void red_alpha_body(const double* partial, int n, double* sc, double* sm) {
-  double s = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s += __ldcg(partial + i);
-  s = block_sum<double>(s, sm);
+  if (threadIdx.x < kRedThreads) {
+    double s = 0;
+    for (int i = threadIdx.x; i < n; i += kRedThreads) s += __ldcg(partial + i);
+    sm[threadIdx.x] = s;
+  }
+  const double s = tree_sum(sm);
   if (threadIdx.x == 0) {
     sc[S_SQ] = s;
     sc[S_ALPHA] = sc[S_RHO] / s;
@@ -499,12 +528,15 @@ __device__ inline void red_alpha_body(const double* partial, int n, double* sc, 
 }
 
 __device__ inline void red_conv_body(const double* partial, int n, double* sc, double* sm) {
-  double m = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const double v = __ldcg(partial + i);
-    m = v > m ? v : m;
+  if (threadIdx.x < kRedThreads) {
+    double m = 0;
+    for (int i = threadIdx.x; i < n; i += kRedThreads) {
+      const double v = __ldcg(partial + i);
+      m = v > m ? v : m;
+    }
+    sm[threadIdx.x] = m;
   }
-  m = block_max<double>(m, sm);
+  const double m = tree_max(sm);
   if (threadIdx.x == 0) {
     sc[S_RES] = m;
     sc[S_ITER] += 1.0;
@@ -515,9 +547,12 @@ __device__ inline void red_conv_body(const double* partial, int n, double* sc, d
 
 __device__ inline void red_beta_body(const double* partial, int n, double* sc, double* sm,
                                      int init) {
-  double s = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s += __ldcg(partial + i);
-  s = block_sum<double>(s, sm);
+  if (threadIdx.x < kRedThreads) {
+    double s = 0;
+    for (int i = threadIdx.x; i < n; i += kRedThreads) s += __ldcg(partial + i);
+    sm[threadIdx.x] = s;
+  }
+  const double s = tree_sum(sm);
   if (threadIdx.x == 0) {
     if (init) {
       sc[S_BETA] = 0.0;

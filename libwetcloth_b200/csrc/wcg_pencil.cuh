@@ -14,14 +14,13 @@
 //   (s-1, a, c): row t-1 of the same line
 //   (s, a-1, c): row t-1 of line - 1
 //   (s, a, c-1): row t-1 of line - 16
-// so a CTA of 256 threads (one per line) walks its patch row by row, one
-// barrier per row, every load and store a coalesced row, rows prefetched kPre
-// ahead in registers.  The factor is stored interleaved per cell
-// {1/sqrt(d'), S_s, S_a, S_c} so a sweep reads it with one vector load.  Values
-// crossing a patch edge go through a global buffer of tagged 64-bit words,
-// (epoch << 32 | 32 data bits), one word per 32 bits of payload: the consumer
-// re-reads its word until the tag equals the launch's epoch, so no fence or
-// flag is needed and a patch waits only for the rows it reads.
+// so a CTA takes a patch, one warp per strip of 32 lines, and every strip walks
+// its rows with contiguous loads and stores.  The factor is stored interleaved
+// per cell {1/sqrt(d'), S_s, S_a, S_c} so a sweep reads it with one vector load.
+// Values crossing a patch edge go through a global buffer of tagged 64-bit
+// words, (epoch << 32 | 32 data bits), one word per 32 bits of payload: the
+// consumer re-reads its word until the tag equals the launch's epoch, so no
+// fence or flag is needed and a patch waits only for the rows it reads.
 // Patches are handed out by an atomic ticket in wave order (PAi + PCi), so a
 // patch's upstream patches always started before it.
 //
@@ -44,8 +43,7 @@
 namespace wcg {
 
 constexpr int kPatch = 16;                    // lines per patch edge
-constexpr int kPatchLines = kPatch * kPatch;  // threads of a sweep CTA
-constexpr int kPre = 4;                       // rows of edge words prefetched ahead
+constexpr int kPatchLines = kPatch * kPatch;
 constexpr int kPlBlocks = 592;                // streaming kernels: 4 x 148 SMs
 // the fused SpMV in FP32 (32 registers): 8 resident CTAs per SM, so twice the
 // loads in flight of the other streaming kernels
@@ -92,129 +90,31 @@ struct TagWords<double> {
   }
 };
 
-// ---- bulk row copies into shared memory (cp.async.bulk + mbarrier) ---------
 __device__ inline unsigned smem_u32(const void* p) {
   return (unsigned)__cvta_generic_to_shared(p);
 }
-__device__ inline void mbar_init(unsigned bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ inline void mbar_expect_tx(unsigned bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-__device__ inline bool mbar_try_wait(unsigned bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// global -> shared, 16-byte aligned addresses, bytes a multiple of 16
-__device__ inline void bulk_g2s(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-      "l"(src), "r"(bytes), "r"(bar)
-      : "memory");
-}
-__device__ inline unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-constexpr unsigned long long kWaitNs = 2000000000ull;  // bound of an mbarrier wait (2 s)
 
-// ---- thread-block clusters: distributed shared memory -----------------------
-__device__ inline unsigned cluster_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// every thread of every CTA of the cluster; release/acquire orders the shared
-// memory each CTA wrote before it against the reads after it
-__device__ inline void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n"
-               "barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// address of the same shared variable in CTA `rank` of the cluster
-__device__ inline unsigned cluster_map(unsigned local, unsigned rank) {
-  unsigned r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
-  return r;
-}
-__device__ inline unsigned ld_cluster_u32(unsigned addr) {
-  unsigned v;
-  asm volatile("ld.relaxed.cluster.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-  return v;
-}
-__device__ inline void st_cluster_u64(unsigned addr, u64 v) {
-  asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
-}
-// a word of this CTA's shared memory that peers of the cluster write
-__device__ inline u64 ld_own_u64(unsigned addr) {
-  u64 v;
-  asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
-  return v;
-}
+// Values a strip stages per cell: factor A_d, A_s, A_a, A_c; forward r, q (with
+// the update), coef x4; backward y, r, coef x4.
+__host__ __device__ constexpr int sweep_slot(int mode) { return mode == 0 ? 4 : 6; }
 
-// Stages of the shared-memory row ring of a sweep.
-template <typename R>
-struct SweepStages {
-  static constexpr int D = sizeof(R) == 4 ? 8 : 6;
-};
-// Arrays staged per row: factor A_d, A_s, A_a, A_c; forward r, coef x4 (, q);
-// backward y, coef x4, r.
-__host__ __device__ constexpr int sweep_nf(int mode, bool upd) {
-  return mode == 0 ? 4 : (mode == 1 ? (upd ? 6 : 5) : 6);
-}
-template <typename R>
-__host__ __device__ constexpr size_t sweep_dyn_smem(int mode, bool upd) {
-  return (size_t)SweepStages<R>::D * sweep_nf(mode, upd) * 256 * sizeof(R) +
-         (size_t)SweepStages<R>::D * 8;
-}
-// With clusters the c-face edge words of the patch upstream in the same
-// cluster land in this CTA's shared memory: Ls x 16 entries, 16-byte aligned
-// after the ring and its mbarriers.
-template <typename R>
-__host__ __device__ constexpr size_t sweep_cedge_off(int mode, bool upd) {
-  return (sweep_dyn_smem<R>(mode, upd) + 15) / 16 * 16;
-}
-template <typename R>
-__host__ __device__ constexpr size_t sweep_cedge_bytes(int mode, int Ls) {
-  return (size_t)Ls * 16 * (mode == 0 ? 2 : 1) * (sizeof(R) / 4) * 8;
-}
-// dynamic shared memory of a cluster sweep: the ring, then the edge words of
-// the clustered faces
-template <typename R>
-__host__ __device__ constexpr size_t sweep_cluster_smem(int mode, bool upd, int Ls, int cc,
-                                                        int ca) {
-  return sweep_cedge_off<R>(mode, upd) + (cc > 1 ? sweep_cedge_bytes<R>(mode, Ls) : 0) +
-         (ca > 1 ? sweep_cedge_bytes<R>(mode, Ls) : 0);
-}
-// the a-face words of a 2-D cluster, after the c-face ones (when present)
-template <typename R>
-__host__ __device__ constexpr size_t sweep_aedge_off(int mode, bool upd, int Ls, bool cfaces) {
-  return sweep_cedge_off<R>(mode, upd) + (cfaces ? sweep_cedge_bytes<R>(mode, Ls) : 0);
-}
-
-// Words of the edge buffer: entry (producer patch, side, s, k), EW words each.
-// side 0: the a-face (k = cl), side 1: the c-face (k = al).
-__device__ inline long long edge_word(const PencilGeom& G, long long p, int side, int s, int k,
+// Words of the edge buffer: entry (patch that writes, face, row, line), EW
+// words each.  face 0: towards the next patch along a (line k = cl), face 1:
+// along c (line k = al); row = the row of the strip that takes the word.
+__host__ __device__ inline long long edge_rows(const PencilGeom& G) { return G.Ls + 15; }
+__device__ inline long long edge_word(const PencilGeom& G, long long p, int face, int row, int k,
                                       int EW) {
-  return (((p * 2 + side) * G.Ls + s) * kPatch + k) * EW;
+  return (((p * 2 + face) * edge_rows(G) + row) * kPatch + k) * EW;
 }
 
 // The MIC(0) factor of a cell, interleaved: {1/sqrt(d'), S_s, S_a, S_c}.
-__device__ inline void ld_coef(const float* p, float* c) {
-  const float4 t = __ldcs(reinterpret_cast<const float4*>(p));
+__device__ inline void ld_coef_shared(const float* p, float* c) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
   c[0] = t.x; c[1] = t.y; c[2] = t.z; c[3] = t.w;
 }
-__device__ inline void ld_coef(const double* p, double* c) {
-  const double2 a = __ldcs(reinterpret_cast<const double2*>(p));
-  const double2 b = __ldcs(reinterpret_cast<const double2*>(p) + 1);
+__device__ inline void ld_coef_shared(const double* p, double* c) {
+  const double2 a = reinterpret_cast<const double2*>(p)[0];
+  const double2 b = reinterpret_cast<const double2*>(p)[1];
   c[0] = a.x; c[1] = a.y; c[2] = b.x; c[3] = b.y;
 }
 __device__ inline void st_coef(float* p, float a, float b, float c, float d) {
@@ -261,448 +161,499 @@ struct PencilSweepArgs {
 // r -= alpha q (and reports max|r|); the matching x += alpha s is applied by
 // the next SpMV (k_pl_spmv_s) or, after the last iteration, by k_pl_axpy.
 //
-// One thread per line, tid = al + 16 cl, warp w holding cl = 2w and 2w + 1;
-// the CTA advances one row per step with one barrier.  The a-neighbour and the
-// c-neighbour inside the warp come by shuffle of the previous step's outputs,
-// the c-neighbour in the adjacent warp through shared memory, and values across
-// the patch faces through the tagged edge words.
+// A patch is one CTA of 8 strip warps and 2 receiver warps.  Strip w holds the
+// 32 lines cl = 2w and 2w + 1 (lane = al + 16 (cl & 1)) and walks its own rows
+// v = 0 .. Ls + 15 (row t = v + 2w of the patch) without any CTA barrier:
+//   * its row data is copied D rows ahead into a shared-memory ring that only
+//     this warp uses (cp.async, 16 bytes per lane);
+//   * the a-neighbour and the c-neighbour inside the strip come by shuffle of
+//     the previous row's outputs;
+//   * the c-neighbour in strip w - 1 and the values from the patches upstream
+//     along a and c come as tagged 64-bit words (tag << 32 | 32 data bits) in
+//     the strip's inbox in shared memory.  Strip w - 1 writes the c words of
+//     row v - 1 of its own count; the receivers write the rest.
+// Words across a patch face go through a global buffer (tag: the launch's
+// epoch).  The receivers (one warp for the a-face, one for the c-face, two
+// lanes per line: even and odd rows) poll it, up to 8 rows per lane in flight,
+// and move what has arrived into the inboxes, so a strip never waits for a
+// round trip to L2 of its own.  An inbox slot is reused once the strip has
+// published that it took the word (s_prog).  Every wait is bounded.
 //
-// CL > 1: launched in clusters of CL CTAs along c.  The patches of a cluster
-// are one cluster column of CL consecutive c-patches; a c-face neighbour in
-// the same cluster writes its tagged words straight into this CTA's shared
-// memory (st.shared::cluster), which takes the global round trip off those
-// hops.  Tickets are handed out per cluster in wave order, so every upstream
-// cluster started earlier.  The cluster syncs after the edge buffers are
-// cleared and before any CTA exits, so no CTA writes into a peer that has not
-// started or has already left.
+// The backward sweep is the same walk mirrored: patches, strips, lanes and
+// rows counted from the other end.
 //
-// CA > 1 as well: clusters of CC x CA CTAs, a tile of CC c-patches by CA
-// a-patches (rank = ra + CA rc); a-face neighbours inside the tile exchange
-// through shared memory the same way (their words after the c-face ones).
+// Bound: the chain of Ls + NA + NC rows that the last cell waits for, then the
+// bytes of a row (forward 8, backward 7 values per cell).  The former CTA of
+// one warp per two lines of c, all eight meeting at a barrier in every row and
+// every face lane polling its own word in L2, took per launch 426 us at 256^3
+// in FP32 (in clusters of 9 along c) where this takes 270; in FP64 287 / 161 us
+// for the half box at 128^3, 105 / 62 us for the dam break at 64^3, 62 / 39 us
+// at 16^3 (all with the events around each launch).
 //
 // The body takes the launch's CTA count (nblocks) as an argument so a launch
 // over several solves (k_pencil_sweep_batch) can run it per solve.
-template <typename R, int MODE, bool UPD, int CC, int CA>
+constexpr int kStrips = kPatchLines / 32;
+constexpr int kPencilThreads = kPatchLines + 64;  // strips, then two receiver warps
+constexpr int kInC = 16;   // inbox rows of c words (16 per row)
+constexpr int kInA = 32;   // inbox rows of a words (2 per row)
+constexpr int kRecv = 8;   // rows a receiver lane polls at once
+constexpr long long kInboxPolls = 1ll << 24;  // bound of a wait in shared memory
+
+template <typename R>
+struct SweepStages {
+  static constexpr int D = sizeof(R) == 4 ? 16 : 8;
+};
+__host__ __device__ constexpr int sweep_words(int mode, size_t rbytes) {
+  return (mode == 0 ? 2 : 1) * (int)(rbytes / 4);  // 64-bit words per edge entry
+}
+template <typename R>
+__host__ __device__ constexpr size_t sweep_ring_bytes(int mode) {
+  return (size_t)kStrips * SweepStages<R>::D * sweep_slot(mode) * 32 * sizeof(R);
+}
+template <typename R>
+__host__ __device__ constexpr size_t sweep_dyn_smem(int mode) {
+  return sweep_ring_bytes<R>(mode) +
+         (size_t)kStrips * (kInC * 16 + kInA * 2) * sweep_words(mode, sizeof(R)) * 8;
+}
+
+__device__ inline void cp_async16(unsigned dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ inline void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ inline void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+// EW tagged words of one entry (each 64-bit word is read and written whole and
+// carries its own tag)
+template <int EW>
+__device__ inline void ld_words_shared(unsigned addr, u64* w) {
+  if (EW == 1) {
+    asm volatile("ld.volatile.shared.u64 %0, [%1];" : "=l"(w[0]) : "r"(addr) : "memory");
+  } else {
+#pragma unroll
+    for (int k = 0; k < EW; k += 2)
+      asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];"
+                   : "=l"(w[k]), "=l"(w[k + 1])
+                   : "r"(addr + 8 * k)
+                   : "memory");
+  }
+}
+template <int EW>
+__device__ inline void st_words_shared(unsigned addr, const u64* w) {
+  if (EW == 1) {
+    asm volatile("st.volatile.shared.u64 [%0], %1;" ::"r"(addr), "l"(w[0]) : "memory");
+  } else {
+#pragma unroll
+    for (int k = 0; k < EW; k += 2)
+      asm volatile("st.volatile.shared.v2.u64 [%0], {%1, %2};" ::"r"(addr + 8 * k), "l"(w[k]),
+                   "l"(w[k + 1])
+                   : "memory");
+  }
+}
+template <int EW>
+__device__ inline bool words_tagged(const u64* w, unsigned tag) {
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < EW; ++k) ok = ok && (unsigned)(w[k] >> 32) == tag;
+  return ok;
+}
+__device__ inline int ld_volatile_int(unsigned addr) {
+  int v;
+  asm volatile("ld.volatile.shared.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ inline void st_volatile_int(unsigned addr, int v) {
+  asm volatile("st.volatile.shared.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
+template <typename R, int MODE, bool UPD>
 __device__ __forceinline__ void pencil_sweep_run(const PencilSweepArgs<R>& A, int nblocks) {
-  constexpr int CL = CC * CA;
   constexpr bool BWD = MODE == kBackward;
   constexpr int PW = MODE == kFactor ? 2 : 1;  // values sent across an edge
   constexpr int TW = TagWords<R>::W;
   constexpr int EW = PW * TW;
-  // prefetched per cell: factor A_d, A_s, A_a, A_c; forward in, coef[4] (, q);
-  // backward in, coef[4], r
-  constexpr int NF = sweep_nf(MODE, UPD);
   static_assert(kFactor == 0 && kForward == 1 && kBackward == 2, "mode numbering");
-  constexpr int RS = BWD ? -kPatchLines : kPatchLines;  // element step per row
-  constexpr int NW = kPatchLines / 32;
-  constexpr int D = SweepStages<R>::D;             // rows in flight
-  constexpr int SLOT = NF * kPatchLines;            // Reals per staged row
+  constexpr int D = SweepStages<R>::D;
+  constexpr int NF = sweep_slot(MODE);
+  constexpr bool TWO = MODE == kBackward || UPD;  // two vectors per row
+  constexpr int SLOT = NF * 32;                   // Reals per staged strip row
+  constexpr unsigned full = 0xffffffffu;
   __shared__ int s_ticket;
-  __shared__ R xc[2][NW][kPatch][PW];
+  __shared__ int s_prog[kStrips];
   __shared__ double red[kPatchLines];
-  extern __shared__ __align__(128) unsigned char dsm[];  // D slots, then D mbarriers
-  R* const ring = reinterpret_cast<R*>(dsm);
-  const unsigned bar0 = smem_u32(dsm + (size_t)D * SLOT * sizeof(R));
+  extern __shared__ __align__(128) unsigned char dsm[];  // strip rings, then the inboxes
   const PencilGeom& G = A.G;
   const int tid = threadIdx.x;
   const int lane = tid & 31, w = tid >> 5;
-  // one ticket per patch (per cluster with CL > 1), taken even by a launch
-  // that returns at once, so the counter stays in step with the host's base
-  const int crank = CL > 1 ? (int)cluster_rank() : 0;
-  if (tid == 0 && crank == 0) s_ticket = atomicAdd(A.ticket, 1) - A.ticket_base;
-  // set by an earlier launch, so uniform: the whole cluster returns before
-  // any cross-CTA access
-  if (*(const int*)(A.sc + S_DONE)) return;
-  for (int i = tid; i < 2 * NW * kPatch * PW; i += kPatchLines) (&xc[0][0][0][0])[i] = R(0);
-  u64* const cedge = CC > 1 ? reinterpret_cast<u64*>(dsm + sweep_cedge_off<R>(MODE, UPD)) : nullptr;
-  u64* const aedge =
-      CA > 1 ? reinterpret_cast<u64*>(dsm + sweep_aedge_off<R>(MODE, UPD, G.Ls, CC > 1)) : nullptr;
-  if (CC > 1)
-    for (int i = tid; i < G.Ls * kPatch * EW; i += kPatchLines) cedge[i] = 0ull;
-  if (CA > 1)
-    for (int i = tid; i < G.Ls * kPatch * EW; i += kPatchLines) aedge[i] = 0ull;
-  if (CL > 1)
-    cluster_sync();
-  else
-    __syncthreads();
-  const int tk = CL > 1 ? (int)ld_cluster_u32(cluster_map(smem_u32(&s_ticket), 0)) : s_ticket;
-  const int nTA = (G.nPA + CA - 1) / CA;
-  const int nunits = CL > 1 ? nTA * ((G.nPC + CC - 1) / CC) : (int)G.npatch;
-  const int ra = crank % CA, rc = crank / CA;
+  // one ticket per patch, taken even by a launch that returns at once, so the
+  // counter stays in step with the host's base
+  if (tid == 0) s_ticket = atomicAdd(A.ticket, 1) - A.ticket_base;
+  if (*(const int*)(A.sc + S_DONE)) return;  // set by an earlier launch: uniform
+  constexpr int INBOX = (kInC * 16 + kInA * 2) * EW;  // words per strip
+  {
+    u64* ib = reinterpret_cast<u64*>(dsm + sweep_ring_bytes<R>(MODE));
+    for (int i = tid; i < kStrips * INBOX; i += kPencilThreads) ib[i] = 0ull;
+    if (tid < kStrips) s_prog[tid] = 0;
+  }
+  __syncthreads();
+  const int tk = s_ticket;
   bool run = true;
-  if (tk < 0 || tk >= nunits) {
+  if (tk < 0 || tk >= (int)G.npatch) {
     if (tid == 0) record_error(A.err, kErrIndex);
     run = false;
   }
-  int p = 0, PAi = 0, PCi = 0;
+  double rmax = 0, dsum = 0;
+  int p = 0;
   if (run) {
-    const int unit = BWD ? A.order[nunits - 1 - tk] : A.order[tk];
-    PAi = CL > 1 ? (unit % nTA) * CA + ra : unit % G.nPA;
-    PCi = CL > 1 ? (unit / nTA) * CC + rc : unit / G.nPA;
-    run = PCi < G.nPC && PAi < G.nPA;  // the last tiles may reach past the box
-    p = PCi * G.nPA + PAi;
-  }
-  if (run) {
-  const int al = tid & (kPatch - 1), cl = tid / kPatch;
-  const bool line = PAi * kPatch + al < G.NA && PCi * kPatch + cl < G.NC;
-  const int dl = al + cl;
-  const int Ls = G.Ls, NR = G.R;
-  const int u0 = BWD ? (NR - Ls) - dl : dl;  // first live step
-  int up_a = -1, up_c = -1;
-  bool pub_a, pub_c;
-  if (!BWD) {
-    if (al == 0 && PAi > 0) up_a = p - 1;
-    if (cl == 0 && PCi > 0) up_c = p - G.nPA;
-    pub_a = al == kPatch - 1 && PAi + 1 < G.nPA;
-    pub_c = cl == kPatch - 1 && PCi + 1 < G.nPC;
-  } else {
-    if (al == kPatch - 1 && PAi + 1 < G.nPA) up_a = p + 1;
-    if (cl == kPatch - 1 && PCi + 1 < G.nPC) up_c = p + G.nPA;
-    pub_a = al == 0 && PAi > 0;
-    pub_c = cl == 0 && PCi > 0;
-  }
-  if (!line) up_a = up_c = -1;
-  // c-face neighbours in the same cluster exchange through shared memory
-  const bool c_loc = CC > 1 && up_c >= 0 && (BWD ? rc < CC - 1 : rc > 0);
-  const bool c_rem = CC > 1 && pub_c && (BWD ? rc > 0 : rc < CC - 1);
-  const bool a_loc = CA > 1 && up_a >= 0 && (BWD ? ra < CA - 1 : ra > 0);
-  const bool a_rem = CA > 1 && pub_a && (BWD ? ra > 0 : ra < CA - 1);
-  if (c_loc) up_c = -1;
-  if (c_rem) pub_c = false;
-  if (a_loc) up_a = -1;
-  if (a_rem) pub_a = false;
-  const unsigned cedge_own = CC > 1 ? smem_u32(cedge) : 0u;
-  const unsigned cedge_dst = c_rem ? cluster_map(cedge_own, BWD ? crank - CA : crank + CA) : 0u;
-  const unsigned aedge_own = CA > 1 ? smem_u32(aedge) : 0u;
-  const unsigned aedge_dst = a_rem ? cluster_map(aedge_own, BWD ? crank - 1 : crank + 1) : 0u;
-  const bool a_edge = al == (BWD ? kPatch - 1 : 0);  // no in-warp a source
-  const bool c_prod = BWD ? lane < 16 : lane >= 16;  // half read by the next warp
-  const int w_src = BWD ? w + 1 : w - 1;
-  const bool has_wsrc = BWD ? w + 1 < NW : w > 0;
-  constexpr int ES = kPatch * EW;  // words between consecutive s of one entry
-  const u64* ea_src = up_a >= 0 ? A.edge + edge_word(G, up_a, 0, 0, cl, EW) : nullptr;
-  const u64* ec_src = up_c >= 0 ? A.edge + edge_word(G, up_c, 1, 0, al, EW) : nullptr;
-  u64* ea_dst = pub_a ? A.edge + edge_word(G, p, 0, 0, cl, EW) : nullptr;
-  u64* ec_dst = pub_c ? A.edge + edge_word(G, p, 1, 0, al, EW) : nullptr;
-  const unsigned ep = A.epoch;
-  // the tag this patch waits for: the launch's, except on the patch a
-  // failure-path test marks, whose waits then run into their limit
-  const unsigned ep_want = p == A.stale_patch ? (ep ^ 0x80000000u) : ep;
-  const long long spin_limit = A.spin_limit;
-  const R al_r = (MODE == kForward && UPD) ? (R)A.sc[S_ALPHA] : R(0);
-  const R omega = A.omega, min_ratio = A.min_ratio;
-  // per-thread base pointers (patch and line applied); rows by 32-bit offset
-  const long long pb = (long long)p * NR * kPatchLines + tid;
-  R* __restrict__ pcoef = A.coef + 4 * pb;
-  R* __restrict__ o_out = MODE == kFactor ? nullptr : A.out + pb;
-  R* __restrict__ o_r = (MODE == kForward && UPD) ? A.r + pb : nullptr;
-  const int off0 = BWD ? (NR - 1) * kPatchLines : 0;
-  auto s_at = [&](int u) { return BWD ? (NR - 1 - u) - dl : u - dl; };
-  auto live_at = [&](int u) { return line && (unsigned)(u - u0) < (unsigned)Ls; };
-  // Rows outside a line's range hold zeros, so whole rows are staged and every
-  // cell is computed (zeros stay zeros); only the edge words need liveness.
-  // Thread 0 copies whole rows (one bulk copy per array) D rows ahead into a
-  // ring slot; the slot layout is [first array][coef x4 or A_s, A_a, A_c][q/r].
-  const long long pbase = (long long)p * NR * kPatchLines;
-  auto issue = [&](int u) {
-    const int j = u % D;
-    const unsigned bar = bar0 + 8 * j;
-    const unsigned dst = smem_u32(ring + (size_t)j * SLOT);
-    const long long rb = pbase + (long long)(BWD ? NR - 1 - u : u) * kPatchLines;
-    constexpr unsigned RB = kPatchLines * sizeof(R);
-    mbar_expect_tx(bar, NF * RB);
-    if (MODE == kFactor) {
-      bulk_g2s(dst, A.AD + rb, RB, bar);
-      bulk_g2s(dst + RB, A.AS + rb, RB, bar);
-      bulk_g2s(dst + 2 * RB, A.AA + rb, RB, bar);
-      bulk_g2s(dst + 3 * RB, A.AC + rb, RB, bar);
+    p = BWD ? A.order[(int)G.npatch - 1 - tk] : A.order[tk];
+    const int PAi = p % G.nPA, PCi = p / G.nPA;
+    const int Ls = G.Ls;
+    const int NV = Ls + kPatch;            // rows of a strip
+    const int na = Ls + 1, nc = Ls + 15;   // rows that take a-face and c-face words
+    // patches upstream (their words come in) and downstream
+    const int up_a = BWD ? (PAi + 1 < G.nPA ? p + 1 : -1) : (PAi > 0 ? p - 1 : -1);
+    const int up_c = BWD ? (PCi + 1 < G.nPC ? p + G.nPA : -1) : (PCi > 0 ? p - G.nPA : -1);
+    const bool pub_a = BWD ? PAi > 0 : PAi + 1 < G.nPA;
+    const bool pub_c = BWD ? PCi > 0 : PCi + 1 < G.nPC;
+    const unsigned inbox0 = smem_u32(dsm + sweep_ring_bytes<R>(MODE));
+    const unsigned prog0 = smem_u32(s_prog);
+    const unsigned ep = A.epoch;
+    if (w >= kStrips) {
+      // ---- receivers ----
+      const bool cface = w == kStrips + 1;
+      const int up = cface ? up_c : up_a;
+      if (up >= 0) {
+        // the tag this patch waits for: the launch's, except on the patch a
+        // failure-path test marks, whose waits then run into their limit
+        const unsigned want = p == A.stale_patch ? (ep ^ 0x80000000u) : ep;
+        const int k = lane & 15;                     // line of the face
+        const int strip = cface ? 0 : k >> 1;
+        const int rows = cface ? nc : na;
+        const unsigned box = inbox0 + (unsigned)(strip * INBOX) * 8u +
+                             (cface ? (unsigned)(k * EW) * 8u
+                                    : (unsigned)((kInC * 16 + (k & 1)) * EW) * 8u);
+        const int depth = cface ? kInC : kInA;
+        const unsigned pitch = (cface ? 16u : 2u) * EW * 8u;
+        const unsigned prog = prog0 + 4u * strip;
+        const u64* src = A.edge + edge_word(G, up, cface ? 1 : 0, 0, k, EW);
+        int v = lane >> 4;  // this lane's next row; rows of one parity
+        long long idle = 0;
+        bool gave_up = false;
+        while (__any_sync(full, v < rows)) {
+          const int room = ld_volatile_int(prog) + depth;  // rows below it may be written
+          // a lane that saw nothing new polls one row, else kRecv rows
+          const int most = idle > 0 ? 1 : kRecv;
+          u64 wd[kRecv][EW];
+          bool mine[kRecv];
+#pragma unroll
+          for (int j = 0; j < kRecv; ++j) {
+            const int vj = v + 2 * j;
+            mine[j] = j < most && vj < rows && vj < room;
+            if (mine[j]) {
+#pragma unroll
+              for (int q = 0; q < EW; ++q)
+                wd[j][q] = ld_relaxed_u64(src + (long long)vj * (16 * EW) + q);
+            }
+          }
+          int got = 0;
+          bool open = true;
+#pragma unroll
+          for (int j = 0; j < kRecv; ++j) {
+            const int vj = v + 2 * j;
+            if (mine[j] && gave_up) {
+#pragma unroll
+              for (int q = 0; q < EW; ++q) wd[j][q] = (u64)want << 32;
+            }
+            open = open && mine[j] && words_tagged<EW>(wd[j], want);
+            if (open) {
+              u64 o[EW];
+#pragma unroll
+              for (int q = 0; q < EW; ++q)
+                o[q] = ((u64)(unsigned)(vj + 1) << 32) | (wd[j][q] & 0xffffffffull);
+              st_words_shared<EW>(box + (unsigned)(vj & (depth - 1)) * pitch, o);
+              got = j + 1;
+            }
+          }
+          v += 2 * got;
+          if (got > 0) {
+            idle = 0;
+          } else if (v < rows && v < room) {
+            if (++idle > A.spin_limit && !gave_up) {
+              record_error(A.err, kErrWaitTimeout);
+              gave_up = true;
+            }
+          } else if (v < rows && ++idle > kInboxPolls) {
+            // the strip no longer takes words (its own wait gave up)
+            record_error(A.err, kErrWaitTimeout);
+            v = rows;
+          }
+        }
+      }
     } else {
-      bulk_g2s(dst, A.in + rb, RB, bar);
-      bulk_g2s(dst + RB, A.coef + 4 * rb, 4 * RB, bar);
-      if (NF == 6) bulk_g2s(dst + 5 * RB, (MODE == kForward ? A.q : A.r) + rb, RB, bar);
-    }
-  };
-  bool gave_up = false;
-  auto mwait = [&](int u) {
-    const unsigned bar = bar0 + 8 * (u % D);
-    const unsigned par = (unsigned)(u / D) & 1u;
-    if (mbar_try_wait(bar, par)) return;
-    const unsigned long long t0 = global_ns();
-    while (!mbar_try_wait(bar, par)) {
-      if (gave_up || global_ns() - t0 > kWaitNs) {
-        if (!gave_up) record_error(A.err, kErrWaitTimeout);
-        gave_up = true;
-        return;
-      }
-    }
-  };
-  if (tid == 0) {
-    for (int j = 0; j < D; ++j) mbar_init(bar0 + 8 * j, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
-  __syncthreads();
-  if (tid == 0)
-    for (int u = 0; u < D && u < NR; ++u) issue(u);
-
-  u64 epa[kPre][EW], epc[kPre][EW];
+      // ---- strips ----
+      // mirrored for the backward sweep: strip w walks the physical strip 7 - w
+      // and lane l the physical lane 31 - l, rows from the end
+      const int pl = BWD ? 31 - lane : lane;
+      const int ps = BWD ? kStrips - 1 - w : w;
+      const long long pbase = (long long)p * G.R * kPatchLines + 32 * ps;
+      const int t0 = BWD ? G.R - 1 - 2 * w : 2 * w;
+      constexpr int RS = BWD ? -kPatchLines : kPatchLines;  // element step per row
+      const long long row0 = pbase + (long long)t0 * kPatchLines;
+      R* const ring = reinterpret_cast<R*>(dsm) + (size_t)w * D * SLOT;
+      const unsigned ring0 = smem_u32(ring);
+      // copies of one row: 16 bytes per lane and pass
+      constexpr int RW = 32 * sizeof(R);  // bytes of one strip row
+      constexpr int PR = RW / 16;         // lanes that copy one array's row
+      auto issue = [&](int v) {
+        if (v < NV) {
+          const long long e = row0 + (long long)v * RS;
+          const unsigned dst = ring0 + (unsigned)(v & (D - 1)) * (SLOT * (unsigned)sizeof(R));
+          if (MODE == kFactor) {
+            const R* a4[4] = {A.AD, A.AS, A.AA, A.AC};
 #pragma unroll
-  for (int v = 0; v < kPre; ++v) {
-    const bool lv = v < NR && live_at(v);
-    const int sv = s_at(v);
-#pragma unroll
-    for (int k = 0; k < EW; ++k) {
-      epa[v][k] = (lv && ea_src) ? ld_relaxed_u64(ea_src + sv * ES + k) : 0ull;
-      epc[v][k] = (lv && ec_src) ? ld_relaxed_u64(ec_src + sv * ES + k) : 0ull;
-    }
-  }
-  R carry[PW], prev_a[PW], prev_c[PW];
-#pragma unroll
-  for (int k = 0; k < PW; ++k) carry[k] = prev_a[k] = prev_c[k] = R(0);
-  R rmax = 0;
-  double dsum = 0;
-  // complete an edge entry: re-read words whose tag is stale (bounded)
-  auto ewait = [&](u64* wd, const u64* src) {
-#pragma unroll
-    for (int k = 0; k < EW; ++k) {
-      if ((unsigned)(wd[k] >> 32) == ep_want) continue;
-      long long it = 0;
-      do {
-        if (gave_up || ++it > spin_limit) {
-          if (!gave_up) record_error(A.err, kErrWaitTimeout);
-          gave_up = true;
-          wd[k] = (u64)ep << 32;
-          break;
-        }
-        wd[k] = ld_relaxed_u64(src + k);
-      } while ((unsigned)(wd[k] >> 32) != ep_want);
-    }
-  };
-
-  for (int ub = 0; ub < NR; ub += kPre) {
-#pragma unroll
-    for (int v = 0; v < kPre; ++v) {
-      const int u = ub + v;
-      if (u >= NR) break;  // uniform over the CTA
-      const int off = off0 + u * RS;
-      const int cur = u & 1, nxt = cur ^ 1;
-      // neighbour inputs of step u = outputs of step u - 1
-      R in_a[PW], in_c[PW];
-#pragma unroll
-      for (int k = 0; k < PW; ++k) {
-        in_a[k] = BWD ? __shfl_down_sync(0xffffffffu, prev_a[k], 1)
-                      : __shfl_up_sync(0xffffffffu, prev_a[k], 1);
-        in_c[k] = BWD ? __shfl_down_sync(0xffffffffu, prev_c[k], 16)
-                      : __shfl_up_sync(0xffffffffu, prev_c[k], 16);
-        if (a_edge) in_a[k] = R(0);
-        if (!c_prod) in_c[k] = has_wsrc ? xc[cur][w_src][al][k] : R(0);
-      }
-      const bool live = live_at(u);
-      const int s = s_at(u);
-      if (live && ea_src) {
-        ewait(epa[v], ea_src + s * ES);
-#pragma unroll
-        for (int k = 0; k < PW; ++k) in_a[k] = TagWords<R>::unpack(epa[v] + k * TW);
-      }
-      if (live && ec_src) {
-        ewait(epc[v], ec_src + s * ES);
-#pragma unroll
-        for (int k = 0; k < PW; ++k) in_c[k] = TagWords<R>::unpack(epc[v] + k * TW);
-      }
-      if (CA > 1 && live && a_loc) {
-        u64 wd[EW];
-        const unsigned a0 = aedge_own + (unsigned)((s * kPatch + cl) * EW) * 8u;
-#pragma unroll
-        for (int k = 0; k < EW; ++k) {
-          wd[k] = ld_own_u64(a0 + 8u * k);
-          long long it = 0;
-          while ((unsigned)(wd[k] >> 32) != ep_want) {
-            if (gave_up || ++it > spin_limit) {
-              if (!gave_up) record_error(A.err, kErrWaitTimeout);
-              gave_up = true;
-              break;
+            for (int i = 0; i < 4 * PR / 32; ++i) {
+              const int c = lane + 32 * i;
+              const int arr = c / PR, off = c % PR;
+              const R* s = arr == 0 ? a4[0] : (arr == 1 ? a4[1] : (arr == 2 ? a4[2] : a4[3]));
+              cp_async16(dst + arr * RW + off * 16,
+                         reinterpret_cast<const unsigned char*>(s + e) + off * 16);
             }
-            wd[k] = ld_own_u64(a0 + 8u * k);
+          } else {
+            // the vectors (one or two rows), then the factor (four rows' worth)
+            const R* v1 = MODE == kForward ? A.q : A.r;
+            if (lane < (TWO ? 2 : 1) * PR) {
+              const R* s = lane < PR ? A.in : v1;
+              const int off = lane % PR;
+              cp_async16(dst + (lane / PR) * RW + off * 16,
+                         reinterpret_cast<const unsigned char*>(s + e) + off * 16);
+            }
+#pragma unroll
+            for (int i = 0; i < PR * 4 / 32; ++i)
+              cp_async16(dst + 2 * RW + (lane + 32 * i) * 16,
+                         reinterpret_cast<const unsigned char*>(A.coef + 4 * e) +
+                             (lane + 32 * i) * 16);
           }
         }
+        cp_async_commit();
+      };
+      for (int j = 0; j < D; ++j) issue(j);
+
+      // the words this lane takes: lanes 0..15 the c-face, 16 and 17 the
+      // a-face lines 2w and 2w + 1
+      const bool has_c = w > 0 || up_c >= 0, has_a = up_a >= 0;
+      const int vlim = lane < 16 ? (has_c ? nc : 0) : (lane < 18 && has_a ? na : 0);
+      const unsigned box = inbox0 + (unsigned)(w * INBOX) * 8u;
+      const unsigned wsrc =
+          lane < 16 ? box + (unsigned)(lane * EW) * 8u
+                    : box + (unsigned)((kInC * 16 + (lane & 1)) * EW) * 8u;
+      const int wmask = lane < 16 ? kInC - 1 : kInA - 1;
+      const unsigned wpitch = (lane < 16 ? 16u : 2u) * EW * 8u;
+      // outgoing: lanes 16..31 the c words of row v - 1 of the next strip (or
+      // of the patch downstream), lanes 15 and 31 the a-face words of row v - 15
+      const bool to_box = w + 1 < kStrips;
+      const bool put_c = lane >= 16 && (to_box || pub_c);
+      const bool put_a = (lane & 15) == 15 && pub_a;
+      const unsigned obox = inbox0 + (unsigned)((w + 1) * INBOX) * 8u +
+                            (unsigned)((lane & 15) * EW) * 8u;
+      u64* const gc = A.edge + edge_word(G, p, 1, 0, lane & 15, EW);
+      u64* const ga = A.edge + edge_word(G, p, 0, 0, 2 * w + (lane >> 4), EW);
+      const unsigned prog = prog0 + 4u * w;
+      const R al_r = (MODE == kForward && UPD) ? (R)A.sc[S_ALPHA] : R(0);
+      const R omega = A.omega, min_ratio = A.min_ratio;
+      const long long eb = row0 + pl;
+      R* const pcoef = MODE == kFactor ? A.coef + 4 * eb : nullptr;
+      R* const o_out = MODE == kFactor ? nullptr : A.out + eb;
+      R* const o_r = (MODE == kForward && UPD) ? A.r + eb : nullptr;
+      R carry[PW], prev_a[PW], prev_c[PW], f[NF];
 #pragma unroll
-        for (int k = 0; k < PW; ++k) in_a[k] = TagWords<R>::unpack(wd + k * TW);
-      }
-      if (CC > 1 && live && c_loc) {
-        u64 wd[EW];
-        const unsigned a0 = cedge_own + (unsigned)((s * kPatch + al) * EW) * 8u;
-#pragma unroll
-        for (int k = 0; k < EW; ++k) {
-          wd[k] = ld_own_u64(a0 + 8u * k);
-          long long it = 0;
-          while ((unsigned)(wd[k] >> 32) != ep_want) {
-            if (gave_up || ++it > spin_limit) {
-              if (!gave_up) record_error(A.err, kErrWaitTimeout);
-              gave_up = true;
-              break;
-            }
-            wd[k] = ld_own_u64(a0 + 8u * k);
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < PW; ++k) in_c[k] = TagWords<R>::unpack(wd + k * TW);
-      }
-      // this row's inputs from the ring
-      R f[NF];
-      mwait(u);
-      {
-        const R* S = ring + (size_t)(u % D) * SLOT;
-        f[0] = S[tid];
+      for (int k = 0; k < PW; ++k) carry[k] = prev_a[k] = prev_c[k] = R(0);
+      R rm = 0;
+      bool gave_up = false;
+      u64 wd[EW];
+      auto load_row = [&](int v) {
+        const R* S = ring + (size_t)(v & (D - 1)) * SLOT;
         if (MODE == kFactor) {
-          f[1] = S[kPatchLines + tid];
-          f[2] = S[2 * kPatchLines + tid];
-          f[3] = S[3 * kPatchLines + tid];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) f[k] = S[32 * k + pl];
         } else {
-          const R* cf = S + kPatchLines + 4 * tid;
-          f[1] = cf[0]; f[2] = cf[1]; f[3] = cf[2]; f[4] = cf[3];
-          if (NF == 6) f[5] = S[5 * kPatchLines + tid];
+          f[0] = S[pl];
+          if (TWO) f[NF - 1] = S[32 + pl];
+          ld_coef_shared(S + 64 + 4 * pl, f + 1);
         }
-      }
-      R out_s[PW], out_a[PW], out_c[PW];
-      if (MODE == kFactor) {
-        const R ad = f[0];
-        R d = ad;
-        R iv = R(0);
-        if (ad != R(0)) {
-          d = d - in_c[0] * in_c[0];
-          d = d - (omega * in_c[0]) * in_c[1];
-          d = d - in_a[0] * in_a[0];
-          d = d - (omega * in_a[0]) * in_a[1];
-          d = d - carry[0] * carry[0];
-          d = d - (omega * carry[0]) * carry[1];
-          const R piv = d < min_ratio * ad ? ad : d;
-          iv = R(1) / sqrt(piv);
+      };
+      cp_async_wait<D - 1>();
+      __syncwarp();
+      load_row(0);
+      ld_words_shared<EW>(wsrc, wd);
+      int room = kInC;  // rows the next strip's inbox can take
+#pragma unroll 2
+      for (int v = 0; v < NV; ++v) {
+        // this row's incoming words
+        {
+          const bool need = v < vlim;
+          const unsigned tag = (unsigned)(v + 1);
+          bool ok = !need || words_tagged<EW>(wd, tag);
+          if (!__all_sync(full, ok)) {
+            long long it = 0;
+            while (!__all_sync(full, ok) && !gave_up) {
+              if (!ok) {
+                ld_words_shared<EW>(wsrc + (unsigned)(v & wmask) * wpitch, wd);
+                ok = words_tagged<EW>(wd, tag);
+              }
+              if (++it > kInboxPolls) {
+                if (lane == 0) record_error(A.err, kErrWaitTimeout);
+                gave_up = true;
+              }
+            }
+          }
         }
-        const R ss = f[1] * iv, sa = f[2] * iv, scv = f[3] * iv;
-        st_coef(pcoef + 4 * off, iv, ss, sa, scv);
-        out_s[0] = ss; out_s[1] = sa + scv;
-        out_a[0] = sa; out_a[1] = ss + scv;
-        out_c[0] = scv; out_c[1] = ss + sa;
-      } else if (MODE == kForward) {
-        R rv = f[0];
-        if (UPD) {
-          rv = rv - al_r * f[5];
-          o_r[off] = rv;
-          const R av = fabs(rv);
-          rmax = av > rmax ? av : rmax;
+        R in_a[PW], in_c[PW];
+        {
+          R word[PW];
+#pragma unroll
+          for (int k = 0; k < PW; ++k) {
+            word[k] = v < vlim ? TagWords<R>::unpack(wd + k * TW) : R(0);
+            const R wa = __shfl_sync(full, word[k], 16 + (lane >> 4));
+            const R sa = __shfl_up_sync(full, prev_a[k], 1);
+            const R sc = __shfl_up_sync(full, prev_c[k], 16);
+            in_a[k] = (lane & 15) == 0 ? wa : sa;
+            in_c[k] = lane < 16 ? word[k] : sc;
+          }
         }
-        R vv = rv;
-        vv -= in_c[0];
-        vv -= in_a[0];
-        vv -= carry[0];
-        const R y = vv * f[1];
-        o_out[off] = y;
-        out_s[0] = f[2] * y;
-        out_a[0] = f[3] * y;
-        out_c[0] = f[4] * y;
-      } else {
-        R vv = f[0];
-        vv -= f[2] * carry[0];
-        vv -= f[3] * in_a[0];
-        vv -= f[4] * in_c[0];
-        const R z = vv * f[1];
-        o_out[off] = z;
-        dsum += (double)z * (double)f[5];
-        out_s[0] = out_a[0] = out_c[0] = z;
-      }
-      if (live && ea_dst) {
-        u64 wd[EW];
-#pragma unroll
-        for (int k = 0; k < PW; ++k) TagWords<R>::pack(out_a[k], ep, wd + k * TW);
-#pragma unroll
-        for (int k = 0; k < EW; ++k) st_relaxed_u64(ea_dst + s * ES + k, wd[k]);
-      }
-      if (live && ec_dst) {
-        u64 wd[EW];
-#pragma unroll
-        for (int k = 0; k < PW; ++k) TagWords<R>::pack(out_c[k], ep, wd + k * TW);
-#pragma unroll
-        for (int k = 0; k < EW; ++k) st_relaxed_u64(ec_dst + s * ES + k, wd[k]);
-      }
-      if (CC > 1 && live && c_rem) {
-        u64 wd[EW];
-#pragma unroll
-        for (int k = 0; k < PW; ++k) TagWords<R>::pack(out_c[k], ep, wd + k * TW);
-        const unsigned a0 = cedge_dst + (unsigned)((s * kPatch + al) * EW) * 8u;
-#pragma unroll
-        for (int k = 0; k < EW; ++k) st_cluster_u64(a0 + 8u * k, wd[k]);
-      }
-      if (CA > 1 && live && a_rem) {
-        u64 wd[EW];
-#pragma unroll
-        for (int k = 0; k < PW; ++k) TagWords<R>::pack(out_a[k], ep, wd + k * TW);
-        const unsigned a0 = aedge_dst + (unsigned)((s * kPatch + cl) * EW) * 8u;
-#pragma unroll
-        for (int k = 0; k < EW; ++k) st_cluster_u64(a0 + 8u * k, wd[k]);
-      }
-#pragma unroll
-      for (int k = 0; k < PW; ++k) {
-        if (c_prod) xc[nxt][w][al][k] = out_c[k];
-        prev_a[k] = out_a[k];
-        prev_c[k] = out_c[k];
-        carry[k] = out_s[k];
-      }
-      // edge words of step u + kPre
-      {
-        const int un = u + kPre;
-        const bool lv = un < NR && live_at(un);
-        const int sn = s_at(un);
-#pragma unroll
-        for (int k = 0; k < EW; ++k) {
-          if (lv && ea_src) epa[v][k] = ld_relaxed_u64(ea_src + sn * ES + k);
-          if (lv && ec_src) epc[v][k] = ld_relaxed_u64(ec_src + sn * ES + k);
+        // the next row's words, read early; taken once their tag is right
+        ld_words_shared<EW>(wsrc + (unsigned)((v + 1) & wmask) * wpitch, wd);
+        if ((v & 3) == 3 && lane == 0) st_volatile_int(prog, v + 1);
+        const long long off = (long long)v * RS;
+        R out_s[PW], out_a[PW], out_c[PW];
+        if (MODE == kFactor) {
+          const R ad = f[0];
+          R d = ad;
+          R iv = R(0);
+          if (ad != R(0)) {
+            d = d - in_c[0] * in_c[0];
+            d = d - (omega * in_c[0]) * in_c[PW - 1];
+            d = d - in_a[0] * in_a[0];
+            d = d - (omega * in_a[0]) * in_a[PW - 1];
+            d = d - carry[0] * carry[0];
+            d = d - (omega * carry[0]) * carry[PW - 1];
+            const R piv = d < min_ratio * ad ? ad : d;
+            iv = R(1) / sqrt(piv);
+          }
+          const R ss = f[1] * iv, sa = f[2] * iv, scv = f[3] * iv;
+          st_coef(pcoef + 4 * off, iv, ss, sa, scv);
+          out_s[0] = ss; out_s[PW - 1] = sa + scv;
+          out_a[0] = sa; out_a[PW - 1] = ss + scv;
+          out_c[0] = scv; out_c[PW - 1] = ss + sa;
+        } else if (MODE == kForward) {
+          R rv = f[0];
+          if (UPD) {
+            rv = rv - al_r * f[NF - 1];
+            o_r[off] = rv;
+            const R av = fabs(rv);
+            rm = av > rm ? av : rm;
+          }
+          R vv = rv;
+          vv -= in_c[0];
+          vv -= in_a[0];
+          vv -= carry[0];
+          const R y = vv * f[1];
+          o_out[off] = y;
+          out_s[0] = f[2] * y;
+          out_a[0] = f[3] * y;
+          out_c[0] = f[NF - 2] * y;
+        } else {
+          R vv = f[0];
+          vv -= f[2] * carry[0];
+          vv -= f[3] * in_a[0];
+          vv -= f[NF - 2] * in_c[0];
+          const R z = vv * f[1];
+          o_out[off] = z;
+          dsum += (double)z * (double)f[NF - 1];
+          out_s[0] = out_a[0] = out_c[0] = z;
         }
+        // c words of row v - 1 downstream
+        if (to_box) {
+          if (v >= room + 1) {
+            // the next strip has to take a row first
+            long long it = 0;
+            const unsigned np = prog0 + 4u * (w + 1);
+            do {
+              room = ld_volatile_int(np) + kInC;
+              if (++it > kInboxPolls) {
+                if (lane == 0) record_error(A.err, kErrWaitTimeout);
+                gave_up = true;
+                room = 1 << 30;
+              }
+            } while (v >= room + 1);
+          }
+          if (put_c && v > 0) {
+            u64 o[EW];
+#pragma unroll
+            for (int k = 0; k < PW; ++k) TagWords<R>::pack(out_c[k], (unsigned)v, o + k * TW);
+            st_words_shared<EW>(obox + (unsigned)((v - 1) & (kInC - 1)) * (16u * EW * 8u), o);
+          }
+        } else if (put_c && v > 0) {
+          u64 o[EW];
+#pragma unroll
+          for (int k = 0; k < PW; ++k) TagWords<R>::pack(out_c[k], ep, o + k * TW);
+#pragma unroll
+          for (int k = 0; k < EW; ++k)
+            st_relaxed_u64(gc + (long long)(v - 1) * (16 * EW) + k, o[k]);
+        }
+        if (put_a && v >= kPatch - 1) {
+          u64 o[EW];
+#pragma unroll
+          for (int k = 0; k < PW; ++k) TagWords<R>::pack(out_a[k], ep, o + k * TW);
+#pragma unroll
+          for (int k = 0; k < EW; ++k)
+            st_relaxed_u64(ga + (long long)(v - (kPatch - 1)) * (16 * EW) + k, o[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < PW; ++k) {
+          prev_a[k] = out_a[k];
+          prev_c[k] = out_c[k];
+          carry[k] = out_s[k];
+        }
+        // every lane has read row v (the shuffles above follow its loads), so
+        // its slot takes row v + D
+        __syncwarp();
+        issue(v + D);
+        cp_async_wait<D - 1>();
+        __syncwarp();
+        if (v + 1 < NV) load_row(v + 1);
       }
-      // Every thread passed row u - 1's barrier, so slot (u - 1) % D is free:
-      // refill it with row u - 1 + D, before this row's barrier, from a lane
-      // that waits on no c-face edge word in this direction.  (Refills
-      // issued by thread 0 after each row's barrier -- of slot u % D, or of
-      // slot (u - 1) % D -- gave solves that differed from run to run at 256
-      // patches; this order repeats bit for bit.)
-      if (tid == (BWD ? 31 : kPatchLines - 1) && u >= 1 && u - 1 + D < NR) issue(u - 1 + D);
-      __syncthreads();
+      if (lane == 0) st_volatile_int(prog, 1 << 29);  // nothing waits for this strip any more
+      cp_async_wait<0>();
+      rmax = (double)rm;
     }
   }
-  if (gave_up) {
-    // a wait gave up: give the copies still in flight into the ring time to
-    // land (bounded) before the CTA exits
-    for (int u = NR - D > 0 ? NR - D : 0; u < NR; ++u) {
-      const unsigned bar = bar0 + 8 * (u % D);
-      const unsigned par = (unsigned)(u / D) & 1u;
-      const unsigned long long t0 = global_ns();
-      while (!mbar_try_wait(bar, par) && global_ns() - t0 < kWaitNs) {
-      }
+  // partials, summed in line order whatever the direction
+  if (A.part && ((MODE == kForward && UPD) || MODE == kBackward)) {
+    const int line = BWD ? kPatchLines - 1 - tid : tid;
+    if (tid < kPatchLines) red[line] = MODE == kForward ? rmax : dsum;
+    __syncthreads();
+    if (MODE == kForward) {
+      const double m = tree_max(red);
+      if (tid == 0 && run) A.part[p] = m;
+    } else {
+      const double sm = tree_sum(red);
+      if (tid == 0 && run) A.part[p] = sm;
+    }
+    // every CTA counts, running or not; the last one reduces the partials
+    if (A.done_ctr && last_block(A.done_ctr, nblocks)) {
+      if (MODE == kForward)
+        red_conv_body(A.part, A.npart, A.sc, red);
+      else
+        red_beta_body(A.part, A.npart, A.sc, red, A.red_init);
     }
   }
-  if (MODE == kForward && UPD && A.part) {
-    const double m = block_max<double>((double)rmax, red);
-    if (tid == 0) A.part[p] = m;
-  }
-  if (MODE == kBackward && A.part) {
-    const double sm = block_sum<double>(dsum, red);
-    if (tid == 0) A.part[p] = sm;
-  }
-  }  // run
-  // every CTA counts, running or not; the last one reduces the partials
-  if (A.done_ctr && A.part && ((MODE == kForward && UPD) || MODE == kBackward) &&
-      last_block(A.done_ctr, nblocks)) {
-    if (MODE == kForward)
-      red_conv_body(A.part, A.npart, A.sc, red);
-    else
-      red_beta_body(A.part, A.npart, A.sc, red, A.red_init);
-  }
-  if (CL > 1) cluster_sync();
 }
 
-template <typename R, int MODE, bool UPD, int CC, int CA>
-__global__ void __launch_bounds__(kPatchLines, 1)
+template <typename R, int MODE, bool UPD>
+__global__ void __launch_bounds__(kPencilThreads, 1)
     k_pencil_sweep(const PencilSweepArgs<R> A) {
-  pencil_sweep_run<R, MODE, UPD, CC, CA>(A, (int)gridDim.x);
+  pencil_sweep_run<R, MODE, UPD>(A, (int)gridDim.x);
 }
 
 // The solve of block b in a launch over several solves: first[] holds each
@@ -719,12 +670,12 @@ __device__ inline int batch_solve_of(const int* __restrict__ first, int n, int b
 }
 
 // One sweep launch over several solves (the shared solve of a batch of
-// scenes): solve s owns first[s + 1] - first[s] CTAs (its patches, plain
-// form) and its arguments come from tab[s].  Launch k of a chunk advances
-// each solve's edge-word epoch by k and its ticket base by k launches of its
-// patches, as k separate launches would.
+// scenes): solve s owns first[s + 1] - first[s] CTAs (its patches) and its
+// arguments come from tab[s].  Launch k of a chunk advances each solve's
+// edge-word epoch by k and its ticket base by k launches of its patches, as k
+// separate launches would.
 template <typename R, int MODE, bool UPD>
-__global__ void __launch_bounds__(kPatchLines, 1)
+__global__ void __launch_bounds__(kPencilThreads, 1)
     k_pencil_sweep_batch(const PencilSweepArgs<R>* __restrict__ tab, const int* __restrict__ first,
                          int nsolve, int k) {
   const int s = batch_solve_of(first, nsolve, (int)blockIdx.x);
@@ -732,7 +683,7 @@ __global__ void __launch_bounds__(kPatchLines, 1)
   const int nb = __ldg(first + s + 1) - __ldg(first + s);
   A.epoch += (unsigned)k;
   A.ticket_base += k * nb;
-  pencil_sweep_run<R, MODE, UPD, 1, 1>(A, nb);
+  pencil_sweep_run<R, MODE, UPD>(A, nb);
 }
 
 // x += alpha s (the update of the last PCG iteration, which no SpMV follows)

@@ -85,8 +85,7 @@ void ctx_free(Context& c) {
                     &c.gfield, &c.gvalid, &c.gdof, &c.wave_list, &c.wave_count,
                     &c.tile_flag, &c.tile_active, &c.tile_part, &c.active_list, &c.p2g_halo,
                     &c.rx64, &c.rr64, &c.rb64,
-                    &c.pl, &c.pl64, &c.pl_edge, &c.pl_order, &c.pl_corder, &c.pl_corder2,
-                    &c.pl_part,
+                    &c.pl, &c.pl64, &c.pl_edge, &c.pl_order, &c.pl_part,
                     &c.mg, &c.mg_mask, &c.mg_vec,
                     &c.adj, &c.adjp, &c.adjmask, &c.adjstage, &c.adjvisc, &c.adjxc, &c.adjam,
                     &c.visc, &c.viscflag, &c.dstage, &c.ustage,
@@ -1291,8 +1290,9 @@ static cudaError_t pl_setup(Context& c, const int* lo, const int* hi) {
     WCG_TRY(c.pl.ensure((size_t)kNumPlFields * G.len * sizeof(R)));
     if (c.prm.precision != 0) WCG_TRY(c.pl64.ensure((size_t)kNumPl64Fields * G.len * sizeof(double)));
   }
-  // edge words: 2 faces x Ls x 16 entries x (2 values x words per value)
-  const size_t edge_bytes = (size_t)G.npatch * 2 * G.Ls * kPatch * 2 * (sizeof(R) / 4) * 8;
+  // edge words: 2 faces x rows x 16 entries x (2 values x words per value)
+  const size_t edge_bytes =
+      (size_t)G.npatch * 2 * edge_rows(G) * kPatch * 2 * (sizeof(R) / 4) * 8;
   if (edge_bytes > c.pl_edge.bytes) {
     WCG_TRY(c.pl_edge.ensure(edge_bytes));
     // tags of a fresh buffer must not match any epoch (epochs start at 1)
@@ -1312,65 +1312,6 @@ static cudaError_t pl_setup(Context& c, const int* lo, const int* hi) {
     WCG_TRY(c.pl_order.ensure((size_t)G.npatch * sizeof(int)));
     WCG_TRY(cudaMemcpyAsync(c.pl_order.p, c.pl_order_h.data(), G.npatch * sizeof(int),
                             cudaMemcpyHostToDevice, c.stream));
-  }
-  // The cluster's extent along c.  Chosen (sweep_cluster 0): a cluster that
-  // tiles the patches along c exactly, so no CTA idles, at most 9 CTAs in
-  // FP32 (two CTAs per SM fit) and 3 in FP64 (one per SM).  At 256^3 (9
-  // patches along c, ms per sweep launch): FP32 plain 0.461, 3 0.436, 8
-  // 0.423, 9 0.415, 16 0.521; FP64 plain 0.594, 3 0.550, 8 0.721, 9 0.638.
-  // On small boxes they cost more than they save (the 64^3 dam break, 2
-  // patches along c: 7.4 ms per step in 2-CTA clusters, 7.0 ms plain).
-  // Given: used where the box has more patches along c than half a cluster.
-  if (c.sweep_cluster == 0) {
-    c.pl_cc = 1;
-    const int fp32[] = {9, 8}, fp64[] = {3};
-    const int* cand = c.prm.precision != 0 ? fp32 : fp64;
-    const int ncand = c.prm.precision != 0 ? 2 : 1;
-    if (G.nPC >= 6)
-      for (int k = 0; k < ncand; ++k)
-        if (G.nPC % cand[k] == 0) {
-          c.pl_cc = cand[k];
-          break;
-        }
-    if (c.pl_cc == 1 && c.prm.precision != 0 && G.nPC >= 6) c.pl_cc = 8;
-  } else {
-    c.pl_cc = G.nPC > c.sweep_cluster / 2 ? c.sweep_cluster : 1;
-  }
-  // the cluster orders are rebuilt only when the patch grid or the cluster
-  // shape changes (a pageable upload waits for the stream)
-  const long long okey = ((long long)G.nPA << 40) | ((long long)G.nPC << 16) |
-                         ((long long)c.pl_cc << 8) | c.sweep_cluster_a;
-  if (c.sweep_cluster_a > 1 && okey != c.pl_corder2_key) {
-    // tiles of pl_cc c-patches by sweep_cluster_a a-patches, in wave order
-    const int CC = c.pl_cc, CA = c.sweep_cluster_a;
-    const int nTA = (G.nPA + CA - 1) / CA, nTC = (G.nPC + CC - 1) / CC;
-    std::vector<int>& co = c.pl_corder2_h;
-    co.clear();
-    for (int w = 0; w <= nTA + nTC - 2; ++w)
-      for (int tc = 0; tc < nTC; ++tc) {
-        const int ta = w - tc;
-        if (ta >= 0 && ta < nTA) co.push_back(tc * nTA + ta);
-      }
-    WCG_TRY(c.pl_corder2.ensure(co.size() * sizeof(int)));
-    WCG_TRY(cudaMemcpyAsync(c.pl_corder2.p, co.data(), co.size() * sizeof(int),
-                            cudaMemcpyHostToDevice, c.stream));
-    c.pl_corder2_key = okey;
-  }
-  if (c.pl_cc > 1 && okey != c.pl_corder_key) {
-    // cluster columns (PAi, PCc) of pl_cc c-patches, in wave order
-    const int CL = c.pl_cc;
-    const int nPCc = (G.nPC + CL - 1) / CL;
-    std::vector<int>& co = c.pl_corder_h;
-    co.clear();
-    for (int w = 0; w <= G.nPA + nPCc - 2; ++w)
-      for (int pc = 0; pc < nPCc; ++pc) {
-        const int pa = w - pc;
-        if (pa >= 0 && pa < G.nPA) co.push_back(pc * G.nPA + pa);
-      }
-    WCG_TRY(c.pl_corder.ensure(co.size() * sizeof(int)));
-    WCG_TRY(cudaMemcpyAsync(c.pl_corder.p, co.data(), co.size() * sizeof(int),
-                            cudaMemcpyHostToDevice, c.stream));
-    c.pl_corder_key = okey;
   }
   // every array starts at zero (rows and lines outside the box stay zero)
   WCG_TRY(cudaMemsetAsync(c.pl.p, 0, (size_t)kNumPlFields * G.len * sizeof(R), c.stream));
@@ -1407,81 +1348,26 @@ static PencilSweepArgs<R> pl_args(Context& c) {
   return a;
 }
 
-// dynamic shared memory a cluster sweep may use (the kernel's static
-// arrays take under 8 KB of the 227 KB per CTA)
-constexpr size_t kSweepSmemMax = 216 * 1024;
-
-template <typename R, int MODE, bool UPD, int CC, int CA>
-static cudaError_t pl_sweep_cl(Context& c, PencilSweepArgs<R> a) {
-  constexpr int CL = CC * CA;
+template <typename R, int MODE, bool UPD>
+static cudaError_t pl_sweep(Context& c, PencilSweepArgs<R> a) {
   ProfScope prof(c, MODE == kFactor ? P_MICFACTOR : P_MICSWEEP);
   const PencilGeom& G = c.plg;
-  const int nTA = (G.nPA + CA - 1) / CA, nTC = (G.nPC + CC - 1) / CC;
-  const int nunits = CL > 1 ? nTA * nTC : (int)G.npatch;
   a.epoch = (unsigned)(++c.tile_epoch);
   a.ticket_base = c.pl_tickets;
-  c.pl_tickets += nunits;
-  const size_t smem = CL > 1 ? sweep_cluster_smem<R>(MODE, UPD, G.Ls, CC, CA)
-                             : sweep_dyn_smem<R>(MODE, UPD);
+  c.pl_tickets += (int)G.npatch;
+  constexpr size_t smem = sweep_dyn_smem<R>(MODE);
   // function attributes are per device: set once per instantiation and
   // device (the batch may step contexts of several devices from several
   // threads; setting them twice is harmless)
   static std::atomic<unsigned long long> attr_set{0};
   const unsigned long long dbit = 1ull << (c.device & 63);
   if (!(attr_set.load(std::memory_order_acquire) & dbit)) {
-    WCG_TRY(cudaFuncSetAttribute(k_pencil_sweep<R, MODE, UPD, CC, CA>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(CL > 1 ? kSweepSmemMax : smem)));
-    if (CL > 8)
-      WCG_TRY(cudaFuncSetAttribute(k_pencil_sweep<R, MODE, UPD, CC, CA>,
-                                   cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    WCG_TRY(cudaFuncSetAttribute(k_pencil_sweep<R, MODE, UPD>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set.fetch_or(dbit, std::memory_order_release);
   }
-  if (CL == 1) {
-    ++c.launches, k_pencil_sweep<R, MODE, UPD, 1, 1><<<(unsigned)G.npatch, kPatchLines, smem,
-                                                       c.stream>>>(a);
-    return cudaGetLastError();
-  }
-  a.order = CA > 1 ? c.pl_corder2.as<int>() : c.pl_corder.as<int>();
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(nunits * CL));
-  cfg.blockDim = dim3(kPatchLines);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = c.stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = CL;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  ++c.launches;
-  return cudaLaunchKernelEx(&cfg, k_pencil_sweep<R, MODE, UPD, CC, CA>, a);
-}
-
-// The cluster forms need the edge buffers of a patch (Ls x 16 tagged entries
-// per clustered face) in shared memory; when they do not fit, a 2-D cluster
-// falls back to its c-clusters and those to the plain form.
-template <typename R, int MODE, bool UPD>
-static cudaError_t pl_sweep(Context& c, PencilSweepArgs<R> a) {
-  const int CC = c.pl_cc, CA = c.sweep_cluster_a;
-  const int Ls = c.plg.Ls;
-  if (CA > 1 && sweep_cluster_smem<R>(MODE, UPD, Ls, CC, CA) <= kSweepSmemMax) {
-    if (CC == 1 && CA == 4) return pl_sweep_cl<R, MODE, UPD, 1, 4>(c, a);
-    if (CC == 1 && CA == 8) return pl_sweep_cl<R, MODE, UPD, 1, 8>(c, a);
-    if (CC == 2 && CA == 4) return pl_sweep_cl<R, MODE, UPD, 2, 4>(c, a);
-    if (CC == 2 && CA == 8) return pl_sweep_cl<R, MODE, UPD, 2, 8>(c, a);
-    if (CC == 4 && CA == 4) return pl_sweep_cl<R, MODE, UPD, 4, 4>(c, a);
-  }
-  if (CC > 1 && sweep_cluster_smem<R>(MODE, UPD, Ls, CC, 1) <= kSweepSmemMax) {
-    if (CC == 2) return pl_sweep_cl<R, MODE, UPD, 2, 1>(c, a);
-    if (CC == 4) return pl_sweep_cl<R, MODE, UPD, 4, 1>(c, a);
-    if (CC == 3) return pl_sweep_cl<R, MODE, UPD, 3, 1>(c, a);
-    if (CC == 8) return pl_sweep_cl<R, MODE, UPD, 8, 1>(c, a);
-    if (CC == 9) return pl_sweep_cl<R, MODE, UPD, 9, 1>(c, a);
-    if (CC == 16) return pl_sweep_cl<R, MODE, UPD, 16, 1>(c, a);
-  }
-  return pl_sweep_cl<R, MODE, UPD, 1, 1>(c, a);
+  ++c.launches, k_pencil_sweep<R, MODE, UPD><<<(unsigned)G.npatch, kPencilThreads, smem, c.stream>>>(a);
+  return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
@@ -1603,7 +1489,7 @@ static cudaError_t ss_chunk(SharedSolve& S, const std::vector<SolveReq*>& L) {
   const int* df2 = reinterpret_cast<const int*>(d + o_f2);
   double* const* dsc = reinterpret_cast<double* const*>(d + o_sc);
   double* dst = reinterpret_cast<double*>(d + o_st);
-  const size_t smf = sweep_dyn_smem<R>(kForward, true), smb = sweep_dyn_smem<R>(kBackward, false);
+  const size_t smf = sweep_dyn_smem<R>(kForward), smb = sweep_dyn_smem<R>(kBackward);
   static std::atomic<unsigned long long> attr_set{0};
   const unsigned long long dbit = 1ull << (S.device & 63);
   if (!(attr_set.load(std::memory_order_acquire) & dbit)) {
@@ -1615,9 +1501,9 @@ static cudaError_t ss_chunk(SharedSolve& S, const std::vector<SolveReq*>& L) {
   }
   for (int b = 0; b < kSharedChunk; ++b) {
     k_pl_spmv_batch<R><<<(unsigned)n1, kRedThreads, 0, S.stream>>>(dsa, df1, n, b);
-    k_pencil_sweep_batch<R, kForward, true><<<(unsigned)n2, kPatchLines, smf, S.stream>>>(
+    k_pencil_sweep_batch<R, kForward, true><<<(unsigned)n2, kPencilThreads, smf, S.stream>>>(
         dfa, df2, n, 2 * b);
-    k_pencil_sweep_batch<R, kBackward, false><<<(unsigned)n2, kPatchLines, smb, S.stream>>>(
+    k_pencil_sweep_batch<R, kBackward, false><<<(unsigned)n2, kPencilThreads, smb, S.stream>>>(
         dba, df2, n, 2 * b + 1);
   }
   k_pl_batch_status<<<(unsigned)((6 * n + 255) / 256), 256, 0, S.stream>>>(dsc, n, dst);
