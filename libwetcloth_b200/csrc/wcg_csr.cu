@@ -8,18 +8,22 @@
 //   * structure: the factor's columns are the upper parts of the matrix rows
 //     (factor_modified_incomplete_cholesky0 copies them, PCGSolver.h:106-117),
 //     their transpose lists for each column the earlier columns that update
-//     it, and two level schedules (forward: a row after every earlier column
-//     that updates it; backward: a row after every later row in its column)
-//     come from iterated frontier kernels;
-//   * the factorisation, one launch per forward level: each column gathers
-//     the eliminations of its earlier columns in ascending column order, with
-//     the reference's dropped-entry rule ("missing", modification 0.97) and
-//     its pivot test (ratio 0.25), so every entry sees the reference's
-//     sequence of subtractions (PCGSolver.h:142-204);
-//   * the triangular solves, one launch per level, each row gathering its
-//     terms in the order solve_lower / solve_lower_transpose_in_place apply
-//     them (:211-239);
-//   * the PCG iteration of PCGSolver::solve with its infinity-norm stop.
+//     it;
+//   * the factorisation, one launch: a thread per column waits for the earlier
+//     columns that update it and gathers their eliminations in ascending
+//     column order, with the reference's dropped-entry rule ("missing",
+//     modification 0.97) and its pivot test (ratio 0.25), so every entry sees
+//     the reference's sequence of subtractions (PCGSolver.h:142-204);
+//   * the triangular solves, one launch each: a thread per row waits for the
+//     rows it depends on and subtracts their terms in the order solve_lower /
+//     solve_lower_transpose_in_place apply them (:211-239);
+//   * the PCG iteration of PCGSolver::solve with its infinity-norm stop, tested
+//     on the device; the host looks at it every kCheck iterations (launches
+//     after the stop return at once).
+// Rows are handed out to blocks by an atomic ticket in the order of the
+// dependencies (ascending, or descending for the backward solve), so whatever
+// a row waits for belongs to a block that started earlier or to its own.  Every
+// wait is bounded.
 // Products and sums are rounded separately (_rn intrinsics), as the
 // reference's compiled code evaluates them.  Dot products are deterministic
 // block reductions; their summation order is not Eigen's, so the iterates
@@ -29,6 +33,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -43,6 +48,7 @@ constexpr double kOmega = 0.97;     // modification parameter (PCGSolver.h:100)
 constexpr double kMinRatio = 0.25;  // min_diagonal_ratio (:101)
 constexpr int kThreads = 256;
 constexpr int kDotBlocks = 296;     // 2 per SM of a B200
+constexpr int kCheck = 8;           // iterations per look at the stop test
 
 inline unsigned nblocks(long long n) { return (unsigned)((n + kThreads - 1) / kThreads); }
 
@@ -142,329 +148,408 @@ __global__ void k_csr_sort_transpose(int n, const int* __restrict__ tstart, int*
   }
 }
 
-// frontier t of the forward schedule: rows whose updating columns all sit on
-// earlier levels
-__global__ void k_csr_level_fwd(int n, const int* __restrict__ tstart, const int* __restrict__ tk,
-                                int* lev, int t, int* assigned) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || lev[i] >= 0) return;
-  for (int q = tstart[i]; q < tstart[i + 1]; ++q) {
-    const int l = ((volatile int*)lev)[tk[q]];
-    if (l < 0 || l >= t) return;
-  }
-  lev[i] = t;
-  atomicAdd(assigned, 1);
-}
+typedef unsigned long long u64;
 
-// frontier t of the backward schedule: rows whose column entries (later
-// rows) all sit on earlier levels
-__global__ void k_csr_level_bwd(int n, const int* __restrict__ ustart, const int* __restrict__ urow,
-                                int* lev, int t, int* assigned) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || lev[i] >= 0) return;
-  for (int p = ustart[i]; p < ustart[i + 1]; ++p) {
-    const int l = ((volatile int*)lev)[urow[p]];
-    if (l < 0 || l >= t) return;
-  }
-  lev[i] = t;
-  atomicAdd(assigned, 1);
+__device__ inline void ld_words(const u64* p, u64& a, u64& b) {
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(a) : "l"(p));
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(b) : "l"(p + 1));
 }
-
-__global__ void k_csr_level_count(int n, const int* __restrict__ lev, int* __restrict__ cnt) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) atomicAdd(&cnt[lev[i]], 1);
+__device__ inline void st_word(u64* p, u64 v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v));
 }
-
-__global__ void k_csr_level_scatter(int n, const int* __restrict__ lev,
-                                    const int* __restrict__ start, int* __restrict__ cur,
-                                    int* __restrict__ rows) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) rows[start[lev[i]] + atomicAdd(&cur[lev[i]], 1)] = i;
+__device__ inline int ld_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
 }
+__device__ inline void st_release(int* p, int v) {
+  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+// rounds without progress before a wait gives up (well over a second)
+constexpr long long kMaxRounds = 1ll << 22;
 
-// factor_modified_incomplete_cholesky0 (PCGSolver.h:142-204) for the columns
-// of one level: column j applies the eliminations of the earlier columns k
-// that hold row j in ascending k (the order in which the reference's column
-// loop reaches j), then takes its pivot and scales itself.
-__global__ void k_csr_factor_level(const int* __restrict__ rows, int cnt,
-                                   const int* __restrict__ rowstart, const int* __restrict__ col,
-                                   const int* __restrict__ ustart, const int* __restrict__ urow,
-                                   double* __restrict__ uval, const int* __restrict__ tstart,
-                                   const int* __restrict__ tk, const int* __restrict__ tp,
-                                   const double* __restrict__ adiag, double* __restrict__ invdiag) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= cnt) return;
-  const int j = rows[t];
-  double d = adiag[j];
+// The eliminations of column k (finished) in column j: mult is the entry of
+// row j in column k, d the running pivot of column j.
+__device__ inline double eliminate(int j, int k, double mult, double d,
+                                   const int* __restrict__ rowstart,
+                                   const int* __restrict__ col, const int* __restrict__ ustart,
+                                   const int* __restrict__ urow, double* uval) {
+  double missing = 0.0;
+  int a = ustart[k];
+  const int ek = ustart[k + 1];
   const int ej = ustart[j + 1];
-  for (int q = tstart[j]; q < tstart[j + 1]; ++q) {
-    const int k = tk[q];
-    if (adiag[k] == 0.0) continue;  // null row/column: skipped (:144)
-    const double mult = uval[tp[q]];
-    double missing = 0.0;
-    int a = ustart[k];
-    const int ek = ustart[k + 1];
-    // dropped entries above the diagonal of column j: rows of column k below
-    // j that row j of the matrix does not hold
-    int b = rowstart[j];
-    const int eb = rowstart[j + 1];
-    while (a < ek && urow[a] < j) {
-      while (b < eb) {
-        const int c = col[b];
-        if (c < urow[a]) {
-          ++b;
-        } else if (c == urow[a]) {
-          break;
-        } else {
-          missing = __dadd_rn(missing, uval[a]);
-          break;
+  // dropped entries above the diagonal of column j: rows of column k below
+  // j that row j of the matrix does not hold
+  int b = rowstart[j];
+  const int eb = rowstart[j + 1];
+  while (a < ek && urow[a] < j) {
+    while (b < eb) {
+      const int c = col[b];
+      if (c < urow[a]) {
+        ++b;
+      } else if (c == urow[a]) {
+        break;
+      } else {
+        missing = __dadd_rn(missing, __ldcg(uval + a));
+        break;
+      }
+    }
+    ++a;
+  }
+  if (a < ek && urow[a] == j) d = __dsub_rn(d, __dmul_rn(mult, __ldcg(uval + a)));
+  ++a;
+  // entries below the diagonal of column j, or dropped into missing
+  int bb = ustart[j];
+  while (a < ek && bb < ej) {
+    if (urow[bb] < urow[a]) {
+      ++bb;
+    } else if (urow[bb] == urow[a]) {
+      uval[bb] = __dsub_rn(uval[bb], __dmul_rn(mult, __ldcg(uval + a)));
+      ++a;
+      ++bb;
+    } else {
+      missing = __dadd_rn(missing, __ldcg(uval + a));
+      ++a;
+    }
+  }
+  while (a < ek) {
+    missing = __dadd_rn(missing, __ldcg(uval + a));
+    ++a;
+  }
+  return __dsub_rn(d, __dmul_rn(__dmul_rn(kOmega, mult), missing));
+}
+
+// factor_modified_incomplete_cholesky0 (PCGSolver.h:142-204): column j applies
+// the eliminations of the earlier columns k that hold row j in ascending k (the
+// order in which the reference's column loop reaches j), each once column k is
+// finished (ready[k] = 1), then takes its pivot and scales itself.
+__global__ void __launch_bounds__(kThreads)
+    k_csr_factor(int n, int* ticket, const int* __restrict__ rowstart,
+                 const int* __restrict__ col, const int* __restrict__ ustart,
+                 const int* __restrict__ urow, double* uval, const int* __restrict__ tstart,
+                 const int* __restrict__ tk, const int* __restrict__ tp,
+                 const double* __restrict__ adiag, double* __restrict__ invdiag, int* ready,
+                 int* err) {
+  __shared__ int s_block;
+  if (threadIdx.x == 0) s_block = atomicAdd(ticket, 1);
+  __syncthreads();
+  const int j = s_block * kThreads + threadIdx.x;
+  bool fin = j >= n;
+  int q = fin ? 0 : tstart[j];
+  const int eq = fin ? 0 : tstart[j + 1];
+  double d = fin ? 0.0 : adiag[j];
+  long long idle = 0;
+  // lanes of a warp may depend on one another: every round lets each lane do
+  // what it can, so the lanes that are ready go on
+  while (__any_sync(0xffffffffu, !fin)) {
+    bool moved = false;
+    if (!fin) {
+      if (q < eq) {
+        const int k = tk[q];
+        if (adiag[k] == 0.0) {  // null row/column: skipped (:144)
+          ++q;
+          moved = true;
+        } else if (ld_acquire(ready + k)) {
+          d = eliminate(j, k, __ldcg(uval + tp[q]), d, rowstart, col, ustart, urow, uval);
+          ++q;
+          moved = true;
+        }
+      } else {
+        double inv = d;
+        if (adiag[j] != 0.0) {
+          const double piv = d < __dmul_rn(kMinRatio, adiag[j]) ? adiag[j] : d;
+          inv = __ddiv_rn(1.0, __dsqrt_rn(piv));
+          for (int p = ustart[j]; p < ustart[j + 1]; ++p) uval[p] = __dmul_rn(uval[p], inv);
+        }
+        invdiag[j] = inv;
+        __threadfence();
+        st_release(ready + j, 1);
+        fin = true;
+        moved = true;
+      }
+    }
+    if (__any_sync(0xffffffffu, moved)) {
+      idle = 0;
+    } else if (++idle > kMaxRounds) {
+      atomicExch(err, 1);
+      fin = true;
+    }
+  }
+}
+
+// scalar slots (doubles); SC_DONE holds an int: 1 converged, 2 iteration limit
+enum : int { SC_RHO = 0, SC_RES, SC_ITER, SC_DONE, SC_ALPHA, SC_BETA, SC_TOL, SC_MAXIT, kNumSc };
+
+// solve_lower (PCGSolver.h:211-222, LOWER) or solve_lower_transpose_in_place
+// (:226-239): a thread per row, rows ascending or descending.  A row's terms
+// are subtracted in list order, four at a time, once the rows they name have
+// published their values: as two tagged words (tag << 32 | 32 data bits) each,
+// in shared memory for rows of the same block and in `words` for all others.
+// Bound by the chain of dependent rows: a hop inside the block costs a pass
+// over shared memory, one between blocks a round trip to L2, so the block is as
+// large as it can be.  The former launch per level took 2.5-3 us a level (two
+// solves over 118 levels of a 40^3 grid: 0.7 ms of a 1 ms iteration).
+constexpr int kTriThreads = 1024;
+template <bool LOWER>
+__global__ void __launch_bounds__(kTriThreads, 1)
+    k_csr_tri(int n, int* ticket, int ticket_base, unsigned tag, const int* __restrict__ start,
+              const int* __restrict__ dep, const int* __restrict__ pos,
+              const double* __restrict__ uval, const double* __restrict__ invdiag,
+              const double* in, double* out, u64* words, const double* __restrict__ sc, int* err) {
+  __shared__ u64 sw[2 * kTriThreads];
+  __shared__ int s_block;
+  constexpr unsigned full = 0xffffffffu;
+  if (threadIdx.x == 0) s_block = atomicAdd(ticket, 1) - ticket_base;
+  if (*(const int*)(sc + SC_DONE)) return;  // set by an earlier launch: uniform
+  sw[2 * threadIdx.x] = sw[2 * threadIdx.x + 1] = 0ull;
+  __syncthreads();
+  const int lo = s_block * kTriThreads;
+  const int idx = lo + threadIdx.x;
+  const int row = LOWER ? idx : n - 1 - idx;
+  bool fin = idx >= n;
+  int q = fin ? 0 : start[row];
+  const int e = fin ? 0 : start[row + 1];
+  double acc = fin ? 0.0 : in[row];
+  const double inv = fin ? 0.0 : invdiag[row];
+  int src[4];       // >= 0: slot in this block, < 0: -1 - row
+  double u[4], val[4];
+  int cnt = 0;
+  unsigned pend = 0, near = 0;
+  volatile u64* const vs = sw;
+  auto next_terms = [&]() {
+    cnt = min(4, e - q);
+    pend = (1u << cnt) - 1u;
+    near = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      src[j] = 0;
+      u[j] = val[j] = 0.0;
+      if (j < cnt) {
+        const int k = dep[q + j];
+        const int at = (LOWER ? k : n - 1 - k) - lo;
+        src[j] = at >= 0 ? at : -1 - k;
+        if (at >= 0) near |= 1u << j;
+        u[j] = uval[LOWER ? pos[q + j] : q + j];
+      }
+    }
+  };
+  if (!fin) next_terms();
+  long long idle = 0;
+  while (!__all_sync(full, fin)) {
+    bool moved = false;
+    // terms from other blocks, all loads in flight at once
+    if (!fin && (pend & ~near)) {
+      u64 w0[4], w1[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if ((pend & ~near) >> j & 1) ld_words(words + 2ll * (-1 - src[j]), w0[j], w1[j]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (((pend & ~near) >> j & 1) && (unsigned)(w0[j] >> 32) == tag &&
+            (unsigned)(w1[j] >> 32) == tag) {
+          val[j] = __longlong_as_double((long long)((w1[j] << 32) | (w0[j] & 0xffffffffull)));
+          pend &= ~(1u << j);
+          moved = true;
+        }
+    }
+    // terms from this block, for as long as any lane of the warp gets on
+    bool again;
+    do {
+      bool step = false;
+      if (!fin) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if ((pend & near) >> j & 1) {
+            const u64 w0 = vs[2 * src[j]], w1 = vs[2 * src[j] + 1];
+            if ((unsigned)(w0 >> 32) == tag && (unsigned)(w1 >> 32) == tag) {
+              val[j] = __longlong_as_double((long long)((w1 << 32) | (w0 & 0xffffffffull)));
+              pend &= ~(1u << j);
+              step = true;
+            }
+          }
+        if (!pend) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (j < cnt) acc = __dsub_rn(acc, __dmul_rn(u[j], val[j]));
+          q += cnt;
+          step = true;
+          if (q < e) {
+            next_terms();
+          } else {
+            const double y = __dmul_rn(acc, inv);
+            const u64 b = (u64)__double_as_longlong(y);
+            const u64 w0 = ((u64)tag << 32) | (b & 0xffffffffull);
+            const u64 w1 = ((u64)tag << 32) | (b >> 32);
+            vs[2 * threadIdx.x] = w0;
+            vs[2 * threadIdx.x + 1] = w1;
+            st_word(words + 2ll * row, w0);
+            st_word(words + 2ll * row + 1, w1);
+            out[row] = y;
+            fin = true;
+          }
         }
       }
-      ++a;
+      again = __any_sync(full, step);
+      moved = moved || again;
+    } while (again);
+    if (__any_sync(full, moved)) {
+      idle = 0;
+    } else if (++idle > kMaxRounds) {
+      if (!fin) atomicExch(err, 1);
+      fin = true;
     }
-    if (a < ek && urow[a] == j) d = __dsub_rn(d, __dmul_rn(mult, uval[a]));
-    ++a;
-    // entries below the diagonal of column j, or dropped into missing
-    int bb = ustart[j];
-    while (a < ek && bb < ej) {
-      if (urow[bb] < urow[a]) {
-        ++bb;
-      } else if (urow[bb] == urow[a]) {
-        uval[bb] = __dsub_rn(uval[bb], __dmul_rn(mult, uval[a]));
-        ++a;
-        ++bb;
-      } else {
-        missing = __dadd_rn(missing, uval[a]);
-        ++a;
-      }
-    }
-    while (a < ek) {
-      missing = __dadd_rn(missing, uval[a]);
-      ++a;
-    }
-    d = __dsub_rn(d, __dmul_rn(__dmul_rn(kOmega, mult), missing));
   }
-  if (adiag[j] == 0.0) {
-    invdiag[j] = d;
-    return;
-  }
-  const double piv = d < __dmul_rn(kMinRatio, adiag[j]) ? adiag[j] : d;
-  const double inv = __ddiv_rn(1.0, __dsqrt_rn(piv));
-  for (int p = ustart[j]; p < ej; ++p) uval[p] = __dmul_rn(uval[p], inv);
-  invdiag[j] = inv;
 }
 
-// solve_lower (PCGSolver.h:211-222) for the rows of one forward level
-__global__ void k_csr_lower_level(const int* __restrict__ rows, int cnt,
-                                  const int* __restrict__ tstart, const int* __restrict__ tk,
-                                  const int* __restrict__ tp, const double* __restrict__ uval,
-                                  const double* __restrict__ invdiag,
-                                  const double* __restrict__ rhs, double* __restrict__ y) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= cnt) return;
-  const int r = rows[t];
-  double acc = rhs[r];
-  for (int q = tstart[r]; q < tstart[r + 1]; ++q)
-    acc = __dsub_rn(acc, __dmul_rn(uval[tp[q]], y[tk[q]]));
-  y[r] = __dmul_rn(acc, invdiag[r]);
-}
-
-// solve_lower_transpose_in_place (:226-239) for the rows of one backward level
-__global__ void k_csr_upper_level(const int* __restrict__ rows, int cnt,
-                                  const int* __restrict__ ustart, const int* __restrict__ urow,
-                                  const double* __restrict__ uval,
-                                  const double* __restrict__ invdiag, double* __restrict__ x) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= cnt) return;
-  const int i = rows[t];
-  double acc = x[i];
-  for (int p = ustart[i]; p < ustart[i + 1]; ++p)
-    acc = __dsub_rn(acc, __dmul_rn(uval[p], x[urow[p]]));
-  x[i] = __dmul_rn(acc, invdiag[i]);
-}
-
-// multiply(FixedSparseMatrix, x, result) (SparseMatrix.h:299-320)
-__global__ void k_csr_spmv(int n, const int* __restrict__ rowstart, const int* __restrict__ col,
-                           const double* __restrict__ val, const double* __restrict__ x,
-                           double* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double acc = 0.0;
-  for (int p = rowstart[i]; p < rowstart[i + 1]; ++p)
-    acc = __dadd_rn(acc, __dmul_rn(val[p], x[col[p]]));
-  out[i] = acc;
-}
-
-// per-block partial of sum a_i b_i (fixed grid, fixed order: deterministic)
-__global__ void k_csr_dot_part(int n, const double* __restrict__ a, const double* __restrict__ b,
-                               double* __restrict__ part) {
-  __shared__ double sm[kThreads];
-  double acc = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    acc = __dadd_rn(acc, __dmul_rn(a[i], b[i]));
-  sm[threadIdx.x] = acc;
-  __syncthreads();
-  for (int s = kThreads / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) sm[threadIdx.x] = __dadd_rn(sm[threadIdx.x], sm[threadIdx.x + s]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = sm[0];
-}
-
-// per-block partial of max |a_i|
-__global__ void k_csr_absmax_part(int n, const double* __restrict__ a, double* __restrict__ part) {
-  __shared__ double sm[kThreads];
-  double m = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double v = fabs(a[i]);
-    m = (v > m || v != v) ? v : m;  // NaN propagates
-  }
-  sm[threadIdx.x] = m;
+// sum (or maximum, NaN first) over a block of kThreads
+__device__ inline double block_reduce(double v, double* sm, bool is_max) {
+  sm[threadIdx.x] = v;
   __syncthreads();
   for (int s = kThreads / 2; s > 0; s >>= 1) {
     if (threadIdx.x < s) {
-      const double o = sm[threadIdx.x + s];
-      if (o > sm[threadIdx.x] || o != o) sm[threadIdx.x] = o;
+      const double a = sm[threadIdx.x], o = sm[threadIdx.x + s];
+      sm[threadIdx.x] = is_max ? ((o > a || o != o) ? o : a) : __dadd_rn(a, o);
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = sm[0];
+  const double r = sm[0];
+  __syncthreads();
+  return r;
 }
 
-// sc[slot] = sum (or max) of the partials, in block order
-__global__ void k_csr_finish(const double* __restrict__ part, int nparts, double* sc, int slot,
-                             int is_max) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// Writes this block's partial; true in the last block, with the reduction of
+// all partials in block order by thread, then the block tree (deterministic).
+__device__ inline bool grid_reduce(double v, double* part, int* ctr, double* sm, bool is_max,
+                                   double* out) {
+  __shared__ int s_last;
+  const double b = block_reduce(v, sm, is_max);
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = b;
+    __threadfence();
+    s_last = atomicAdd(ctr, 1) == (int)gridDim.x - 1;
+    if (s_last) {
+      atomicExch(ctr, 0);
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (!s_last) return false;
   double acc = 0.0;
-  for (int b = 0; b < nparts; ++b) {
-    const double v = part[b];
-    if (is_max)
-      acc = (v > acc || v != v) ? v : acc;
-    else
-      acc = __dadd_rn(acc, v);
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) {
+    const double o = __ldcg(part + i);
+    acc = is_max ? ((o > acc || o != o) ? o : acc) : __dadd_rn(acc, o);
   }
-  sc[slot] = acc;
+  *out = block_reduce(acc, sm, is_max);
+  return true;
 }
 
-// scalar slots
-enum : int { SC_RHO = 0, SC_SZ, SC_RES, SC_RHONEW, SC_ALPHA, SC_BETA, kNumSc = 8 };
-
-__global__ void k_csr_alpha(double* sc) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) sc[SC_ALPHA] = __ddiv_rn(sc[SC_RHO], sc[SC_SZ]);
-}
-
-__global__ void k_csr_beta(double* sc) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    sc[SC_BETA] = __ddiv_rn(sc[SC_RHONEW], sc[SC_RHO]);
-    sc[SC_RHO] = sc[SC_RHONEW];
+// z = A s (multiply(FixedSparseMatrix, x, result), SparseMatrix.h:299-320);
+// the last block: alpha = rho / s.z
+__global__ void __launch_bounds__(kThreads)
+    k_csr_spmv(int n, const int* __restrict__ rowstart, const int* __restrict__ col,
+               const double* __restrict__ val, const double* __restrict__ s,
+               double* __restrict__ z, double* sc, double* part, int* ctr) {
+  __shared__ double sm[kThreads];
+  if (*(const int*)(sc + SC_DONE)) return;
+  double dot = 0.0;
+  for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
+    double acc = 0.0;
+    for (int p = rowstart[i]; p < rowstart[i + 1]; ++p)
+      acc = __dadd_rn(acc, __dmul_rn(val[p], s[col[p]]));
+    z[i] = acc;
+    dot = __dadd_rn(dot, __dmul_rn(s[i], acc));
   }
+  double sz;
+  if (grid_reduce(dot, part, ctr, sm, false, &sz) && threadIdx.x == 0)
+    sc[SC_ALPHA] = __ddiv_rn(sc[SC_RHO], sz);
 }
 
-// result += s * alpha;  r += z * (-alpha)  (BLAS::add_scaled, BLASWrapper.h:52-56)
-__global__ void k_csr_update_xr(int n, const double* __restrict__ s, const double* __restrict__ z,
-                                double* __restrict__ x, double* __restrict__ r,
-                                const double* __restrict__ sc) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// result += s * alpha;  r += z * (-alpha)  (BLAS::add_scaled, BLASWrapper.h:
+// 52-56); the last block: the stop test on max |r|.  x null: max |r| alone.
+__global__ void __launch_bounds__(kThreads)
+    k_csr_update_xr(int n, const double* __restrict__ s, const double* __restrict__ z,
+                    double* __restrict__ x, double* __restrict__ r, double* sc, double* part,
+                    int* ctr) {
+  __shared__ double sm[kThreads];
+  if (*(const int*)(sc + SC_DONE)) return;
   const double alpha = sc[SC_ALPHA];
-  x[i] = __dadd_rn(x[i], __dmul_rn(s[i], alpha));
-  r[i] = __dadd_rn(r[i], __dmul_rn(z[i], -alpha));
-}
-
-// z += s * beta (then the host swaps s and z)
-__global__ void k_csr_update_z(int n, const double* __restrict__ s, double* __restrict__ z,
-                               const double* __restrict__ sc) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) z[i] = __dadd_rn(z[i], __dmul_rn(s[i], sc[SC_BETA]));
-}
-
-struct Levels {
-  std::vector<int> start;  // host copy of the level offsets
-  Mem rows;                // rows ordered by level
-};
-
-// iterated frontier: level t holds the rows whose dependencies all sit on
-// levels below t; every step assigns at least the lowest unassigned row
-template <bool kForward>
-cudaError_t make_levels(int n, const int* dep_start, const int* dep_list, Levels& L,
-                        cudaStream_t st) {
-  Mem lev, cnt, cur, assigned;
-  CSR_TRY(lev.alloc((size_t)n * sizeof(int)));
-  CSR_TRY(assigned.alloc(sizeof(int)));
-  CSR_TRY(cudaMemsetAsync(lev.p, 0xff, (size_t)n * sizeof(int), st));
-  CSR_TRY(cudaMemsetAsync(assigned.p, 0, sizeof(int), st));
-  int total = 0, t = 0;
-  while (total < n) {
-    if (kForward)
-      k_csr_level_fwd<<<nblocks(n), kThreads, 0, st>>>(n, dep_start, dep_list, lev.as<int>(), t,
-                                                       assigned.as<int>());
-    else
-      k_csr_level_bwd<<<nblocks(n), kThreads, 0, st>>>(n, dep_start, dep_list, lev.as<int>(), t,
-                                                       assigned.as<int>());
-    CSR_TRY(cudaGetLastError());
-    int now = 0;
-    CSR_TRY(cudaMemcpyAsync(&now, assigned.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CSR_TRY(cudaStreamSynchronize(st));
-    if (now == total) return cudaErrorInvalidValue;  // cannot happen for a triangular order
-    total = now;
-    ++t;
+  double m = 0.0;
+  for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
+    double rv = r[i];
+    if (x) {
+      x[i] = __dadd_rn(x[i], __dmul_rn(s[i], alpha));
+      rv = __dadd_rn(rv, __dmul_rn(z[i], -alpha));
+      r[i] = rv;
+    }
+    const double v = fabs(rv);
+    m = (v > m || v != v) ? v : m;  // NaN propagates
   }
-  const int nlev = t;
-  CSR_TRY(cnt.alloc((size_t)(nlev + 1) * sizeof(int)));
-  CSR_TRY(cur.alloc((size_t)nlev * sizeof(int)));
-  CSR_TRY(cudaMemsetAsync(cnt.p, 0, (size_t)(nlev + 1) * sizeof(int), st));
-  CSR_TRY(cudaMemsetAsync(cur.p, 0, (size_t)nlev * sizeof(int), st));
-  k_csr_level_count<<<nblocks(n), kThreads, 0, st>>>(n, lev.as<int>(), cnt.as<int>());
-  std::vector<int> c(nlev);
-  CSR_TRY(cudaMemcpyAsync(c.data(), cnt.p, (size_t)nlev * sizeof(int), cudaMemcpyDeviceToHost, st));
-  CSR_TRY(cudaStreamSynchronize(st));
-  L.start.assign(nlev + 1, 0);
-  for (int l = 0; l < nlev; ++l) L.start[l + 1] = L.start[l] + c[l];
-  CSR_TRY(cudaMemcpyAsync(cnt.p, L.start.data(), (size_t)(nlev + 1) * sizeof(int),
-                          cudaMemcpyHostToDevice, st));
-  CSR_TRY(L.rows.alloc((size_t)n * sizeof(int)));
-  k_csr_level_scatter<<<nblocks(n), kThreads, 0, st>>>(n, lev.as<int>(), cnt.as<int>(),
-                                                       cur.as<int>(), L.rows.as<int>());
-  CSR_TRY(cudaGetLastError());
-  return cudaStreamSynchronize(st);
+  double res;
+  if (grid_reduce(m, part, ctr, sm, true, &res) && threadIdx.x == 0) {
+    sc[SC_RES] = res;
+    if (x) {
+      sc[SC_ITER] += 1.0;
+      if (res <= sc[SC_TOL]) *(int*)(sc + SC_DONE) = 1;
+      else if (sc[SC_ITER] >= sc[SC_MAXIT]) *(int*)(sc + SC_DONE) = 2;
+    }
+  }
+}
+
+// the last block: rho_new = z.r, beta = rho_new / rho (init: rho alone)
+__global__ void __launch_bounds__(kThreads)
+    k_csr_dot(int n, const double* __restrict__ z, const double* __restrict__ r, double* sc,
+              double* part, int* ctr, int init) {
+  __shared__ double sm[kThreads];
+  if (*(const int*)(sc + SC_DONE)) return;
+  double acc = 0.0;
+  for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads)
+    acc = __dadd_rn(acc, __dmul_rn(z[i], r[i]));
+  double rho;
+  if (grid_reduce(acc, part, ctr, sm, false, &rho) && threadIdx.x == 0) {
+    if (!init) sc[SC_BETA] = __ddiv_rn(rho, sc[SC_RHO]);
+    sc[SC_RHO] = rho;
+  }
+}
+
+// s = z + s * beta
+__global__ void __launch_bounds__(kThreads)
+    k_csr_direction(int n, const double* __restrict__ z, double* __restrict__ s,
+                    const double* __restrict__ sc) {
+  if (*(const int*)(sc + SC_DONE)) return;
+  const double beta = sc[SC_BETA];
+  for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads)
+    s[i] = __dadd_rn(z[i], __dmul_rn(s[i], beta));
 }
 
 struct Solver {
   int n = 0;
   cudaStream_t st = nullptr;
-  Mem rowstart, col, val, adiag, invdiag, ustart, urow, uval, tstart, tk, tp;
-  Levels fwd, bwd;
-  Mem vx, vr, vz, vs, part, sc;
+  int *rowstart, *col, *ustart, *urow, *tstart, *tk, *tp, *ctl;
+  double *val, *adiag, *invdiag, *uval, *x, *r, *z, *s, *part, *sc;
+  u64* words;
+  unsigned tag = 0;   // of the last triangular solve
+  int tickets = 0;    // handed out by the triangular solves so far
 
-  void precondition(double* in, double* out) {
-    for (size_t l = 0; l + 1 < fwd.start.size(); ++l) {
-      const int cnt = fwd.start[l + 1] - fwd.start[l];
-      k_csr_lower_level<<<nblocks(cnt), kThreads, 0, st>>>(
-          fwd.rows.as<int>() + fwd.start[l], cnt, tstart.as<int>(), tk.as<int>(), tp.as<int>(),
-          uval.as<double>(), invdiag.as<double>(), in, out);
-    }
-    for (size_t l = 0; l + 1 < bwd.start.size(); ++l) {
-      const int cnt = bwd.start[l + 1] - bwd.start[l];
-      k_csr_upper_level<<<nblocks(cnt), kThreads, 0, st>>>(
-          bwd.rows.as<int>() + bwd.start[l], cnt, ustart.as<int>(), urow.as<int>(),
-          uval.as<double>(), invdiag.as<double>(), out);
-    }
+  // ctl: 0 malformed matrix, 1 wait given up, 2 reduction count, 3 ticket of
+  // the triangular solves, 4 ticket of the factorisation
+  void precondition(const double* in, double* out) {
+    const int nb = (n + kTriThreads - 1) / kTriThreads;
+    k_csr_tri<true><<<nb, kTriThreads, 0, st>>>(n, ctl + 3, tickets, ++tag, tstart, tk, tp, uval,
+                                                invdiag, in, out, words, sc, ctl + 1);
+    tickets += nb;
+    k_csr_tri<false><<<nb, kTriThreads, 0, st>>>(n, ctl + 3, tickets, ++tag, ustart, urow, nullptr,
+                                                 uval, invdiag, out, out, words, sc, ctl + 1);
+    tickets += nb;
   }
-  void dot(const double* a, const double* b, int slot) {
-    k_csr_dot_part<<<kDotBlocks, kThreads, 0, st>>>(n, a, b, part.as<double>());
-    k_csr_finish<<<1, 1, 0, st>>>(part.as<double>(), kDotBlocks, sc.as<double>(), slot, 0);
-  }
-  void absmax(const double* a, int slot) {
-    k_csr_absmax_part<<<kDotBlocks, kThreads, 0, st>>>(n, a, part.as<double>());
-    k_csr_finish<<<1, 1, 0, st>>>(part.as<double>(), kDotBlocks, sc.as<double>(), slot, 1);
-  }
-  cudaError_t read(int slot, double* out) {
-    CSR_TRY(cudaMemcpyAsync(out, sc.as<double>() + slot, sizeof(double), cudaMemcpyDeviceToHost, st));
+  unsigned grid() const { return std::min(nblocks(n), (unsigned)kDotBlocks); }
+  cudaError_t read(double* out, int slot, int k) {
+    CSR_TRY(cudaMemcpyAsync(out, sc + slot, k * sizeof(double), cudaMemcpyDeviceToHost, st));
     return cudaStreamSynchronize(st);
   }
 };
 
-// 0: converged, 1: not converged (iteration limit or rho 0/NaN), 2: bad matrix
+// 0: converged, 1: not converged (iteration limit or rho 0/NaN), 2: bad matrix,
+// 3: a wait gave up
 cudaError_t csr_solve(const int* h_rowstart, const int* h_col, const double* h_val, int n,
                       const double* h_rhs, double* h_x, double tolerance_factor, int maxiter,
                       double* residual_out, int* iters_out, int* outcome) {
@@ -476,137 +561,137 @@ cudaError_t csr_solve(const int* h_rowstart, const int* h_col, const double* h_v
     ~StreamGuard() { cudaStreamDestroy(s); }
   } guard{S.st};
   cudaStream_t st = S.st;
-  const int nnz = h_rowstart[n] - h_rowstart[0];
-  CSR_TRY(S.rowstart.alloc((size_t)(n + 1) * sizeof(int)));
-  CSR_TRY(S.col.alloc((size_t)nnz * sizeof(int)));
-  CSR_TRY(S.val.alloc((size_t)nnz * sizeof(double)));
+  const long long nnz = (long long)h_rowstart[n] - h_rowstart[0];
+  // one allocation for everything (the factor has at most nnz entries)
+  const size_t vb = (size_t)n * sizeof(double), ib = (size_t)(n + 1) * sizeof(int);
+  const size_t scan_b = (size_t)((n + 1 + kScanTile - 1) / kScanTile + 1) * sizeof(int);
+  Mem mem;
+  size_t total = 0;
+  auto place = [&](size_t bytes) {
+    const size_t at = total;
+    total += (bytes + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t o_rs = place(ib), o_col = place(nnz * sizeof(int)), o_val = place(nnz * sizeof(double));
+  const size_t o_us = place(ib), o_ur = place(nnz * sizeof(int)), o_uv = place(nnz * sizeof(double));
+  const size_t o_ts = place(ib), o_tk = place(nnz * sizeof(int)), o_tp = place(nnz * sizeof(int));
+  const size_t o_ad = place(vb), o_id = place(vb);
+  const size_t o_x = place(vb), o_r = place(vb), o_z = place(vb), o_s = place(vb);
+  const size_t o_part = place(kDotBlocks * sizeof(double)), o_tmp = place(scan_b);
+  // zeroed: counters, the transpose counts and cursors, the ready flags, the
+  // words of the triangular solves, the scalars
+  const size_t o_zero = total;
+  const size_t o_ctl = place(8 * sizeof(int)), o_tc = place(ib), o_tcur = place(ib);
+  const size_t o_rdy = place(ib), o_w = place(2 * (size_t)n * sizeof(u64));
+  const size_t o_sc = place(kNumSc * sizeof(double));
+  CSR_TRY(mem.alloc(total));
+  unsigned char* const m = mem.as<unsigned char>();
+  S.rowstart = (int*)(m + o_rs);
+  S.col = (int*)(m + o_col);
+  S.val = (double*)(m + o_val);
+  S.ustart = (int*)(m + o_us);
+  S.urow = (int*)(m + o_ur);
+  S.uval = (double*)(m + o_uv);
+  S.tstart = (int*)(m + o_ts);
+  S.tk = (int*)(m + o_tk);
+  S.tp = (int*)(m + o_tp);
+  S.adiag = (double*)(m + o_ad);
+  S.invdiag = (double*)(m + o_id);
+  S.x = (double*)(m + o_x);
+  S.r = (double*)(m + o_r);
+  S.z = (double*)(m + o_z);
+  S.s = (double*)(m + o_s);
+  S.part = (double*)(m + o_part);
+  S.ctl = (int*)(m + o_ctl);
+  S.words = (u64*)(m + o_w);
+  S.sc = (double*)(m + o_sc);
+  int* const tmp = (int*)(m + o_tmp);
+  int* const tcount = (int*)(m + o_tc);
+  int* const tcur = (int*)(m + o_tcur);
+  int* const ready = (int*)(m + o_rdy);
+  CSR_TRY(cudaMemsetAsync(m + o_zero, 0, total - o_zero, st));
   // rowstart relative to its first entry
   std::vector<int> rs(h_rowstart, h_rowstart + n + 1);
   const int base = rs[0];
   for (int& v : rs) v -= base;
-  CSR_TRY(cudaMemcpyAsync(S.rowstart.p, rs.data(), (size_t)(n + 1) * sizeof(int),
-                          cudaMemcpyHostToDevice, st));
-  CSR_TRY(cudaMemcpyAsync(S.col.p, h_col + base, (size_t)nnz * sizeof(int), cudaMemcpyHostToDevice, st));
-  CSR_TRY(cudaMemcpyAsync(S.val.p, h_val + base, (size_t)nnz * sizeof(double),
-                          cudaMemcpyHostToDevice, st));
-  Mem ucount, bad, tcount, tcur;
-  CSR_TRY(ucount.alloc((size_t)(n + 1) * sizeof(int)));
-  CSR_TRY(S.adiag.alloc((size_t)n * sizeof(double)));
-  CSR_TRY(S.invdiag.alloc((size_t)n * sizeof(double)));
-  CSR_TRY(bad.alloc(sizeof(int)));
-  CSR_TRY(cudaMemsetAsync(bad.p, 0, sizeof(int), st));
-  k_csr_rows<<<nblocks(n), kThreads, 0, st>>>(n, S.rowstart.as<int>(), S.col.as<int>(),
-                                              S.val.as<double>(), ucount.as<int>(),
-                                              S.adiag.as<double>(), bad.as<int>());
-  int hbad = 0;
-  CSR_TRY(cudaMemcpyAsync(&hbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CSR_TRY(cudaMemcpyAsync(S.rowstart, rs.data(), ib, cudaMemcpyHostToDevice, st));
+  CSR_TRY(cudaMemcpyAsync(S.col, h_col + base, nnz * sizeof(int), cudaMemcpyHostToDevice, st));
+  CSR_TRY(cudaMemcpyAsync(S.val, h_val + base, nnz * sizeof(double), cudaMemcpyHostToDevice, st));
+  // the upper counts of the rows go to tstart's place until they are scanned
+  int* const ucount = S.tstart;
+  k_csr_rows<<<nblocks(n), kThreads, 0, st>>>(n, S.rowstart, S.col, S.val, ucount, S.adiag, S.ctl);
+  int hctl[2] = {0, 0};
+  CSR_TRY(cudaMemcpyAsync(hctl, S.ctl, sizeof(int), cudaMemcpyDeviceToHost, st));
   CSR_TRY(cudaStreamSynchronize(st));
-  if (hbad) {
+  if (hctl[0]) {
     *outcome = 2;
     return cudaSuccess;
   }
   // factor columns (upper parts of the rows) and their transpose
-  Mem tmp;
-  CSR_TRY(tmp.alloc((size_t)((n + 1 + kScanTile - 1) / kScanTile + 1) * sizeof(int)));
-  CSR_TRY(S.ustart.alloc((size_t)(n + 1) * sizeof(int)));
-  exclusive_scan<int, int>(ucount.as<int>(), n, S.ustart.as<int>(), tmp.as<int>(),
-                           S.ustart.as<int>() + n, st);
-  int nu = 0;
-  CSR_TRY(cudaMemcpyAsync(&nu, S.ustart.as<int>() + n, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CSR_TRY(cudaStreamSynchronize(st));
-  CSR_TRY(S.urow.alloc((size_t)nu * sizeof(int)));
-  CSR_TRY(S.uval.alloc((size_t)nu * sizeof(double)));
-  CSR_TRY(tcount.alloc((size_t)(n + 1) * sizeof(int)));
-  CSR_TRY(tcur.alloc((size_t)n * sizeof(int)));
-  CSR_TRY(cudaMemsetAsync(tcount.p, 0, (size_t)(n + 1) * sizeof(int), st));
-  CSR_TRY(cudaMemsetAsync(tcur.p, 0, (size_t)n * sizeof(int), st));
-  k_csr_upper<<<nblocks(n), kThreads, 0, st>>>(n, S.rowstart.as<int>(), S.col.as<int>(),
-                                               S.val.as<double>(), S.ustart.as<int>(),
-                                               S.urow.as<int>(), S.uval.as<double>(),
-                                               tcount.as<int>());
-  CSR_TRY(S.tstart.alloc((size_t)(n + 1) * sizeof(int)));
-  exclusive_scan<int, int>(tcount.as<int>(), n, S.tstart.as<int>(), tmp.as<int>(),
-                           S.tstart.as<int>() + n, st);
-  CSR_TRY(S.tk.alloc((size_t)nu * sizeof(int)));
-  CSR_TRY(S.tp.alloc((size_t)nu * sizeof(int)));
-  k_csr_transpose<<<nblocks(n), kThreads, 0, st>>>(n, S.ustart.as<int>(), S.urow.as<int>(),
-                                                   S.tstart.as<int>(), tcur.as<int>(),
-                                                   S.tk.as<int>(), S.tp.as<int>());
-  k_csr_sort_transpose<<<nblocks(n), kThreads, 0, st>>>(n, S.tstart.as<int>(), S.tk.as<int>(),
-                                                        S.tp.as<int>());
+  exclusive_scan<int, int>(ucount, n, S.ustart, tmp, S.ustart + n, st);
+  k_csr_upper<<<nblocks(n), kThreads, 0, st>>>(n, S.rowstart, S.col, S.val, S.ustart, S.urow,
+                                               S.uval, tcount);
+  exclusive_scan<int, int>(tcount, n, S.tstart, tmp, S.tstart + n, st);
+  k_csr_transpose<<<nblocks(n), kThreads, 0, st>>>(n, S.ustart, S.urow, S.tstart, tcur, S.tk, S.tp);
+  k_csr_sort_transpose<<<nblocks(n), kThreads, 0, st>>>(n, S.tstart, S.tk, S.tp);
   CSR_TRY(cudaGetLastError());
-  CSR_TRY((make_levels<true>(n, S.tstart.as<int>(), S.tk.as<int>(), S.fwd, st)));
-  CSR_TRY((make_levels<false>(n, S.ustart.as<int>(), S.urow.as<int>(), S.bwd, st)));
 
-  // PCG vectors
-  const size_t vb = (size_t)n * sizeof(double);
-  CSR_TRY(S.vx.alloc(vb));
-  CSR_TRY(S.vr.alloc(vb));
-  CSR_TRY(S.vz.alloc(vb));
-  CSR_TRY(S.vs.alloc(vb));
-  CSR_TRY(S.part.alloc(kDotBlocks * sizeof(double)));
-  CSR_TRY(S.sc.alloc(kNumSc * sizeof(double)));
-  double* x = S.vx.as<double>();
-  double* r = S.vr.as<double>();
-  double* z = S.vz.as<double>();
-  double* s = S.vs.as<double>();
-  CSR_TRY(cudaMemsetAsync(x, 0, vb, st));
-  CSR_TRY(cudaMemcpyAsync(r, h_rhs, vb, cudaMemcpyHostToDevice, st));
+  // PCG
+  CSR_TRY(cudaMemsetAsync(S.x, 0, vb, st));
+  CSR_TRY(cudaMemcpyAsync(S.r, h_rhs, vb, cudaMemcpyHostToDevice, st));
   int iters = 0;
   bool ok = false;
   double res = 0.0;
-  S.absmax(r, SC_RES);
-  CSR_TRY(S.read(SC_RES, &res));
+  k_csr_update_xr<<<S.grid(), kThreads, 0, st>>>(n, nullptr, nullptr, nullptr, S.r, S.sc, S.part,
+                                                 S.ctl + 2);
+  CSR_TRY(S.read(&res, SC_RES, 1));
   if (res < 1e-30) {
     ok = true;
   } else {
     const double tf = tolerance_factor < 1e-30 ? 1e-30 : tolerance_factor;
-    const double tol = tf * res;
-    // the factorisation, level by level
-    for (size_t l = 0; l + 1 < S.fwd.start.size(); ++l) {
-      const int cnt = S.fwd.start[l + 1] - S.fwd.start[l];
-      k_csr_factor_level<<<nblocks(cnt), kThreads, 0, st>>>(
-          S.fwd.rows.as<int>() + S.fwd.start[l], cnt, S.rowstart.as<int>(), S.col.as<int>(),
-          S.ustart.as<int>(), S.urow.as<int>(), S.uval.as<double>(), S.tstart.as<int>(),
-          S.tk.as<int>(), S.tp.as<int>(), S.adiag.as<double>(), S.invdiag.as<double>());
-    }
+    const double lim[2] = {tf * res, (double)maxiter};  // SC_TOL, SC_MAXIT
+    CSR_TRY(cudaMemcpyAsync(S.sc + SC_TOL, lim, sizeof(lim), cudaMemcpyHostToDevice, st));
+    k_csr_factor<<<nblocks(n), kThreads, 0, st>>>(n, S.ctl + 4, S.rowstart, S.col, S.ustart, S.urow,
+                                                  S.uval, S.tstart, S.tk, S.tp, S.adiag, S.invdiag,
+                                                  ready, S.ctl + 1);
+    S.precondition(S.r, S.z);
+    k_csr_dot<<<S.grid(), kThreads, 0, st>>>(n, S.z, S.r, S.sc, S.part, S.ctl + 2, 1);
     CSR_TRY(cudaGetLastError());
-    S.precondition(r, z);
-    S.dot(z, r, SC_RHO);
     double rho = 0.0;
-    CSR_TRY(S.read(SC_RHO, &rho));
-    if (!(rho == 0.0 || rho != rho)) {
-      CSR_TRY(cudaMemcpyAsync(s, z, vb, cudaMemcpyDeviceToDevice, st));
-      int it = 0;
-      for (; it < maxiter; ++it) {
-        k_csr_spmv<<<nblocks(n), kThreads, 0, st>>>(n, S.rowstart.as<int>(), S.col.as<int>(),
-                                                    S.val.as<double>(), s, z);
-        S.dot(s, z, SC_SZ);
-        k_csr_alpha<<<1, 1, 0, st>>>(S.sc.as<double>());
-        k_csr_update_xr<<<nblocks(n), kThreads, 0, st>>>(n, s, z, x, r, S.sc.as<double>());
-        S.absmax(r, SC_RES);
+    CSR_TRY(S.read(&rho, SC_RHO, 1));
+    if (!(rho == 0.0 || rho != rho) && maxiter > 0) {
+      CSR_TRY(cudaMemcpyAsync(S.s, S.z, vb, cudaMemcpyDeviceToDevice, st));
+      for (;;) {
+        for (int k = 0; k < kCheck; ++k) {
+          k_csr_spmv<<<S.grid(), kThreads, 0, st>>>(n, S.rowstart, S.col, S.val, S.s, S.z, S.sc,
+                                                    S.part, S.ctl + 2);
+          k_csr_update_xr<<<S.grid(), kThreads, 0, st>>>(n, S.s, S.z, S.x, S.r, S.sc, S.part,
+                                                         S.ctl + 2);
+          S.precondition(S.r, S.z);
+          k_csr_dot<<<S.grid(), kThreads, 0, st>>>(n, S.z, S.r, S.sc, S.part, S.ctl + 2, 0);
+          k_csr_direction<<<S.grid(), kThreads, 0, st>>>(n, S.z, S.s, S.sc);
+        }
         CSR_TRY(cudaGetLastError());
-        CSR_TRY(S.read(SC_RES, &res));
-        if (res <= tol) {
-          iters = it + 1;
-          ok = true;
+        double h[3];
+        CSR_TRY(S.read(h, SC_RES, 3));  // residual, iterations, done
+        int done;
+        std::memcpy(&done, &h[2], sizeof(done));
+        res = h[0];
+        iters = (int)h[1];
+        if (done) {
+          ok = done == 1;
           break;
         }
-        S.precondition(r, z);
-        S.dot(z, r, SC_RHONEW);
-        k_csr_beta<<<1, 1, 0, st>>>(S.sc.as<double>());
-        k_csr_update_z<<<nblocks(n), kThreads, 0, st>>>(n, s, z, S.sc.as<double>());
-        std::swap(s, z);
       }
-      if (!ok) iters = it;
     }
   }
-  CSR_TRY(cudaMemcpyAsync(h_x, x, vb, cudaMemcpyDeviceToHost, st));
+  CSR_TRY(cudaMemcpyAsync(hctl, S.ctl, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  CSR_TRY(cudaMemcpyAsync(h_x, S.x, vb, cudaMemcpyDeviceToHost, st));
   CSR_TRY(cudaStreamSynchronize(st));
   CSR_TRY(cudaGetLastError());
   *residual_out = res;
   *iters_out = iters;
-  *outcome = ok ? 0 : 1;
+  *outcome = hctl[1] ? 3 : (ok ? 0 : 1);
   return cudaSuccess;
 }
 
@@ -638,6 +723,9 @@ extern "C" int wcg_pcg_solve_csr(const int* rowstart, const int* col, const doub
     return wcg::set_last_error(WCG_ERR_ARG,
                                "wcg_pcg_solve_csr: rows must hold strictly ascending columns "
                                "in [0, n) and rowstart must not decrease");
+  if (outcome == 3)
+    return wcg::set_last_error(WCG_ERR_DEVICE,
+                               "wcg_pcg_solve_csr: a row reached its wait limit");
   if (outcome == 1)
     return wcg::set_last_error(WCG_ERR_NOT_CONVERGED,
                                "wcg_pcg_solve_csr: iteration limit reached or rho was 0/NaN");
