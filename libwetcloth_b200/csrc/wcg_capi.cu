@@ -298,9 +298,6 @@ int wcg_create(const wcg_params* params, wcg_ctx** out) {
   if (const char* v = getenv("WCG_PCG_LAYOUT")) ctx->c.pcg_layout = !strcmp(v, "tiles") ? 1 : 0;
   // transfer formulation: bucket tiles (default) or the global gathers
   if (const char* v = getenv("WCG_TRANSFERS")) ctx->c.xfer_mode = !strcmp(v, "gather") ? 1 : 0;
-  // the PCG's SpMV: row-parallel (default) or patch-streamed (performance
-  // knob; the dot products' partial sums are grouped differently)
-  if (const char* v = getenv("WCG_SPMV")) ctx->c.spmv_rows = !strcmp(v, "stream") ? 0 : 1;
   // cluster extents of the launch schedule (wcg_schedule): held for
   // wcg_get_schedule, without effect on the sweeps
   ctx->c.sweep_cluster = 0;

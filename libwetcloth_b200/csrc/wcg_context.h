@@ -154,14 +154,14 @@ struct PencilGeom {
   int lo[3];             // low corner of the DOF box (grid cells, physical axes)
   int Ls, NA, NC;        // box extent along s, a, c
   int nPA, nPC;          // patches along a, c
-  int R;                 // rows per patch (Ls + 2 * (patch edge - 1))
+  int R;                 // steps per strip (pairs of a line + patch edge, in whole chunks)
   long long npatch;      // nPA * nPC
-  long long len;         // elements per array (npatch * R * lines per patch)
+  long long len;         // elements per array (npatch * R * 2 * lines per patch)
 };
 
 // Arrays of the pencil layout (Reals, len each; PL64_* are doubles).
-// PL_COEF spans four arrays: the MIC(0) factor interleaved per cell,
-// {1/sqrt(d'), S_s, S_a, S_c}.
+// PL_COEF spans four arrays: the MIC(0) factor, per step of a strip four rows
+// of 64: 1/sqrt(d'), S_s, S_a, S_c.
 enum PlField : int {
   PL_AD = 0, PL_AS, PL_AA, PL_AC, PL_B,        // assembled system
   PL_COEF,                                     // MIC(0) factor (4 arrays)
@@ -252,12 +252,12 @@ struct Context {
   DevBuf pl;                     // kNumPlFields * pl_cap Reals
   DevBuf pl64;                   // kNumPl64Fields * pl_cap doubles
   DevBuf pl_edge;                // tagged edge words
-  DevBuf pl_order;               // patches in wave order (int32)
+  DevBuf pl_order;               // clusters of the sweeps in wave order (int32)
+  int pl_cl = 4;                 // groups per cluster in this solve's sweeps
   // cluster extents of the launch schedule, kept for wcg_get_schedule (the
-  // sweeps run one CTA per patch whatever they say)
+  // sweeps choose their clusters whatever they say)
   int sweep_cluster = 1;
   int sweep_cluster_a = 1;
-  int spmv_rows = 1;             // 0: the patch-streamed SpMV instead of the row-parallel one
   int pcg_batch = 8;             // PCG iterations launched per host convergence check
   DevBuf pl_part;                // per-patch partials (double)
   long long pl_cap = 0;

@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(kRedThreads)
 // (last_block).  Partials are summed thread-strided, then by the block tree,
 // so both forms give the same bits.
 // The tree of block_sum / block_max over kRedThreads values in shared memory,
-// for blocks of at least kRedThreads threads (the first kRedThreads add).
+// for blocks of at least kRedThreads / 2 threads.
 template <typename T>
 __device__ inline T tree_sum(T* sm) {
   __syncthreads();
@@ -515,10 +515,10 @@ __device__ inline T tree_max(T* sm) {
 }
 
 __device__ inline void red_alpha_body(const double* partial, int n, double* sc, double* sm) {
-  if (threadIdx.x < kRedThreads) {
+  for (int t = threadIdx.x; t < kRedThreads; t += blockDim.x) {
     double s = 0;
-    for (int i = threadIdx.x; i < n; i += kRedThreads) s += __ldcg(partial + i);
-    sm[threadIdx.x] = s;
+    for (int i = t; i < n; i += kRedThreads) s += __ldcg(partial + i);
+    sm[t] = s;
   }
   const double s = tree_sum(sm);
   if (threadIdx.x == 0) {
@@ -528,13 +528,13 @@ __device__ inline void red_alpha_body(const double* partial, int n, double* sc, 
 }
 
 __device__ inline void red_conv_body(const double* partial, int n, double* sc, double* sm) {
-  if (threadIdx.x < kRedThreads) {
+  for (int t = threadIdx.x; t < kRedThreads; t += blockDim.x) {
     double m = 0;
-    for (int i = threadIdx.x; i < n; i += kRedThreads) {
+    for (int i = t; i < n; i += kRedThreads) {
       const double v = __ldcg(partial + i);
       m = v > m ? v : m;
     }
-    sm[threadIdx.x] = m;
+    sm[t] = m;
   }
   const double m = tree_max(sm);
   if (threadIdx.x == 0) {
@@ -547,10 +547,10 @@ __device__ inline void red_conv_body(const double* partial, int n, double* sc, d
 
 __device__ inline void red_beta_body(const double* partial, int n, double* sc, double* sm,
                                      int init) {
-  if (threadIdx.x < kRedThreads) {
+  for (int t = threadIdx.x; t < kRedThreads; t += blockDim.x) {
     double s = 0;
-    for (int i = threadIdx.x; i < n; i += kRedThreads) s += __ldcg(partial + i);
-    sm[threadIdx.x] = s;
+    for (int i = t; i < n; i += kRedThreads) s += __ldcg(partial + i);
+    sm[t] = s;
   }
   const double s = tree_sum(sm);
   if (threadIdx.x == 0) {

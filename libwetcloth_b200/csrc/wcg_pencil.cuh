@@ -3,20 +3,23 @@
 // The pressure unknowns of one solve (the bounding box of the DOF cells) are
 // copied once into a layout built for the triangular sweeps.  One grid axis is
 // the stream axis s (the longest extent of the box); the other two (a, c) are
-// cut into patches of 16 x 16 lines.  Line (al, cl) of a patch is skewed by
-// d = al + cl rows: cell (s, a, c) sits at row t = s + d of its patch, and
-// element (patch, t, line) is stored at ((patch * R + t) * 256 + line) with
-// line = al + 16 cl and R = Ls + 30 rows.  Rows outside a line's range and
-// lines outside the box hold zeros.
+// cut into patches of 16 x 16 lines, a patch into 8 strips of 16 x 2 lines.
+// A lane takes the cells of its line in pairs along s, one pair per step.  Line
+// (al, cl) is skewed by al + (cl & 1) steps within its strip w = cl / 2: cell
+// (s, a, c) is element b = s & 1 of the pair at step v = s / 2 + al + (cl & 1),
+// stored at (((patch * 8 + w) * R + v) * 32 + lane) * 2 + b with lane = al +
+// 16 (cl & 1) and R = (Ls + 1) / 2 + 16 steps, rounded up to a whole chunk of 2.
+// Pairs outside a line's range and lines outside the box hold zeros.
 //
-// In this layout every MIC(0) hyperplane dependency is one row back (one row
-// forward for the backward sweep):
-//   (s-1, a, c): row t-1 of the same line
-//   (s, a-1, c): row t-1 of line - 1
-//   (s, a, c-1): row t-1 of line - 16
-// so a CTA takes a patch, one warp per strip of 32 lines, and every strip walks
-// its rows with contiguous loads and stores.  The factor is stored interleaved
-// per cell {1/sqrt(d'), S_s, S_a, S_c} so a sweep reads it with one vector load.
+// In this layout every MIC(0) dependency of a pair is one step back (one step
+// forward for the backward sweep) or inside the pair:
+//   (s-1, a, c): the pair itself, or step v-1 of the same lane
+//   (s, a-1, c): step v-1 of lane - 1 (step v+15 of lane + 15 of the patch below)
+//   (s, a, c-1): step v-1 of lane - 16, or step v+1 of lane + 16 of the strip
+//                before (of the last strip of the patch before along c)
+// so a CTA takes a patch, one warp per strip, and every strip reads and writes
+// one contiguous run of memory.  The factor lies step by step too, four rows of
+// 64 per step: 1/sqrt(d'), S_s, S_a, S_c.
 // Values crossing a patch edge go through a global buffer of tagged 64-bit
 // words, (epoch << 32 | 32 data bits), one word per 32 bits of payload: the
 // consumer re-reads its word until the tag equals the launch's epoch, so no
@@ -44,14 +47,50 @@ namespace wcg {
 
 constexpr int kPatch = 16;                    // lines per patch edge
 constexpr int kPatchLines = kPatch * kPatch;
+constexpr int kStrips = kPatchLines / 32;     // strips of 32 lines per patch
+constexpr int kChunk = 2;                     // steps a strip stages at a time
 constexpr int kPlBlocks = 592;                // streaming kernels: 4 x 148 SMs
-// the fused SpMV in FP32 (32 registers): 8 resident CTAs per SM, so twice the
-// loads in flight of the other streaming kernels
-constexpr int kPlSpmvBlocks32 = 1184;
 static_assert(kRedThreads == kPatchLines, "streaming kernels walk one row per block");
 
-__host__ __device__ inline long long pl_index(const PencilGeom& G, long long p, int t, int l) {
-  return (p * G.R + t) * kPatchLines + l;
+// element of line (al, cl) of patch p at stream position s
+__host__ __device__ inline long long pl_index(const PencilGeom& G, long long p, int s, int al,
+                                              int cl) {
+  const long long step = (p * kStrips + (cl >> 1)) * G.R + ((s >> 1) + al + (cl & 1));
+  return step * 64 + 2 * (al + 16 * (cl & 1)) + (s & 1);
+}
+
+// a lane's pair of cells
+template <typename R>
+struct Pair;
+template <>
+struct Pair<float> {
+  using T = float2;
+};
+template <>
+struct Pair<double> {
+  using T = double2;
+};
+
+// Strips of a sweep CTA.  FP32: a whole patch.  FP64: half a patch, since eight
+// FP64 strips keep one SM's issue slots and shared memory busy (per sweep launch
+// in groups of 8 / 4: 178 / 149 us for the half box at 128^3, 65 / 52 us for the
+// dam break at 64^3; FP32 at 256^3 211 / 260 us, 12 and more warps per SM).
+template <typename R>
+__host__ __device__ constexpr int sweep_group() {
+  return sizeof(R) == 4 ? kStrips : kStrips / 2;
+}
+template <typename R>
+__host__ __device__ constexpr int sweep_threads() {
+  return sweep_group<R>() * 32 + 64;  // strips, then two receiver warps
+}
+// groups of strips in a column of patches, and over the whole box
+template <typename R>
+__host__ __device__ inline int pl_groups(const PencilGeom& G) {
+  return G.nPC * (kStrips / sweep_group<R>());
+}
+template <typename R>
+__host__ __device__ inline int pl_units(const PencilGeom& G) {
+  return G.nPA * pl_groups<R>(G);
 }
 
 // ---- tagged edge words -----------------------------------------------------------
@@ -98,37 +137,24 @@ __device__ inline unsigned smem_u32(const void* p) {
 // the update), coef x4; backward y, r, coef x4.
 __host__ __device__ constexpr int sweep_slot(int mode) { return mode == 0 ? 4 : 6; }
 
-// Words of the edge buffer: entry (patch that writes, face, row, line), EW
-// words each.  face 0: towards the next patch along a (line k = cl), face 1:
-// along c (line k = al); row = the row of the strip that takes the word.
-__host__ __device__ inline long long edge_rows(const PencilGeom& G) { return G.Ls + 15; }
-__device__ inline long long edge_word(const PencilGeom& G, long long p, int face, int row, int k,
-                                      int EW) {
-  return (((p * 2 + face) * edge_rows(G) + row) * kPatch + k) * EW;
+// Words of the edge buffer, EW words per entry.  a-face: entry (patch that
+// writes, step, line cl of the sweep); c-face: (group that writes, step, line
+// al).  step = the step of the strip that wrote it (the strip that takes it does
+// so 15 steps earlier in its own count along a, one along c).
+__host__ __device__ inline long long edge_words(const PencilGeom& G, int units, int EW) {
+  return (G.npatch + units) * G.R * kPatch * EW;
 }
-
-// The MIC(0) factor of a cell, interleaved: {1/sqrt(d'), S_s, S_a, S_c}.
-__device__ inline void ld_coef_shared(const float* p, float* c) {
-  const float4 t = *reinterpret_cast<const float4*>(p);
-  c[0] = t.x; c[1] = t.y; c[2] = t.z; c[3] = t.w;
+__device__ inline long long edge_a(const PencilGeom& G, long long p, int step, int k, int EW) {
+  return ((p * G.R + step) * kPatch + k) * EW;
 }
-__device__ inline void ld_coef_shared(const double* p, double* c) {
-  const double2 a = reinterpret_cast<const double2*>(p)[0];
-  const double2 b = reinterpret_cast<const double2*>(p)[1];
-  c[0] = a.x; c[1] = a.y; c[2] = b.x; c[3] = b.y;
-}
-__device__ inline void st_coef(float* p, float a, float b, float c, float d) {
-  *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
-}
-__device__ inline void st_coef(double* p, double a, double b, double c, double d) {
-  reinterpret_cast<double2*>(p)[0] = make_double2(a, b);
-  reinterpret_cast<double2*>(p)[1] = make_double2(c, d);
+__device__ inline long long edge_c(const PencilGeom& G, long long unit, int step, int k, int EW) {
+  return (((G.npatch + unit) * G.R + step) * kPatch + k) * EW;
 }
 
 template <typename R>
 struct PencilSweepArgs {
   PencilGeom G;
-  const int* order;   // patches in wave order
+  const int* order;   // clusters in wave order: column + nPA * cluster of the column
   int* ticket;
   int ticket_base;    // tickets already handed out this solve
   unsigned epoch;     // tag of this launch's edge words
@@ -138,20 +164,20 @@ struct PencilSweepArgs {
   const R* AS;
   const R* AA;
   const R* AC;
-  R* coef;      // factor: 4 per cell {1/sqrt(d'), S_s, S_a, S_c}
+  R* coef;      // factor: 4 rows of 64 per step, 1/sqrt(d'), S_s, S_a, S_c
   // sweeps
   const R* in;  // forward: r; backward: y
   R* out;       // forward: y; backward: z
   R* r;         // forward (update): r updated in place; backward: r for z.r
   const R* q;   // forward (update)
   double* sc;            // device scalars (the last CTA of a reducing sweep writes them)
-  double* part;  // per-patch partial: forward max|r|, backward z.r
+  double* part;  // per-group partial: forward max|r|, backward z.r
   R omega, min_ratio;
   int* err;
   int* done_ctr;         // with part: the last CTA reduces the partials (forward with
                          // update: max|r| and the stop test; backward: z.r and beta)
   int red_init;          // backward: the first z.r of a solve (beta = 0)
-  int npart;             // partials (patches)
+  int npart;             // partials (groups)
   long long spin_limit;  // polls of an edge word before the wait gives up
   int stale_patch;       // failure-path test: this patch waits for a tag nothing
                          // writes (-1: none)
@@ -161,20 +187,23 @@ struct PencilSweepArgs {
 // r -= alpha q (and reports max|r|); the matching x += alpha s is applied by
 // the next SpMV (k_pl_spmv_s) or, after the last iteration, by k_pl_axpy.
 //
-// A patch is one CTA of 8 strip warps and 2 receiver warps.  Strip w holds the
-// 32 lines cl = 2w and 2w + 1 (lane = al + 16 (cl & 1)) and walks its own rows
-// v = 0 .. Ls + 15 (row t = v + 2w of the patch) without any CTA barrier:
-//   * its row data is copied D rows ahead into a shared-memory ring that only
-//     this warp uses (cp.async, 16 bytes per lane);
+// The strips of one column of patches (all c, one a) form a chain.  A CTA takes
+// a group of consecutive strips of it, one warp each, with two receiver warps; the
+// CTAs of a thread-block cluster take consecutive groups.  A strip walks its R
+// steps (two cells of every line each) without any CTA barrier:
+//   * its cells are copied a few chunks ahead into a shared-memory ring that
+//     only this warp uses (cp.async, 16 bytes per lane: a chunk is contiguous);
 //   * the a-neighbour and the c-neighbour inside the strip come by shuffle of
-//     the previous row's outputs;
-//   * the c-neighbour in strip w - 1 and the values from the patches upstream
-//     along a and c come as tagged 64-bit words (tag << 32 | 32 data bits) in
-//     the strip's inbox in shared memory.  Strip w - 1 writes the c words of
-//     row v - 1 of its own count; the receivers write the rest.
-// Words across a patch face go through a global buffer (tag: the launch's
-// epoch).  The receivers (one warp for the a-face, one for the c-face, two
-// lanes per line: even and odd rows) poll it, up to 8 rows per lane in flight,
+//     the previous step's outputs;
+//   * the c-neighbour in the strip before and the values of the column before
+//     along a come as tagged 64-bit words (tag << 32 | 32 data bits) in the
+//     strip's inbox in shared memory.  The strip before writes the c words of
+//     step v - 1 of its own count, through the cluster's shared memory where it
+//     is in the CTA before; the receivers write the rest.  A step's words are
+//     read a step ahead and read again only where they were not there yet.
+// Words to the next column, and along c out of a cluster, go through a global
+// buffer (tag: the launch's epoch).  The receivers (one warp for the a-face, one for the c-face, two
+// lanes per line: even and odd steps) poll it, up to 4 steps per lane in flight,
 // and move what has arrived into the inboxes, so a strip never waits for a
 // round trip to L2 of its own.  An inbox slot is reused once the strip has
 // published that it took the word (s_prog).  Every wait is bounded.
@@ -182,38 +211,44 @@ struct PencilSweepArgs {
 // The backward sweep is the same walk mirrored: patches, strips, lanes and
 // rows counted from the other end.
 //
-// Bound: the chain of Ls + NA + NC rows that the last cell waits for, then the
-// bytes of a row (forward 8, backward 7 values per cell).  The former CTA of
-// one warp per two lines of c, all eight meeting at a barrier in every row and
-// every face lane polling its own word in L2, took per launch 426 us at 256^3
-// in FP32 (in clusters of 9 along c) where this takes 270; in FP64 287 / 161 us
-// for the half box at 128^3, 105 / 62 us for the dam break at 64^3, 62 / 39 us
-// at 16^3 (all with the events around each launch).
+// Bound: the chain of Ls / 2 + NA + NC steps that the last cell waits for, then
+// the bytes of a step (forward 8, backward 7 values per cell).  A step takes
+// about 500 cycles of a warp in FP32 and 900 in FP64, so it is kept to two cells
+// per lane: with single cells a row took 320-400 and 450-500 and a hop between
+// strips 1500.  Per launch (the events around it included), one CTA barrier per
+// row and every face lane polling L2 / one-cell strips / this: 256^3 half box in
+// FP32 426 / 270 / 213 us; FP64 half box at 128^3 287 / 161 / 138, dam break at
+// 64^3 105 / 62 / 53, at 16^3 62 / 39 / 34.
 //
 // The body takes the launch's CTA count (nblocks) as an argument so a launch
 // over several solves (k_pencil_sweep_batch) can run it per solve.
-constexpr int kStrips = kPatchLines / 32;
-constexpr int kPencilThreads = kPatchLines + 64;  // strips, then two receiver warps
-constexpr int kInC = 16;   // inbox rows of c words (16 per row)
-constexpr int kInA = 32;   // inbox rows of a words (2 per row)
-constexpr int kRecv = 8;   // rows a receiver lane polls at once
+constexpr int kInA = 16;   // inbox steps of a entries (2 per step)
+// inbox steps of c entries (16 per step): as many as shared memory has room for,
+// so that a strip seldom has to look whether the next one took some
+template <typename R>
+__host__ __device__ constexpr int sweep_inc() {
+  return sizeof(R) == 4 ? 16 : 8;
+}
+constexpr int kRecv = 4;   // steps a receiver lane polls at once
 constexpr long long kInboxPolls = 1ll << 24;  // bound of a wait in shared memory
 
+// chunks of a strip in flight or in use (one CTA per SM: 96 KB of FP32 or 144 KB
+// of FP64 cells, enough for the latency of HBM at its full rate)
 template <typename R>
-struct SweepStages {
-  static constexpr int D = sizeof(R) == 4 ? 16 : 8;
+struct SweepSlots {
+  static constexpr int N = sizeof(R) == 4 ? 4 : 3;
 };
 __host__ __device__ constexpr int sweep_words(int mode, size_t rbytes) {
-  return (mode == 0 ? 2 : 1) * (int)(rbytes / 4);  // 64-bit words per edge entry
+  return 2 * (mode == 0 ? 2 : 1) * (int)(rbytes / 4);  // 64-bit words per edge entry
 }
 template <typename R>
 __host__ __device__ constexpr size_t sweep_ring_bytes(int mode) {
-  return (size_t)kStrips * SweepStages<R>::D * sweep_slot(mode) * 32 * sizeof(R);
+  return (size_t)sweep_group<R>() * SweepSlots<R>::N * sweep_slot(mode) * kChunk * 64 * sizeof(R);
 }
 template <typename R>
 __host__ __device__ constexpr size_t sweep_dyn_smem(int mode) {
   return sweep_ring_bytes<R>(mode) +
-         (size_t)kStrips * (kInC * 16 + kInA * 2) * sweep_words(mode, sizeof(R)) * 8;
+         (size_t)sweep_group<R>() * (sweep_inc<R>() * 16 + kInA * 2) * sweep_words(mode, sizeof(R)) * 8;
 }
 
 __device__ inline void cp_async16(unsigned dst, const void* src) {
@@ -251,6 +286,46 @@ __device__ inline void st_words_shared(unsigned addr, const u64* w) {
                    : "memory");
   }
 }
+// the same from the lanes with on != 0 alone, to shared (32-bit address) or
+// global memory (predicated: the lanes of a strip never part)
+template <int EW>
+__device__ inline void st_words_shared_if(int on, unsigned addr, const u64* w) {
+#pragma unroll
+  for (int k = 0; k < EW; k += 2)
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.s32 q, %3, 0;\n @q st.volatile.shared.v2.u64 [%0], {%1, %2};\n}" ::
+            "r"(addr + 8 * k), "l"(w[k]), "l"(w[k + 1]), "r"(on)
+        : "memory");
+}
+template <int EW>
+__device__ inline void st_words_global_if(int on, u64* p, const u64* w) {
+#pragma unroll
+  for (int k = 0; k < EW; k += 2)
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.s32 q, %3, 0;\n @q st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};\n}" ::
+            "l"(p + k), "l"(w[k]), "l"(w[k + 1]), "r"(on)
+        : "memory");
+}
+// nonzero where a tag of the entry is not `tag`
+template <int EW>
+__device__ inline unsigned words_off(const u64* w, unsigned tag) {
+  unsigned off = 0;
+#pragma unroll
+  for (int k = 0; k < EW; ++k) off |= (unsigned)(w[k] >> 32) ^ tag;
+  return off;
+}
+// the value's bits under a mask of all ones or zeros, and (a & m) | b
+__device__ inline float keep(float v, unsigned m) { return __uint_as_float(__float_as_uint(v) & m); }
+__device__ inline double keep(double v, unsigned m) {
+  return __hiloint2double(__double2hiint(v) & (int)m, __double2loint(v) & (int)m);
+}
+__device__ inline float merge(float a, unsigned m, float b) {
+  return __uint_as_float((__float_as_uint(a) & m) | __float_as_uint(b));
+}
+__device__ inline double merge(double a, unsigned m, double b) {
+  return __hiloint2double((__double2hiint(a) & (int)m) | __double2hiint(b),
+                          (__double2loint(a) & (int)m) | __double2loint(b));
+}
 template <int EW>
 __device__ inline bool words_tagged(const u64* w, unsigned tag) {
   bool ok = true;
@@ -267,67 +342,119 @@ __device__ inline void st_volatile_int(unsigned addr, int v) {
   asm volatile("st.volatile.shared.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
-template <typename R, int MODE, bool UPD>
+// thread-block clusters
+__device__ inline int cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return (int)r;
+}
+// every thread of every CTA of the cluster; orders the shared memory each CTA
+// wrote before it against the accesses after it
+__device__ inline void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n"
+               "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// address of the same shared variable in CTA `rank` of the cluster
+__device__ inline unsigned cluster_map(unsigned local, int rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"((unsigned)rank));
+  return r;
+}
+__device__ inline int ld_cluster_int(unsigned addr) {
+  int v;
+  asm volatile("ld.relaxed.cluster.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+template <int EW>
+__device__ inline void st_words_cluster_if(int on, unsigned addr, const u64* w) {
+#pragma unroll
+  for (int k = 0; k < EW; ++k)
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n"
+        " @q st.relaxed.cluster.shared::cluster.u64 [%0], %1;\n}" ::"r"(addr + 8 * k),
+        "l"(w[k]), "r"(on)
+        : "memory");
+}
+
+template <typename R, int MODE, bool UPD, int CL>
 __device__ __forceinline__ void pencil_sweep_run(const PencilSweepArgs<R>& A, int nblocks) {
   constexpr bool BWD = MODE == kBackward;
   constexpr int PW = MODE == kFactor ? 2 : 1;  // values sent across an edge
   constexpr int TW = TagWords<R>::W;
-  constexpr int EW = PW * TW;
+  constexpr int EW = 2 * PW * TW;              // words of an entry: both cells
   static_assert(kFactor == 0 && kForward == 1 && kBackward == 2, "mode numbering");
-  constexpr int D = SweepStages<R>::D;
+  constexpr int NS = SweepSlots<R>::N;
   constexpr int NF = sweep_slot(MODE);
   constexpr bool TWO = MODE == kBackward || UPD;  // two vectors per row
-  constexpr int SLOT = NF * 32;                   // Reals per staged strip row
+  constexpr int SLOT = NF * kChunk * 64;          // Reals per staged chunk
+  using P2 = typename Pair<R>::T;
   constexpr unsigned full = 0xffffffffu;
   __shared__ int s_ticket;
-  __shared__ int s_prog[kStrips];
-  __shared__ double red[kPatchLines];
+  constexpr int kGroup = sweep_group<R>();
+  __shared__ int s_prog[kGroup];
+  __shared__ double red[kRedThreads];
   extern __shared__ __align__(128) unsigned char dsm[];  // strip rings, then the inboxes
   const PencilGeom& G = A.G;
   const int tid = threadIdx.x;
   const int lane = tid & 31, w = tid >> 5;
-  // one ticket per patch, taken even by a launch that returns at once, so the
+  const int rank = CL > 1 ? cluster_rank() : 0;
+  // one ticket per cluster, taken even by a launch that returns at once, so the
   // counter stays in step with the host's base
-  if (tid == 0) s_ticket = atomicAdd(A.ticket, 1) - A.ticket_base;
-  if (*(const int*)(A.sc + S_DONE)) return;  // set by an earlier launch: uniform
+  if (tid == 0 && rank == 0) s_ticket = atomicAdd(A.ticket, 1) - A.ticket_base;
+  // set by an earlier launch, so uniform: the whole cluster returns before any
+  // access to another CTA
+  if (*(const int*)(A.sc + S_DONE)) return;
+  constexpr int kPencilThreads = sweep_threads<R>();
+  constexpr int kInC = sweep_inc<R>();
   constexpr int INBOX = (kInC * 16 + kInA * 2) * EW;  // words per strip
   {
     u64* ib = reinterpret_cast<u64*>(dsm + sweep_ring_bytes<R>(MODE));
-    for (int i = tid; i < kStrips * INBOX; i += kPencilThreads) ib[i] = 0ull;
-    if (tid < kStrips) s_prog[tid] = 0;
+    for (int i = tid; i < kGroup * INBOX; i += kPencilThreads) ib[i] = 0ull;
+    if (tid < kGroup) s_prog[tid] = 0;
   }
-  __syncthreads();
-  const int tk = s_ticket;
+  if (CL > 1) cluster_sync();
+  else __syncthreads();
+  const int tk = CL > 1 ? ld_cluster_int(cluster_map(smem_u32(&s_ticket), 0)) : s_ticket;
+  const int ngroup = pl_groups<R>(G), ncl = (ngroup + CL - 1) / CL;
   bool run = true;
-  if (tk < 0 || tk >= (int)G.npatch) {
+  if (tk < 0 || tk >= G.nPA * ncl) {
     if (tid == 0) record_error(A.err, kErrIndex);
     run = false;
   }
   double rmax = 0, dsum = 0;
-  int p = 0;
+  int col = 0, grp = 0;  // column along a and group along c, in sweep order
   if (run) {
-    p = BWD ? A.order[(int)G.npatch - 1 - tk] : A.order[tk];
-    const int PAi = p % G.nPA, PCi = p / G.nPA;
-    const int Ls = G.Ls;
-    const int NV = Ls + kPatch;            // rows of a strip
-    const int na = Ls + 1, nc = Ls + 15;   // rows that take a-face and c-face words
-    // patches upstream (their words come in) and downstream
-    const int up_a = BWD ? (PAi + 1 < G.nPA ? p + 1 : -1) : (PAi > 0 ? p - 1 : -1);
-    const int up_c = BWD ? (PCi + 1 < G.nPC ? p + G.nPA : -1) : (PCi > 0 ? p - G.nPA : -1);
-    const bool pub_a = BWD ? PAi > 0 : PAi + 1 < G.nPA;
-    const bool pub_c = BWD ? PCi > 0 : PCi + 1 < G.nPC;
+    const int unit = A.order[tk];
+    col = unit % G.nPA;
+    grp = unit / G.nPA * CL + rank;
+    run = grp < ngroup;  // the last cluster of a column may reach past its end
+  }
+  if (run) {
+    const int NV = G.R;
+    const int na = NV - 15, nc = NV - 1;   // steps that take a-face and c-face words
+    const int S0 = grp * kGroup;           // first strip of the group in its column
+    const int PCs = S0 / kStrips;          // its patch along c, in sweep order
+    const int p = BWD ? (G.nPC - 1 - PCs) * G.nPA + (G.nPA - 1 - col) : PCs * G.nPA + col;
+    // upstream: the column before (same strips) and the group before; the groups
+    // of a cluster reach one another through shared memory
+    const bool up_a = col > 0, dn_a = col + 1 < G.nPA;
+    const bool up_c = grp > 0, dn_c = grp + 1 < ngroup;
+    const bool up_near = CL > 1 && rank > 0, dn_near = CL > 1 && dn_c && rank + 1 < CL;
+    const long long unit_id = (long long)grp * G.nPA + col;
     const unsigned inbox0 = smem_u32(dsm + sweep_ring_bytes<R>(MODE));
     const unsigned prog0 = smem_u32(s_prog);
     const unsigned ep = A.epoch;
-    if (w >= kStrips) {
+    if (w >= kGroup) {
       // ---- receivers ----
-      const bool cface = w == kStrips + 1;
-      const int up = cface ? up_c : up_a;
-      if (up >= 0) {
+      const bool cface = w == kGroup + 1;
+      if (cface ? up_c && !up_near : up_a) {
         // the tag this patch waits for: the launch's, except on the patch a
         // failure-path test marks, whose waits then run into their limit
         const unsigned want = p == A.stale_patch ? (ep ^ 0x80000000u) : ep;
-        const int k = lane & 15;                     // line of the face
+        // lanes per line: steps v, v + nl, ... each
+        const int lines = cface ? 16 : 2 * kGroup;
+        const int nl = 32 / lines;
+        const int k = lane % lines;                  // line of the face
         const int strip = cface ? 0 : k >> 1;
         const int rows = cface ? nc : na;
         const unsigned box = inbox0 + (unsigned)(strip * INBOX) * 8u +
@@ -336,8 +463,10 @@ __device__ __forceinline__ void pencil_sweep_run(const PencilSweepArgs<R>& A, in
         const int depth = cface ? kInC : kInA;
         const unsigned pitch = (cface ? 16u : 2u) * EW * 8u;
         const unsigned prog = prog0 + 4u * strip;
-        const u64* src = A.edge + edge_word(G, up, cface ? 1 : 0, 0, k, EW);
-        int v = lane >> 4;  // this lane's next row; rows of one parity
+        const long long up_p = BWD ? p + 1 : p - 1;
+        const u64* src = A.edge + (cface ? edge_c(G, unit_id - G.nPA, 1, k, EW)
+                                         : edge_a(G, up_p, 15, 2 * (S0 % kStrips) + k, EW));
+        int v = lane / lines;  // this lane's next step
         long long idle = 0;
         bool gave_up = false;
         while (__any_sync(full, v < rows)) {
@@ -348,7 +477,7 @@ __device__ __forceinline__ void pencil_sweep_run(const PencilSweepArgs<R>& A, in
           bool mine[kRecv];
 #pragma unroll
           for (int j = 0; j < kRecv; ++j) {
-            const int vj = v + 2 * j;
+            const int vj = v + nl * j;
             mine[j] = j < most && vj < rows && vj < room;
             if (mine[j]) {
 #pragma unroll
@@ -360,7 +489,7 @@ __device__ __forceinline__ void pencil_sweep_run(const PencilSweepArgs<R>& A, in
           bool open = true;
 #pragma unroll
           for (int j = 0; j < kRecv; ++j) {
-            const int vj = v + 2 * j;
+            const int vj = v + nl * j;
             if (mine[j] && gave_up) {
 #pragma unroll
               for (int q = 0; q < EW; ++q) wd[j][q] = (u64)want << 32;
@@ -375,7 +504,7 @@ __device__ __forceinline__ void pencil_sweep_run(const PencilSweepArgs<R>& A, in
               got = j + 1;
             }
           }
-          v += 2 * got;
+          v += nl * got;
           if (got > 0) {
             idle = 0;
           } else if (v < rows && v < room) {
@@ -392,236 +521,283 @@ __device__ __forceinline__ void pencil_sweep_run(const PencilSweepArgs<R>& A, in
       }
     } else {
       // ---- strips ----
-      // mirrored for the backward sweep: strip w walks the physical strip 7 - w
-      // and lane l the physical lane 31 - l, rows from the end
+      // mirrored for the backward sweep: strips, lanes, steps and the cells of a
+      // pair from the end
       const int pl = BWD ? 31 - lane : lane;
-      const int ps = BWD ? kStrips - 1 - w : w;
-      const long long pbase = (long long)p * G.R * kPatchLines + 32 * ps;
-      const int t0 = BWD ? G.R - 1 - 2 * w : 2 * w;
-      constexpr int RS = BWD ? -kPatchLines : kPatchLines;  // element step per row
-      const long long row0 = pbase + (long long)t0 * kPatchLines;
-      R* const ring = reinterpret_cast<R*>(dsm) + (size_t)w * D * SLOT;
-      const unsigned ring0 = smem_u32(ring);
-      // copies of one row: 16 bytes per lane and pass
-      constexpr int RW = 32 * sizeof(R);  // bytes of one strip row
-      constexpr int PR = RW / 16;         // lanes that copy one array's row
-      auto issue = [&](int v) {
-        if (v < NV) {
-          const long long e = row0 + (long long)v * RS;
-          const unsigned dst = ring0 + (unsigned)(v & (D - 1)) * (SLOT * (unsigned)sizeof(R));
-          if (MODE == kFactor) {
-            const R* a4[4] = {A.AD, A.AS, A.AA, A.AC};
+      const int sp = (S0 + w) % kStrips;  // strip of the patch, in sweep order
+      const int ps = BWD ? kStrips - 1 - sp : sp;
+      const long long strip0 = ((long long)p * kStrips + ps) * NV * 64;  // its first element
+      constexpr int RS = BWD ? -64 : 64;                                 // element step per step
+      R* const ring = reinterpret_cast<R*>(dsm) + (size_t)w * NS * SLOT;
+      // Copies of one chunk, 16 bytes per lane and pass.  Slot layout: the
+      // arrays one after the other, each kChunk steps in memory order (the
+      // backward sweep takes them from the last).
+      constexpr int AB = kChunk * 64 * sizeof(R);  // bytes of one array's chunk
+      const long long e00 = strip0 + (BWD ? (long long)(NV - kChunk) * 64 : 0);
+      const unsigned char *g0, *g1, *g2, *g3;
+      if (MODE == kFactor) {
+        g0 = reinterpret_cast<const unsigned char*>(A.AD + e00) + lane * 16;
+        g1 = reinterpret_cast<const unsigned char*>(A.AS + e00) + lane * 16;
+        g2 = reinterpret_cast<const unsigned char*>(A.AA + e00) + lane * 16;
+        g3 = reinterpret_cast<const unsigned char*>(A.AC + e00) + lane * 16;
+      } else {
+        g0 = reinterpret_cast<const unsigned char*>(A.in + e00) + lane * 16;
+        g1 = reinterpret_cast<const unsigned char*>((MODE == kForward ? A.q : A.r) + e00) + lane * 16;
+        g2 = reinterpret_cast<const unsigned char*>(A.coef + 4 * e00) + lane * 16;
+        g3 = nullptr;
+      }
+      int left = NV / kChunk;  // chunks still to copy
+      auto issue = [&](unsigned dst) {
+        if (left > 0) {
+          auto copy = [&](unsigned at, const unsigned char* g, int nbytes) {
 #pragma unroll
-            for (int i = 0; i < 4 * PR / 32; ++i) {
-              const int c = lane + 32 * i;
-              const int arr = c / PR, off = c % PR;
-              const R* s = arr == 0 ? a4[0] : (arr == 1 ? a4[1] : (arr == 2 ? a4[2] : a4[3]));
-              cp_async16(dst + arr * RW + off * 16,
-                         reinterpret_cast<const unsigned char*>(s + e) + off * 16);
-            }
-          } else {
-            // the vectors (one or two rows), then the factor (four rows' worth)
-            const R* v1 = MODE == kForward ? A.q : A.r;
-            if (lane < (TWO ? 2 : 1) * PR) {
-              const R* s = lane < PR ? A.in : v1;
-              const int off = lane % PR;
-              cp_async16(dst + (lane / PR) * RW + off * 16,
-                         reinterpret_cast<const unsigned char*>(s + e) + off * 16);
-            }
-#pragma unroll
-            for (int i = 0; i < PR * 4 / 32; ++i)
-              cp_async16(dst + 2 * RW + (lane + 32 * i) * 16,
-                         reinterpret_cast<const unsigned char*>(A.coef + 4 * e) +
-                             (lane + 32 * i) * 16);
+            for (int i = 0; i < nbytes / 512; ++i) cp_async16(dst + at + i * 512, g + i * 512);
+          };
+          constexpr int CS = BWD ? -AB : AB;
+          copy(0, g0, AB);
+          g0 += CS;
+          if (MODE == kFactor || TWO) {
+            copy(AB, g1, AB);
+            g1 += CS;
           }
+          copy(2 * AB, g2, MODE == kFactor ? AB : 4 * AB);
+          g2 += MODE == kFactor ? CS : 4 * CS;
+          if (MODE == kFactor) {
+            copy(3 * AB, g3, AB);
+            g3 += CS;
+          }
+          --left;
         }
         cp_async_commit();
       };
-      for (int j = 0; j < D; ++j) issue(j);
+      const unsigned ring0 = smem_u32(ring) + lane * 16;
+      constexpr unsigned SB = SLOT * (unsigned)sizeof(R);
+#pragma unroll
+      for (int k = 0; k < NS; ++k) issue(ring0 + k * SB);
 
-      // the words this lane takes: lanes 0..15 the c-face, 16 and 17 the
-      // a-face lines 2w and 2w + 1
-      const bool has_c = w > 0 || up_c >= 0, has_a = up_a >= 0;
-      const int vlim = lane < 16 ? (has_c ? nc : 0) : (lane < 18 && has_a ? na : 0);
-      const unsigned box = inbox0 + (unsigned)(w * INBOX) * 8u;
-      const unsigned wsrc =
-          lane < 16 ? box + (unsigned)(lane * EW) * 8u
-                    : box + (unsigned)((kInC * 16 + (lane & 1)) * EW) * 8u;
-      const int wmask = lane < 16 ? kInC - 1 : kInA - 1;
-      const unsigned wpitch = (lane < 16 ? 16u : 2u) * EW * 8u;
-      // outgoing: lanes 16..31 the c words of row v - 1 of the next strip (or
-      // of the patch downstream), lanes 15 and 31 the a-face words of row v - 15
-      const bool to_box = w + 1 < kStrips;
-      const bool put_c = lane >= 16 && (to_box || pub_c);
-      const bool put_a = (lane & 15) == 15 && pub_a;
-      const unsigned obox = inbox0 + (unsigned)((w + 1) * INBOX) * 8u +
-                            (unsigned)((lane & 15) * EW) * 8u;
-      u64* const gc = A.edge + edge_word(G, p, 1, 0, lane & 15, EW);
-      u64* const ga = A.edge + edge_word(G, p, 0, 0, 2 * w + (lane >> 4), EW);
+      // the entries this lane takes: lanes 0..15 the c-face, lanes 0 and 16 the
+      // a-face lines of the strip (the others read along)
+      const int lim_c = (w > 0 || up_c) && lane < 16 ? nc : 0;
+      const int lim_a = up_a && (lane & 15) == 0 ? na : 0;
+      u64* const box = reinterpret_cast<u64*>(dsm + sweep_ring_bytes<R>(MODE)) + w * INBOX;
+      const unsigned csrc = smem_u32(box + (lane & 15) * EW);
+      const unsigned asrc = smem_u32(box + (kInC * 16 + (lane >> 4)) * EW);
+      constexpr unsigned CP = 16u * EW * 8u, AP = 2u * EW * 8u;  // bytes of an inbox step
+      // outgoing: lanes 16..31 the c entries of step v - 1 of the next strip (in
+      // this CTA, in the next one of the cluster, or beyond it), lanes 15 and 31
+      // the a-face entries
+      const bool last = w + 1 == kGroup;
+      const bool to_box = !last || dn_near;
+      const int put_c = lane >= 16 && (!last || dn_c);
+      const int put_a = (lane & 15) == 15 && dn_a;
+      const unsigned obox0 = smem_u32(box + (last ? -(kGroup - 1) : 1) * INBOX + (lane & 15) * EW);
+      const unsigned obox = CL > 1 && last && dn_near ? cluster_map(obox0, rank + 1) : obox0;
+      // lanes that take the shuffled value along c and along a
+      const unsigned from_c = lane < 16 ? 0u : ~0u, from_a = (lane & 15) == 0 ? 0u : ~0u;
+      u64* gc = A.edge + edge_c(G, unit_id, 0, lane & 15, EW);
+      u64* ga = A.edge + edge_a(G, p, 0, 2 * sp + (lane >> 4), EW);
       const unsigned prog = prog0 + 4u * w;
       const R al_r = (MODE == kForward && UPD) ? (R)A.sc[S_ALPHA] : R(0);
       const R omega = A.omega, min_ratio = A.min_ratio;
-      const long long eb = row0 + pl;
-      R* const pcoef = MODE == kFactor ? A.coef + 4 * eb : nullptr;
-      R* const o_out = MODE == kFactor ? nullptr : A.out + eb;
-      R* const o_r = (MODE == kForward && UPD) ? A.r + eb : nullptr;
-      R carry[PW], prev_a[PW], prev_c[PW], f[NF];
+      const long long eb = strip0 + (BWD ? (long long)(NV - 1) * 64 : 0) + 2 * pl;
+      R* pcoef = MODE == kFactor ? A.coef + 4 * strip0 + 2 * pl : nullptr;
+      R* o_out = MODE == kFactor ? nullptr : A.out + eb;
+      R* o_r = (MODE == kForward && UPD) ? A.r + eb : nullptr;
+      // prev_*: the previous step's outputs, [cell][value]; cells in sweep order
+      R carry[PW], prev_a[2][PW], prev_c[2][PW];
 #pragma unroll
-      for (int k = 0; k < PW; ++k) carry[k] = prev_a[k] = prev_c[k] = R(0);
+      for (int k = 0; k < PW; ++k)
+        carry[k] = prev_a[0][k] = prev_a[1][k] = prev_c[0][k] = prev_c[1][k] = R(0);
       R rm = 0;
       bool gave_up = false;
-      u64 wd[EW];
-      auto load_row = [&](int v) {
-        const R* S = ring + (size_t)(v & (D - 1)) * SLOT;
+      // a step's values, cells in sweep order (the backward sweep takes the
+      // second cell of a pair first)
+      auto load_step = [&](int slot, int j, R (&f)[2][NF]) {
+        const R* S = ring + slot * SLOT;
+        const int at = (BWD ? kChunk - 1 - j : j) * 64 + 2 * pl;
+        constexpr int B0 = BWD ? 1 : 0, B1 = BWD ? 0 : 1;
+        auto pair = [&](int off, int k) {
+          const P2 t = *reinterpret_cast<const P2*>(S + off);
+          f[B0][k] = t.x;
+          f[B1][k] = t.y;
+        };
+        pair(at, 0);
         if (MODE == kFactor) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) f[k] = S[32 * k + pl];
+          for (int k = 1; k < 4; ++k) pair(k * kChunk * 64 + at, k);
         } else {
-          f[0] = S[pl];
-          if (TWO) f[NF - 1] = S[32 + pl];
-          ld_coef_shared(S + 64 + 4 * pl, f + 1);
+          if (TWO) pair(kChunk * 64 + at, NF - 1);
+          const int ac = 2 * kChunk * 64 + (BWD ? kChunk - 1 - j : j) * 256 + 2 * pl;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) pair(ac + 64 * k, 1 + k);
         }
       };
-      cp_async_wait<D - 1>();
+      u64 wc[EW], wa[EW];
+      auto load_words = [&](int v) {
+        ld_words_shared<EW>(csrc + (unsigned)(v & (kInC - 1)) * CP, wc);
+        ld_words_shared<EW>(asrc + (unsigned)(v & (kInA - 1)) * AP, wa);
+      };
+      auto step = [&](int v, const R (&f)[2][NF], unsigned oc, int j) __attribute__((always_inline)) {
+        // all ones where the lane takes an entry of this step
+        const unsigned mc = (unsigned)((v - lim_c) >> 31), ma = (unsigned)((v - lim_a) >> 31);
+        const unsigned tag = (unsigned)(v + 1);
+        unsigned off = (words_off<EW>(wc, tag) & mc) | (words_off<EW>(wa, tag) & ma);
+        if (__any_sync(full, off != 0)) {
+          long long it = 0;
+          do {
+            load_words(v);
+            off = (words_off<EW>(wc, tag) & mc) | (words_off<EW>(wa, tag) & ma);
+            if (++it > kInboxPolls) {
+              if (lane == 0) record_error(A.err, kErrWaitTimeout);
+              gave_up = true;
+            }
+          } while (__any_sync(full, off != 0) && !gave_up);
+        }
+        R in_a[2][PW], in_c[2][PW];
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+          for (int k = 0; k < PW; ++k) {
+            const R sa = __shfl_up_sync(full, prev_a[b][k], 1);
+            const R sc = __shfl_up_sync(full, prev_c[b][k], 16);
+            in_a[b][k] = merge(sa, from_a, keep(TagWords<R>::unpack(wa + (b * PW + k) * TW), ma));
+            in_c[b][k] = merge(sc, from_c, keep(TagWords<R>::unpack(wc + (b * PW + k) * TW), mc));
+          }
+        // the next step's words, read early; taken once their tag is right
+        load_words(v + 1);
+        P2 o2, r2;       // in memory order
+        R cf[2][4];      // the factor's coefficients
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          R out_s[PW], out_a[PW], out_c[PW];
+          if (MODE == kFactor) {
+            const R ad = f[b][0];
+            R d = ad;
+            R iv = R(0);
+            if (ad != R(0)) {
+              d = d - in_c[b][0] * in_c[b][0];
+              d = d - (omega * in_c[b][0]) * in_c[b][PW - 1];
+              d = d - in_a[b][0] * in_a[b][0];
+              d = d - (omega * in_a[b][0]) * in_a[b][PW - 1];
+              d = d - carry[0] * carry[0];
+              d = d - (omega * carry[0]) * carry[PW - 1];
+              const R piv = d < min_ratio * ad ? ad : d;
+              iv = R(1) / sqrt(piv);
+            }
+            const R ss = f[b][1] * iv, sa = f[b][2] * iv, scv = f[b][3] * iv;
+            cf[b][0] = iv; cf[b][1] = ss; cf[b][2] = sa; cf[b][3] = scv;
+            out_s[0] = ss; out_s[PW - 1] = sa + scv;
+            out_a[0] = sa; out_a[PW - 1] = ss + scv;
+            out_c[0] = scv; out_c[PW - 1] = ss + sa;
+          } else if (MODE == kForward) {
+            R rv = f[b][0];
+            if (UPD) {
+              rv = rv - al_r * f[b][NF - 1];
+              if (b == 0) r2.x = rv;
+              else r2.y = rv;
+              const R av = fabs(rv);
+              rm = av > rm ? av : rm;
+            }
+            R vv = rv;
+            vv -= in_c[b][0];
+            vv -= in_a[b][0];
+            vv -= carry[0];
+            const R y = vv * f[b][1];
+            if (b == 0) o2.x = y;
+            else o2.y = y;
+            out_s[0] = f[b][2] * y;
+            out_a[0] = f[b][3] * y;
+            out_c[0] = f[b][NF - 2] * y;
+          } else {
+            R vv = f[b][0];
+            vv -= f[b][2] * carry[0];
+            vv -= f[b][3] * in_a[b][0];
+            vv -= f[b][NF - 2] * in_c[b][0];
+            const R z = vv * f[b][1];
+            if (b == 0) o2.y = z;
+            else o2.x = z;
+            dsum += (double)z * (double)f[b][NF - 1];
+            out_s[0] = out_a[0] = out_c[0] = z;
+          }
+#pragma unroll
+          for (int k = 0; k < PW; ++k) {
+            prev_a[b][k] = out_a[k];
+            prev_c[b][k] = out_c[k];
+            carry[k] = out_s[k];
+          }
+        }
+        u64 o[EW];
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+          for (int k = 0; k < PW; ++k)
+            TagWords<R>::pack(prev_c[b][k], to_box ? (unsigned)v : ep, o + (b * PW + k) * TW);
+        if (!last) st_words_shared_if<EW>(put_c, oc, o);
+        else if (CL > 1 && dn_near) st_words_cluster_if<EW>(put_c, oc, o);
+        else st_words_global_if<EW>(put_c, gc + j * (16 * EW), o);
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+          for (int k = 0; k < PW; ++k)
+            TagWords<R>::pack(prev_a[b][k], ep, o + (b * PW + k) * TW);
+        st_words_global_if<EW>(put_a, ga + j * (16 * EW), o);
+        if (MODE == kFactor) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            P2 t;
+            t.x = cf[0][k];
+            t.y = cf[1][k];
+            *reinterpret_cast<P2*>(pcoef + j * 256 + 64 * k) = t;
+          }
+        } else {
+          *reinterpret_cast<P2*>(o_out + j * RS) = o2;
+        }
+        if (MODE == kForward && UPD) *reinterpret_cast<P2*>(o_r + j * RS) = r2;
+      };
+      int slot = 0;
+      R f0[2][NF], f1[2][NF];
+      cp_async_wait<NS - 1>();
       __syncwarp();
-      load_row(0);
-      ld_words_shared<EW>(wsrc, wd);
-      int room = kInC;  // rows the next strip's inbox can take
-#pragma unroll 2
-      for (int v = 0; v < NV; ++v) {
-        // this row's incoming words
-        {
-          const bool need = v < vlim;
-          const unsigned tag = (unsigned)(v + 1);
-          bool ok = !need || words_tagged<EW>(wd, tag);
-          if (!__all_sync(full, ok)) {
-            long long it = 0;
-            while (!__all_sync(full, ok) && !gave_up) {
-              if (!ok) {
-                ld_words_shared<EW>(wsrc + (unsigned)(v & wmask) * wpitch, wd);
-                ok = words_tagged<EW>(wd, tag);
-              }
-              if (++it > kInboxPolls) {
-                if (lane == 0) record_error(A.err, kErrWaitTimeout);
-                gave_up = true;
-              }
+      load_step(0, 0, f0);
+      load_words(0);
+      const unsigned next_prog = last ? (CL > 1 && dn_near ? cluster_map(prog0, rank + 1) : prog)
+                                      : prog0 + 4u * (w + 1);
+      auto look = [&]() {
+        return CL > 1 && last && dn_near ? ld_cluster_int(next_prog) : ld_volatile_int(next_prog);
+      };
+      int taken = 0;  // steps the next strip had taken when last looked at
+      for (int v0 = 0; v0 < NV; v0 += 2) {
+        load_step(slot, 1, f1);
+        if (to_box && v0 >= taken + kInC && !gave_up) {
+          // the next strip has to take its steps first
+          long long it = 0;
+          while (v0 >= (taken = look()) + kInC) {
+            if (++it > kInboxPolls) {
+              if (lane == 0) record_error(A.err, kErrWaitTimeout);
+              gave_up = true;
+              break;
             }
           }
         }
-        R in_a[PW], in_c[PW];
-        {
-          R word[PW];
-#pragma unroll
-          for (int k = 0; k < PW; ++k) {
-            word[k] = v < vlim ? TagWords<R>::unpack(wd + k * TW) : R(0);
-            const R wa = __shfl_sync(full, word[k], 16 + (lane >> 4));
-            const R sa = __shfl_up_sync(full, prev_a[k], 1);
-            const R sc = __shfl_up_sync(full, prev_c[k], 16);
-            in_a[k] = (lane & 15) == 0 ? wa : sa;
-            in_c[k] = lane < 16 ? word[k] : sc;
-          }
-        }
-        // the next row's words, read early; taken once their tag is right
-        ld_words_shared<EW>(wsrc + (unsigned)((v + 1) & wmask) * wpitch, wd);
-        if ((v & 3) == 3 && lane == 0) st_volatile_int(prog, v + 1);
-        const long long off = (long long)v * RS;
-        R out_s[PW], out_a[PW], out_c[PW];
-        if (MODE == kFactor) {
-          const R ad = f[0];
-          R d = ad;
-          R iv = R(0);
-          if (ad != R(0)) {
-            d = d - in_c[0] * in_c[0];
-            d = d - (omega * in_c[0]) * in_c[PW - 1];
-            d = d - in_a[0] * in_a[0];
-            d = d - (omega * in_a[0]) * in_a[PW - 1];
-            d = d - carry[0] * carry[0];
-            d = d - (omega * carry[0]) * carry[PW - 1];
-            const R piv = d < min_ratio * ad ? ad : d;
-            iv = R(1) / sqrt(piv);
-          }
-          const R ss = f[1] * iv, sa = f[2] * iv, scv = f[3] * iv;
-          st_coef(pcoef + 4 * off, iv, ss, sa, scv);
-          out_s[0] = ss; out_s[PW - 1] = sa + scv;
-          out_a[0] = sa; out_a[PW - 1] = ss + scv;
-          out_c[0] = scv; out_c[PW - 1] = ss + sa;
-        } else if (MODE == kForward) {
-          R rv = f[0];
-          if (UPD) {
-            rv = rv - al_r * f[NF - 1];
-            o_r[off] = rv;
-            const R av = fabs(rv);
-            rm = av > rm ? av : rm;
-          }
-          R vv = rv;
-          vv -= in_c[0];
-          vv -= in_a[0];
-          vv -= carry[0];
-          const R y = vv * f[1];
-          o_out[off] = y;
-          out_s[0] = f[2] * y;
-          out_a[0] = f[3] * y;
-          out_c[0] = f[NF - 2] * y;
-        } else {
-          R vv = f[0];
-          vv -= f[2] * carry[0];
-          vv -= f[3] * in_a[0];
-          vv -= f[NF - 2] * in_c[0];
-          const R z = vv * f[1];
-          o_out[off] = z;
-          dsum += (double)z * (double)f[NF - 1];
-          out_s[0] = out_a[0] = out_c[0] = z;
-        }
-        // c words of row v - 1 downstream
-        if (to_box) {
-          if (v >= room + 1) {
-            // the next strip has to take a row first
-            long long it = 0;
-            const unsigned np = prog0 + 4u * (w + 1);
-            do {
-              room = ld_volatile_int(np) + kInC;
-              if (++it > kInboxPolls) {
-                if (lane == 0) record_error(A.err, kErrWaitTimeout);
-                gave_up = true;
-                room = 1 << 30;
-              }
-            } while (v >= room + 1);
-          }
-          if (put_c && v > 0) {
-            u64 o[EW];
-#pragma unroll
-            for (int k = 0; k < PW; ++k) TagWords<R>::pack(out_c[k], (unsigned)v, o + k * TW);
-            st_words_shared<EW>(obox + (unsigned)((v - 1) & (kInC - 1)) * (16u * EW * 8u), o);
-          }
-        } else if (put_c && v > 0) {
-          u64 o[EW];
-#pragma unroll
-          for (int k = 0; k < PW; ++k) TagWords<R>::pack(out_c[k], ep, o + k * TW);
-#pragma unroll
-          for (int k = 0; k < EW; ++k)
-            st_relaxed_u64(gc + (long long)(v - 1) * (16 * EW) + k, o[k]);
-        }
-        if (put_a && v >= kPatch - 1) {
-          u64 o[EW];
-#pragma unroll
-          for (int k = 0; k < PW; ++k) TagWords<R>::pack(out_a[k], ep, o + k * TW);
-#pragma unroll
-          for (int k = 0; k < EW; ++k)
-            st_relaxed_u64(ga + (long long)(v - (kPatch - 1)) * (16 * EW) + k, o[k]);
-        }
-#pragma unroll
-        for (int k = 0; k < PW; ++k) {
-          prev_a[k] = out_a[k];
-          prev_c[k] = out_c[k];
-          carry[k] = out_s[k];
-        }
-        // every lane has read row v (the shuffles above follow its loads), so
-        // its slot takes row v + D
+        // the c entries go to steps v0 - 1 and v0 of the next strip's inbox
+        // (step -1: the last slot with tag 0, which nothing takes), or to steps
+        // v0 and v0 + 1 of the patch's own face
+        step(v0, f0, obox + (unsigned)((v0 - 1) & (kInC - 1)) * CP, 0);
+        // every lane holds this chunk's values: its slot takes a later one
         __syncwarp();
-        issue(v + D);
-        cp_async_wait<D - 1>();
+        issue(ring0 + slot * SB);
+        slot = slot + 1 == NS ? 0 : slot + 1;
+        taken = look();
+        cp_async_wait<NS - 1>();
         __syncwarp();
-        if (v + 1 < NV) load_row(v + 1);
+        if (v0 + 2 < NV) load_step(slot, 0, f0);
+        step(v0 + 1, f1, obox + (unsigned)(v0 & (kInC - 1)) * CP, 1);
+        st_volatile_int(prog, v0 + 2);  // (every lane the same)
+        gc += 2 * 16 * EW;
+        ga += 2 * 16 * EW;
+        if (MODE == kFactor) pcoef += 2 * 256;
+        else o_out += 2 * RS;
+        if (MODE == kForward && UPD) o_r += 2 * RS;
       }
       if (lane == 0) st_volatile_int(prog, 1 << 29);  // nothing waits for this strip any more
       cp_async_wait<0>();
@@ -630,15 +806,17 @@ __device__ __forceinline__ void pencil_sweep_run(const PencilSweepArgs<R>& A, in
   }
   // partials, summed in line order whatever the direction
   if (A.part && ((MODE == kForward && UPD) || MODE == kBackward)) {
-    const int line = BWD ? kPatchLines - 1 - tid : tid;
-    if (tid < kPatchLines) red[line] = MODE == kForward ? rmax : dsum;
+    constexpr int NL = kGroup * 32;
+    for (int i = tid; i < kRedThreads; i += kPencilThreads) red[i] = 0;
     __syncthreads();
+    if (tid < NL) red[BWD ? NL - 1 - tid : tid] = MODE == kForward ? rmax : dsum;
+    const int at = (BWD ? ngroup - 1 - grp : grp) * G.nPA + (BWD ? G.nPA - 1 - col : col);
     if (MODE == kForward) {
       const double m = tree_max(red);
-      if (tid == 0 && run) A.part[p] = m;
+      if (tid == 0 && run) A.part[at] = m;
     } else {
       const double sm = tree_sum(red);
-      if (tid == 0 && run) A.part[p] = sm;
+      if (tid == 0 && run) A.part[at] = sm;
     }
     // every CTA counts, running or not; the last one reduces the partials
     if (A.done_ctr && last_block(A.done_ctr, nblocks)) {
@@ -648,12 +826,14 @@ __device__ __forceinline__ void pencil_sweep_run(const PencilSweepArgs<R>& A, in
         red_beta_body(A.part, A.npart, A.sc, red, A.red_init);
     }
   }
+  // no CTA leaves while another may write to its inbox or look at its progress
+  if (CL > 1) cluster_sync();
 }
 
-template <typename R, int MODE, bool UPD>
-__global__ void __launch_bounds__(kPencilThreads, 1)
+template <typename R, int MODE, bool UPD, int CL>
+__global__ void __launch_bounds__(sweep_threads<R>(), 1)
     k_pencil_sweep(const PencilSweepArgs<R> A) {
-  pencil_sweep_run<R, MODE, UPD>(A, (int)gridDim.x);
+  pencil_sweep_run<R, MODE, UPD, CL>(A, (int)gridDim.x);
 }
 
 // The solve of block b in a launch over several solves: first[] holds each
@@ -670,20 +850,20 @@ __device__ inline int batch_solve_of(const int* __restrict__ first, int n, int b
 }
 
 // One sweep launch over several solves (the shared solve of a batch of
-// scenes): solve s owns first[s + 1] - first[s] CTAs (its patches) and its
+// scenes): solve s owns first[s + 1] - first[s] CTAs (whole clusters) and its
 // arguments come from tab[s].  Launch k of a chunk advances each solve's
-// edge-word epoch by k and its ticket base by k launches of its patches, as k
+// edge-word epoch by k and its ticket base by k launches of its clusters, as k
 // separate launches would.
-template <typename R, int MODE, bool UPD>
-__global__ void __launch_bounds__(kPencilThreads, 1)
+template <typename R, int MODE, bool UPD, int CL>
+__global__ void __launch_bounds__(sweep_threads<R>(), 1)
     k_pencil_sweep_batch(const PencilSweepArgs<R>* __restrict__ tab, const int* __restrict__ first,
                          int nsolve, int k) {
   const int s = batch_solve_of(first, nsolve, (int)blockIdx.x);
   PencilSweepArgs<R> A = tab[s];
   const int nb = __ldg(first + s + 1) - __ldg(first + s);
   A.epoch += (unsigned)k;
-  A.ticket_base += k * nb;
-  pencil_sweep_run<R, MODE, UPD>(A, nb);
+  A.ticket_base += k * (nb / CL);
+  pencil_sweep_run<R, MODE, UPD, CL>(A, nb);
 }
 
 // x += alpha s (the update of the last PCG iteration, which no SpMV follows)
@@ -697,29 +877,44 @@ __global__ void k_pl_axpy(long long len, const double* __restrict__ sc, const R*
 }
 
 // ---- streaming kernels over the pencil layout --------------------------------
-// Element e -> (patch, row, line) and the cell's position in the box.
+// Element e -> (patch, strip, step, lane, cell) and the position in the box.
 struct PlCell {
-  long long p;
-  int t, l, al, cl, PAi, PCi, s;
+  int p, w, al, cl, PAi, PCi, s;
   bool live;
 };
 
-// Cell of line l in row `row` (= patch * R + t) of the layout; 32-bit math
-// (npatch * R stays far below 2^31).
-__device__ inline PlCell pl_cell(const PencilGeom& G, int row, int l) {
+__device__ inline PlCell pl_cell(const PencilGeom& G, long long e) {
   PlCell c;
-  const int p = row / G.R;
-  c.p = p;
-  c.t = row - p * G.R;
-  c.l = l;
-  c.al = l & (kPatch - 1);
-  c.cl = l / kPatch;
-  c.PAi = p % G.nPA;
-  c.PCi = p / G.nPA;
-  c.s = c.t - c.al - c.cl;
+  const int row = (int)(e >> 6), lane = (int)(e >> 1) & 31;  // npatch * 8 * R far below 2^31
+  const int strip = row / G.R;
+  const int v = row - strip * G.R;
+  c.p = strip / kStrips;
+  c.w = strip - c.p * kStrips;
+  c.al = lane & (kPatch - 1);
+  c.cl = 2 * c.w + (lane >> 4);
+  c.PAi = c.p % G.nPA;
+  c.PCi = c.p / G.nPA;
+  c.s = 2 * (v - c.al - (lane >> 4)) + (int)(e & 1);
   c.live = c.s >= 0 && c.s < G.Ls && c.PAi * kPatch + c.al < G.NA &&
            c.PCi * kPatch + c.cl < G.NC;
   return c;
+}
+
+// Element offsets from a cell to its neighbours outside its strip: the
+// c-neighbour (-c for the 16 lanes of even cl, +c for those of odd cl) sits one
+// strip on, the a-neighbour across the patch face (al = 0: -a, al = 15: +a) in
+// the same strip of the next patch.
+__device__ inline long long pl_out_c(const PencilGeom& G, int w, bool minus) {
+  // strips of consecutive patches along c are nPA patches apart
+  const long long rows = (long long)G.R * 64;
+  const long long far = ((long long)G.nPA * kStrips - (kStrips - 1)) * rows;
+  if (minus) return -(w > 0 ? rows : far) + 64 + 32;
+  return (w + 1 < kStrips ? rows : far) - 64 - 32;
+}
+__device__ inline long long pl_out_a(const PencilGeom& G, bool minus) {
+  const long long patch = (long long)kStrips * G.R * 64;
+  const long long step = (kPatch - 1) * 64 + (kPatch - 1) * 2;
+  return minus ? -patch + step : patch - step;
 }
 
 // Indices of the six neighbours of a live cell (-1 where the box ends).
@@ -729,124 +924,57 @@ struct PlNbr {
 
 __device__ inline PlNbr pl_nbr(const PencilGeom& G, const PlCell& c, long long e) {
   PlNbr n;
-  n.ms = c.s > 0 ? e - kPatchLines : -1;
-  n.ps = c.s + 1 < G.Ls ? e + kPatchLines : -1;
-  if (c.al > 0) n.ma = e - kPatchLines - 1;
-  else n.ma = c.PAi > 0 ? pl_index(G, c.p - 1, c.t + kPatch - 1, c.l + kPatch - 1) : -1;
-  if (c.al < kPatch - 1) n.pa = e + kPatchLines + 1;
-  else n.pa = c.PAi + 1 < G.nPA ? pl_index(G, c.p + 1, c.t - (kPatch - 1), c.l - (kPatch - 1)) : -1;
-  if (c.cl > 0) n.mc = e - kPatchLines - kPatch;
-  else n.mc = c.PCi > 0 ? pl_index(G, c.p - G.nPA, c.t + kPatch - 1,
-                                    c.l + kPatch * (kPatch - 1)) : -1;
-  if (c.cl < kPatch - 1) n.pc = e + kPatchLines + kPatch;
-  else n.pc = c.PCi + 1 < G.nPC ? pl_index(G, c.p + G.nPA, c.t - (kPatch - 1),
-                                            c.l - kPatch * (kPatch - 1)) : -1;
+  n.ms = c.s > 0 ? (c.s & 1 ? e - 1 : e - 63) : -1;
+  n.ps = c.s + 1 < G.Ls ? (c.s & 1 ? e + 63 : e + 1) : -1;
+  if (c.al > 0) n.ma = e - 66;
+  else n.ma = c.PAi > 0 ? e + pl_out_a(G, true) : -1;
+  if (c.al < kPatch - 1) n.pa = e + 66;
+  else n.pa = c.PAi + 1 < G.nPA ? e + pl_out_a(G, false) : -1;
+  if (c.cl & 1) n.mc = e - 96;
+  else n.mc = c.cl > 0 || c.PCi > 0 ? e + pl_out_c(G, c.w, true) : -1;
+  if (!(c.cl & 1)) n.pc = e + 96;
+  else n.pc = c.cl < kPatch - 1 || c.PCi + 1 < G.nPC ? e + pl_out_c(G, c.w, false) : -1;
   return n;
 }
 
-// s_new = z + beta s_old (at all 7 stencil points), q = A s_new,
-// partial[block] = sum s_new.q.  Row order of the reference's sorted row for
-// interior cells: -c, -a, -s, diagonal, +s, +a, +c.
+// s_new = z + beta s_old, q = A s_new, partial[block] = sum s_new.q.  Row order
+// of the reference's sorted row for interior cells: -c, -a, -s, diagonal, +s,
+// +a, +c.
 //
 // The previous iteration's x += alpha s_old is applied here too (alpha is
 // still the previous iteration's when this kernel runs; 0 before the first).
 //
-// Block bid of nblk: the arithmetic of k_pl_spmv_s (below) for one solve of a
-// launch over several solves (k_pl_spmv_batch).
-template <typename R>
-__device__ __forceinline__ void pl_spmv_run(
-    const PencilGeom& G, const R* __restrict__ AD, const R* __restrict__ AS,
-    const R* __restrict__ AA, const R* __restrict__ AC, const R* __restrict__ z,
-    const R* __restrict__ sold, R* __restrict__ snew, R* __restrict__ q, R* __restrict__ x,
-    double* __restrict__ sc, double* __restrict__ partial, int* __restrict__ done_ctr, int bid,
-    int nblk) {
-  __shared__ double sm[kRedThreads];
-  if (*(const int*)(sc + S_DONE)) return;
-  const R be = (R)sc[S_BETA];
-  const R al = (R)sc[S_ALPHA];
-  double acc = 0;
-  const int nrow = (int)(G.npatch * G.R);
-  for (int row = bid; row < nrow; row += nblk) {
-    const long long e = (long long)row * kPatchLines + threadIdx.x;
-    const PlCell c = pl_cell(G, row, threadIdx.x);
-    if (!c.live) continue;
-    const PlNbr n = pl_nbr(G, c, e);
-    R r = 0;
-    if (n.mc >= 0) r += AC[n.mc] * (z[n.mc] + be * sold[n.mc]);
-    if (n.ma >= 0) r += AA[n.ma] * (z[n.ma] + be * sold[n.ma]);
-    if (n.ms >= 0) r += AS[n.ms] * (z[n.ms] + be * sold[n.ms]);
-    const R so = sold[e];
-    x[e] = x[e] + al * so;
-    const R sn = z[e] + be * so;
-    r += AD[e] * sn;
-    if (n.ps >= 0) r += AS[e] * (z[n.ps] + be * sold[n.ps]);
-    if (n.pa >= 0) r += AA[e] * (z[n.pa] + be * sold[n.pa]);
-    if (n.pc >= 0) r += AC[e] * (z[n.pc] + be * sold[n.pc]);
-    snew[e] = sn;
-    q[e] = r;
-    acc += (double)sn * (double)r;
-  }
-  acc = block_sum<double>(acc, sm);
-  if (threadIdx.x == 0) partial[bid] = acc;
-  // the last block: alpha = rho / s.q (k_red_alpha's body)
-  if (done_ctr && last_block(done_ctr, nblk)) red_alpha_body(partial, nblk, sc, sm);
+// Bound by memory: 10 values per cell (z, s_old, four coefficients and x in;
+// s_new, q and x out).  A block takes a chunk of steps of one patch, warp w its
+// strip w, and walks them in order, a pair of cells per lane: s_new of the steps
+// before, at and after the current one and the couplings of the step before
+// stay in registers, and neighbours inside the strip come by shuffle, so a value
+// is loaded once by its own strip.  Only the c-neighbours in the strips beside
+// it (half the lanes each way, the same steps of the same block: L1) and the
+// neighbours across a patch face are loaded again.  The
+// former kernel, one row per block and every neighbour loaded, read each value
+// of z and s_old seven times through L1 and three times through L2: 139 us an
+// iteration at 256^3 in FP32, 104 here (67 at the copy rate).
+constexpr int kSpmvSteps = 8;    // steps of a strip per block, at most
+constexpr int kSpmvStepsMin = 2;
+
+struct SpmvGrid {
+  int steps, nchunk, blocks;
+};
+// Steps per block: 8 blocks per SM before a block takes more than kSpmvStepsMin
+// (a chunk also reads the step before and after it, from L2), at most
+// kSpmvSteps.  A solve alone and in a launch over several solves use the same
+// count, so their partial sums are the same.
+__host__ __device__ inline SpmvGrid pl_spmv_grid(const PencilGeom& G) {
+  SpmvGrid g;
+  long long n = (G.npatch * G.R + 1183) / 1184;
+  n = n < kSpmvStepsMin ? kSpmvStepsMin : (n > kSpmvSteps ? kSpmvSteps : n);
+  g.nchunk = (int)((G.R + n - 1) / n);
+  g.steps = (int)((G.R + g.nchunk - 1) / g.nchunk);
+  g.blocks = (int)(G.npatch * g.nchunk);
+  return g;
 }
 
-// (written out rather than through pl_spmv_run: the launch alone ran about
-// 10 % slower through the shared body)
-template <typename R>
-__global__ void __launch_bounds__(kRedThreads, sizeof(R) == 4 ? 8 : 4)
-    k_pl_spmv_s(PencilGeom G, const R* __restrict__ AD, const R* __restrict__ AS,
-                const R* __restrict__ AA, const R* __restrict__ AC, const R* __restrict__ z,
-                const R* __restrict__ sold, R* __restrict__ snew, R* __restrict__ q,
-                R* __restrict__ x, double* __restrict__ sc,
-                double* __restrict__ partial, int* __restrict__ done_ctr) {
-  __shared__ double sm[kRedThreads];
-  if (*(const int*)(sc + S_DONE)) return;
-  const R be = (R)sc[S_BETA];
-  const R al = (R)sc[S_ALPHA];
-  double acc = 0;
-  const int nrow = (int)(G.npatch * G.R);
-  for (int row = blockIdx.x; row < nrow; row += gridDim.x) {
-    const long long e = (long long)row * kPatchLines + threadIdx.x;
-    const PlCell c = pl_cell(G, row, threadIdx.x);
-    if (!c.live) continue;
-    const PlNbr n = pl_nbr(G, c, e);
-    R r = 0;
-    if (n.mc >= 0) r += AC[n.mc] * (z[n.mc] + be * sold[n.mc]);
-    if (n.ma >= 0) r += AA[n.ma] * (z[n.ma] + be * sold[n.ma]);
-    if (n.ms >= 0) r += AS[n.ms] * (z[n.ms] + be * sold[n.ms]);
-    const R so = sold[e];
-    x[e] = x[e] + al * so;
-    const R sn = z[e] + be * so;
-    r += AD[e] * sn;
-    if (n.ps >= 0) r += AS[e] * (z[n.ps] + be * sold[n.ps]);
-    if (n.pa >= 0) r += AA[e] * (z[n.pa] + be * sold[n.pa]);
-    if (n.pc >= 0) r += AC[e] * (z[n.pc] + be * sold[n.pc]);
-    snew[e] = sn;
-    q[e] = r;
-    acc += (double)sn * (double)r;
-  }
-  acc = block_sum<double>(acc, sm);
-  if (threadIdx.x == 0) partial[blockIdx.x] = acc;
-  // the last block: alpha = rho / s.q (k_red_alpha's body)
-  if (done_ctr && last_block(done_ctr, (int)gridDim.x))
-    red_alpha_body(partial, (int)gridDim.x, sc, sm);
-}
-
-// Blocks of k_pl_spmv_s for a layout: about four rows per block, at most the
-// resident capacity (kPlSpmvBlocks32).  The partial sums of s.q follow the
-// block count, so a solve alone and in a launch over several solves use this
-// same count and give the same bits.
-__host__ __device__ inline int pl_spmv_blocks(const PencilGeom& G) {
-  const long long nrow = G.npatch * G.R;
-  const long long b = (nrow + 3) / 4;
-  return (int)(b < 1 ? 1 : (b > kPlSpmvBlocks32 ? kPlSpmvBlocks32 : b));
-}
-
-// One SpMV launch over several solves: solve s owns first[s + 1] - first[s]
-// blocks; iteration it of a chunk takes s_old / s_new from s0 / s1 by the
-// solve's iteration parity.
 template <typename R>
 struct PlSpmvArgs {
   PencilGeom G;
@@ -862,19 +990,169 @@ struct PlSpmvArgs {
   double* sc;
   double* part;
   int* done_ctr;
-  int parity;  // iterations the solve ran before the chunk, mod 2
+  int parity;  // iterations the solve ran before, mod 2: s_old is s0 (even) or s1
 };
 
+// Block bid of nblk of one solve.
 template <typename R>
-__global__ void __launch_bounds__(kRedThreads, sizeof(R) == 4 ? 6 : 3)
+__device__ __forceinline__ void pl_spmv_run(const PlSpmvArgs<R>& A, bool odd, int bid, int nblk) {
+  __shared__ double sm[kRedThreads];
+  double* const sc = A.sc;
+  if (*(const int*)(sc + S_DONE)) return;
+  constexpr unsigned full = 0xffffffffu;
+  const R be = (R)sc[S_BETA];
+  const R al = (R)sc[S_ALPHA];
+  const PencilGeom& G = A.G;
+  const R* __restrict__ const z = A.z;
+  const R* __restrict__ const sold = odd ? A.s1 : A.s0;
+  R* __restrict__ const snew = odd ? A.s0 : A.s1;
+  R* __restrict__ const x = A.x;
+  const SpmvGrid g = pl_spmv_grid(G);
+  const int p = bid / g.nchunk;
+  const int v0 = (bid - p * g.nchunk) * g.steps;
+  const int PAi = p % G.nPA, PCi = p / G.nPA;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int NV = G.R;
+  const int v1 = min(NV, v0 + g.steps);
+  const int alp = lane & 15;
+  const int dl = alp + (lane >> 4);
+  using P2 = typename Pair<R>::T;
+  const int np = (G.Ls + 1) / 2;  // pairs of a line
+  const long long e0 = (((long long)p * kStrips + w) * NV) * 64 + 2 * lane;
+  // c-neighbour outside the strip: lanes 0..15 the -c side, 16..31 the +c side
+  const bool cm = lane < 16;
+  const bool has_c = cm ? (w > 0 || PCi > 0) : (w + 1 < kStrips || PCi + 1 < G.nPC);
+  const long long dc = pl_out_c(G, w, cm);
+  // a-neighbour across the patch face: al = 0 the -a side, al = 15 the +a side
+  const bool am = alp == 0;
+  const bool has_a = (am && PAi > 0) || (alp == kPatch - 1 && PAi + 1 < G.nPA);
+  const long long da = pl_out_a(G, am);
+  double acc = 0;
+  auto ld2 = [](const R* q, long long e) { return *reinterpret_cast<const P2*>(q + e); };
+  auto st2 = [](R* q, long long e, P2 t) { *reinterpret_cast<P2*>(q + e) = t; };
+  auto mix = [&](P2 a, P2 b) {  // a + beta b
+    P2 t;
+    t.x = a.x + be * b.x;
+    t.y = a.y + be * b.y;
+    return t;
+  };
+  if (v0 < v1) {
+    P2 zero;
+    zero.x = zero.y = R(0);
+    // the values of one step: its own, and those of its neighbours outside
+    struct Row {
+      P2 ad, as, aa, ac, xv, zc, oc, cc, za, oa, ca;
+    };
+    auto fetch = [&](int v) {
+      Row o;
+      const long long e = e0 + (long long)v * 64;
+      const bool live = (unsigned)(v - dl) < (unsigned)np;
+      o.ad = ld2(A.AD, e);
+      o.as = ld2(A.AS, e);
+      o.aa = ld2(A.AA, e);
+      o.ac = ld2(A.AC, e);
+      o.xv = ld2(x, e);
+      o.zc = o.oc = o.cc = o.za = o.oa = o.ca = zero;
+      if (has_c && live) {
+        o.zc = ld2(z, e + dc);
+        o.oc = ld2(sold, e + dc);
+        if (cm) o.cc = ld2(A.AC, e + dc);
+      }
+      if (has_a && live) {
+        o.za = ld2(z, e + da);
+        o.oa = ld2(sold, e + da);
+        if (am) o.ca = ld2(A.AA, e + da);
+      }
+      return o;
+    };
+    // s_new of steps v - 1, v, v + 1; couplings of step v - 1
+    P2 sm1 = zero, ps = zero, pa = zero, pc = zero;
+    if (v0 > 0) {
+      const long long e = e0 + (long long)(v0 - 1) * 64;
+      sm1 = mix(ld2(z, e), ld2(sold, e));
+      ps = ld2(A.AS, e);
+      pa = ld2(A.AA, e);
+      pc = ld2(A.AC, e);
+    }
+    long long e = e0 + (long long)v0 * 64;
+    P2 so = ld2(sold, e);
+    P2 s0v = mix(ld2(z, e), so);
+    P2 nz = zero, ns = zero;
+    if (v0 + 1 < NV) {
+      nz = ld2(z, e + 64);
+      ns = ld2(sold, e + 64);
+    }
+    for (int v = v0; v < v1; ++v, e += 64) {
+      const Row cur = fetch(v);
+      P2 nz2 = zero, ns2 = zero;  // two steps on: s_new of step v + 2
+      if (v + 1 < v1 && v + 2 < NV) {
+        nz2 = ld2(z, e + 128);
+        ns2 = ld2(sold, e + 128);
+      }
+      const P2 sp1 = mix(nz, ns);
+      const P2 sco = mix(cur.zc, cur.oc), sao = mix(cur.za, cur.oa);
+      // one cell: couplings and s_new of its neighbours in the order of the row
+      auto cell = [&](R o_cc, R o_sc, R o_ca, R o_sa, R m1, R ppa, R ppc, R n1, R ms_c, R ms_s,
+                      R ad, R s, R ps_c, R ps_s, R aa, R ac) {
+        const R m_a = __shfl_up_sync(full, m1, 1), m_pa = __shfl_up_sync(full, ppa, 1);
+        const R m_c = __shfl_up_sync(full, m1, 16), m_pc = __shfl_up_sync(full, ppc, 16);
+        const R p_a = __shfl_down_sync(full, n1, 1), p_c = __shfl_down_sync(full, n1, 16);
+        R r = 0;
+        r += (cm ? o_cc : m_pc) * (cm ? o_sc : m_c);
+        r += (am ? o_ca : m_pa) * (am ? o_sa : m_a);
+        r += ms_c * ms_s;
+        r += ad * s;
+        r += ps_c * ps_s;
+        r += aa * (alp == kPatch - 1 ? o_sa : p_a);
+        r += ac * (cm ? p_c : o_sc);
+        return r;
+      };
+      P2 q2;
+      q2.x = cell(cur.cc.x, sco.x, cur.ca.x, sao.x, sm1.x, pa.x, pc.x, sp1.x, ps.y, sm1.y, cur.ad.x,
+                  s0v.x, cur.as.x, s0v.y, cur.aa.x, cur.ac.x);
+      q2.y = cell(cur.cc.y, sco.y, cur.ca.y, sao.y, sm1.y, pa.y, pc.y, sp1.y, cur.as.x, s0v.x,
+                  cur.ad.y, s0v.y, cur.as.y, sp1.x, cur.aa.y, cur.ac.y);
+      P2 x2;
+      x2.x = cur.xv.x + al * so.x;
+      x2.y = cur.xv.y + al * so.y;
+      st2(x, e, x2);
+      st2(snew, e, s0v);
+      st2(A.q, e, q2);
+      acc += (double)s0v.x * (double)q2.x;
+      acc += (double)s0v.y * (double)q2.y;
+      ps = cur.as;
+      pa = cur.aa;
+      pc = cur.ac;
+      sm1 = s0v;
+      s0v = sp1;
+      so = ns;
+      nz = nz2;
+      ns = ns2;
+    }
+  }
+  acc = block_sum<double>(acc, sm);
+  if (threadIdx.x == 0) A.part[bid] = acc;
+  // the last block: alpha = rho / s.q
+  if (last_block(A.done_ctr, nblk)) red_alpha_body(A.part, nblk, sc, sm);
+}
+
+template <typename R>
+__global__ void __launch_bounds__(kRedThreads, sizeof(R) == 4 ? 4 : 2)
+    k_pl_spmv_s(const PlSpmvArgs<R> A) {
+  pl_spmv_run<R>(A, A.parity != 0, (int)blockIdx.x, (int)gridDim.x);
+}
+
+// One SpMV launch over several solves: solve s owns first[s + 1] - first[s]
+// blocks; iteration it of a chunk takes s_old / s_new by the solve's iteration
+// parity.
+template <typename R>
+__global__ void __launch_bounds__(kRedThreads, sizeof(R) == 4 ? 4 : 2)
     k_pl_spmv_batch(const PlSpmvArgs<R>* __restrict__ tab, const int* __restrict__ first,
                     int nsolve, int it) {
   const int s = batch_solve_of(first, nsolve, (int)blockIdx.x);
-  const PlSpmvArgs<R>& a = tab[s];
+  const PlSpmvArgs<R> a = tab[s];
   const int b0 = __ldg(first + s);
-  const bool odd = ((a.parity + it) & 1) != 0;
-  pl_spmv_run<R>(a.G, a.AD, a.AS, a.AA, a.AC, a.z, odd ? a.s1 : a.s0, odd ? a.s0 : a.s1, a.q,
-                 a.x, a.sc, a.part, a.done_ctr, (int)blockIdx.x - b0, __ldg(first + s + 1) - b0);
+  pl_spmv_run<R>(a, ((a.parity + it) & 1) != 0, (int)blockIdx.x - b0, __ldg(first + s + 1) - b0);
 }
 
 // status[6 s + j] = sc_s[S_RES + j] (residual, beta, tolerance, iteration,
@@ -883,139 +1161,6 @@ __global__ void k_pl_batch_status(double* const* __restrict__ scs, int nsolve,
                                   double* __restrict__ status) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < 6 * nsolve) status[i] = __ldcg(scs[i / 6] + S_RES + i % 6);
-}
-
-// k_pl_spmv_s's arithmetic, streamed: block (patch p, chunk k) walks rows
-// [t0, t1) of one patch in order, one thread per line.  s_new of rows t - 1,
-// t and t + 1 sits in a ring of three shared-memory rows and the couplings
-// A_s, A_a, A_c of row t - 1 in a second ring, so every in-patch neighbour
-// (one row back or ahead, the same line, line -+1 or line -+16) is read from
-// shared memory and each value is loaded from global memory once; only the
-// neighbours across a patch face (lines at a = 0 / 15, c = 0 / 15) are read
-// from global memory as k_pl_spmv_s reads them.  Terms are summed in the same
-// order as k_pl_spmv_s, missing neighbours skipped.  partial[block] = s_new.q
-// over the chunk (blocks ordered patch-major, then chunk).
-template <typename R>
-__global__ void __launch_bounds__(kRedThreads)
-    k_pl_spmv_stream(PencilGeom G, int rows_per_chunk, int nchunk, const R* __restrict__ AD,
-                     const R* __restrict__ AS, const R* __restrict__ AA,
-                     const R* __restrict__ AC, const R* __restrict__ z,
-                     const R* __restrict__ sold, R* __restrict__ snew, R* __restrict__ q,
-                     R* __restrict__ x, const double* __restrict__ sc,
-                     double* __restrict__ partial) {
-  __shared__ R ring[3][kPatchLines];
-  __shared__ R cs[2][kPatchLines], ca[2][kPatchLines], cc[2][kPatchLines];
-  __shared__ double sm[kRedThreads];
-  if (*(const int*)(sc + S_DONE)) return;
-  const R be = (R)sc[S_BETA];
-  const R al = (R)sc[S_ALPHA];
-  const int l = threadIdx.x;
-  const int p = blockIdx.x / nchunk;
-  const int k = blockIdx.x - p * nchunk;
-  const int t0 = k * rows_per_chunk;
-  const int t1 = min(G.R, t0 + rows_per_chunk);
-  double acc = 0;
-  if (t0 < t1) {
-    const long long base = (long long)p * G.R * kPatchLines + l;
-    // s_new and the couplings of row t0 - 1 (zero before the first row)
-    if (t0 > 0) {
-      const long long e = base + (long long)(t0 - 1) * kPatchLines;
-      ring[(t0 + 2) % 3][l] = z[e] + be * sold[e];
-      cs[(t0 + 1) & 1][l] = AS[e];
-      ca[(t0 + 1) & 1][l] = AA[e];
-      cc[(t0 + 1) & 1][l] = AC[e];
-    } else {
-      ring[2][l] = R(0);
-      cs[1][l] = ca[1][l] = cc[1][l] = R(0);
-    }
-    // row t's own values and row t + 1's z, s_old, held one row ahead in
-    // registers so the loads of the next row overlap this row's work
-    long long e0 = base + (long long)t0 * kPatchLines;
-    R nz = z[e0], ns = sold[e0];
-    ring[t0 % 3][l] = nz + be * ns;
-    R ad = AD[e0], as = AS[e0], aa = AA[e0], ac = AC[e0], so = ns, xv = x[e0];
-    if (t0 + 1 < G.R) {
-      nz = z[e0 + kPatchLines];
-      ns = sold[e0 + kPatchLines];
-    }
-    for (int t = t0; t < t1; ++t) {
-      const long long e = base + (long long)t * kPatchLines;
-      if (t + 1 < G.R) ring[(t + 1) % 3][l] = nz + be * ns;
-      cs[t & 1][l] = as;
-      ca[t & 1][l] = aa;
-      cc[t & 1][l] = ac;
-      const R ns1 = ns;
-      // prefetch: row t + 1's own values, row t + 2's z and s_old
-      R ad_n = 0, as_n = 0, aa_n = 0, ac_n = 0, xv_n = 0;
-      if (t + 1 < t1) {
-        ad_n = AD[e + kPatchLines];
-        as_n = AS[e + kPatchLines];
-        aa_n = AA[e + kPatchLines];
-        ac_n = AC[e + kPatchLines];
-        xv_n = x[e + kPatchLines];
-        if (t + 2 < G.R) {
-          nz = z[e + 2 * kPatchLines];
-          ns = sold[e + 2 * kPatchLines];
-        }
-      }
-      __syncthreads();
-      const PlCell c = pl_cell(G, p * G.R + t, l);
-      if (c.live) {
-        const R* sm1 = ring[(t + 2) % 3];
-        const R* s0 = ring[t % 3];
-        const R* sp1 = ring[(t + 1) % 3];
-        const int pr = (t + 1) & 1;  // coupling ring slot of row t - 1
-        R r = 0;
-        // -c
-        if (c.cl > 0) {
-          r += cc[pr][l - kPatch] * sm1[l - kPatch];
-        } else if (c.PCi > 0) {
-          const long long n = pl_index(G, p - G.nPA, t + kPatch - 1, l + kPatch * (kPatch - 1));
-          r += AC[n] * (z[n] + be * sold[n]);
-        }
-        // -a
-        if (c.al > 0) {
-          r += ca[pr][l - 1] * sm1[l - 1];
-        } else if (c.PAi > 0) {
-          const long long n = pl_index(G, p - 1, t + kPatch - 1, l + kPatch - 1);
-          r += AA[n] * (z[n] + be * sold[n]);
-        }
-        // -s
-        if (c.s > 0) r += cs[pr][l] * sm1[l];
-        x[e] = xv + al * so;
-        const R sn = s0[l];
-        r += ad * sn;
-        // +s
-        if (c.s + 1 < G.Ls) r += as * sp1[l];
-        // +a
-        if (c.al < kPatch - 1) {
-          r += aa * sp1[l + 1];
-        } else if (c.PAi + 1 < G.nPA) {
-          const long long n = pl_index(G, p + 1, t - (kPatch - 1), l - (kPatch - 1));
-          r += aa * (z[n] + be * sold[n]);
-        }
-        // +c
-        if (c.cl < kPatch - 1) {
-          r += ac * sp1[l + kPatch];
-        } else if (c.PCi + 1 < G.nPC) {
-          const long long n = pl_index(G, p + G.nPA, t - (kPatch - 1), l - kPatch * (kPatch - 1));
-          r += ac * (z[n] + be * sold[n]);
-        }
-        snew[e] = sn;
-        q[e] = r;
-        acc += (double)sn * (double)r;
-      }
-      ad = ad_n;
-      as = as_n;
-      aa = aa_n;
-      ac = ac_n;
-      xv = xv_n;
-      so = ns1;
-      __syncthreads();
-    }
-  }
-  acc = block_sum<double>(acc, sm);
-  if (threadIdx.x == 0) partial[blockIdx.x] = acc;
 }
 
 // FP64 residual r64 = b - A x64 with the coefficients promoted; partial max|r64|
@@ -1027,10 +1172,10 @@ __global__ void __launch_bounds__(kRedThreads)
                     double* __restrict__ r, double* __restrict__ partial) {
   __shared__ double sm[kRedThreads];
   double m = 0;
-  const int nrow = (int)(G.npatch * G.R);
+  const int nrow = (int)(G.len / kPatchLines);
   for (int row = blockIdx.x; row < nrow; row += gridDim.x) {
     const long long e = (long long)row * kPatchLines + threadIdx.x;
-    const PlCell c = pl_cell(G, row, threadIdx.x);
+    const PlCell c = pl_cell(G, e);
     if (!c.live) continue;
     const PlNbr n = pl_nbr(G, c, e);
     double acc = (double)AD[e] * x[e];
@@ -1136,10 +1281,10 @@ __global__ void __launch_bounds__(kRedThreads)
                 const unsigned char* __restrict__ dof, const R* __restrict__ F,
                 long long fs, R* __restrict__ AD, R* __restrict__ AS, R* __restrict__ AA,
                 R* __restrict__ AC, R* __restrict__ B) {
-  const int nrow = (int)(G.npatch * G.R);
+  const int nrow = (int)(G.len / kPatchLines);
   for (int row = blockIdx.x; row < nrow; row += gridDim.x) {
     const long long e = (long long)row * kPatchLines + threadIdx.x;
-    const PlCell c = pl_cell(G, row, threadIdx.x);
+    const PlCell c = pl_cell(G, e);
     R ad = 0, as = 0, aa = 0, ac = 0, bv = 0;
     if (c.live) {
       int P[3];
@@ -1188,7 +1333,7 @@ __global__ void k_pl_scatter_pressure(PencilGeom G, GridDesc g, const int* __res
       const int c = P[G.ax_c] - G.lo[G.ax_c];
       const int PAi = a / kPatch, al = a - PAi * kPatch;
       const int PCi = c / kPatch, cl = c - PCi * kPatch;
-      const long long idx = pl_index(G, (long long)PCi * G.nPA + PAi, s + al + cl, al + kPatch * cl);
+      const long long idx = pl_index(G, (long long)PCi * G.nPA + PAi, s, al, cl);
       v = x64 ? (R)x64[idx] : x32[idx];
     }
     p[n] = v;

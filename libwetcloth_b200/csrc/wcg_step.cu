@@ -1280,9 +1280,9 @@ static cudaError_t pl_setup(Context& c, const int* lo, const int* hi) {
   G.NC = ext[G.ax_c];
   G.nPA = (G.NA + kPatch - 1) / kPatch;
   G.nPC = (G.NC + kPatch - 1) / kPatch;
-  G.R = G.Ls + 2 * (kPatch - 1);
+  G.R = ((G.Ls + 1) / 2 + kPatch + kChunk - 1) / kChunk * kChunk;
   G.npatch = (long long)G.nPA * G.nPC;
-  G.len = G.npatch * G.R * kPatchLines;
+  G.len = G.npatch * G.R * kPatchLines * 2;
   const bool same_shape = c.plg.npatch == G.npatch && c.plg.nPA == G.nPA;
   c.plg = G;
   if (G.len > c.pl_cap) {
@@ -1290,27 +1290,34 @@ static cudaError_t pl_setup(Context& c, const int* lo, const int* hi) {
     WCG_TRY(c.pl.ensure((size_t)kNumPlFields * G.len * sizeof(R)));
     if (c.prm.precision != 0) WCG_TRY(c.pl64.ensure((size_t)kNumPl64Fields * G.len * sizeof(double)));
   }
-  // edge words: 2 faces x rows x 16 entries x (2 values x words per value)
-  const size_t edge_bytes =
-      (size_t)G.npatch * 2 * edge_rows(G) * kPatch * 2 * (sizeof(R) / 4) * 8;
+  // edge words (those of the factorisation, two values per cell)
+  const size_t edge_bytes = (size_t)edge_words(G, pl_units<R>(G), sweep_words(kFactor, sizeof(R))) * sizeof(u64);
   if (edge_bytes > c.pl_edge.bytes) {
     WCG_TRY(c.pl_edge.ensure(edge_bytes));
     // tags of a fresh buffer must not match any epoch (epochs start at 1)
     WCG_TRY(cudaMemsetAsync(c.pl_edge.p, 0, c.pl_edge.bytes, c.stream));
   }
   WCG_TRY(c.pl_part.ensure(
-      (size_t)std::max<long long>(G.npatch, std::max(kPlBlocks, kPlSpmvBlocks32)) * sizeof(double)));
-  if (!same_shape || c.pl_order_h.size() != (size_t)G.npatch) {
-    // patches in wave order PAi + PCi
-    c.pl_order_h.resize(G.npatch);
-    int k = 0;
-    for (int w = 0; w <= G.nPA + G.nPC - 2; ++w)
-      for (int pc = 0; pc < G.nPC; ++pc) {
+      (size_t)std::max(pl_units<R>(G), kPlBlocks) * sizeof(double)));
+  // Clusters of 4 groups along c where the box leaves SMs idle: their c-faces
+  // then go through the cluster's shared memory (64^3 dam break, FP64, per PCG
+  // iteration: 138.6 us in clusters of 2, 134.3 in larger ones).  A box that fills
+  // the SMs runs without, so that no group waits for a whole cluster's place; there
+  // the shape made no difference (256^3 FP32: 669 / 661 / 666 us an iteration in
+  // clusters of 2, 4 and 8).
+  const int ngroup = pl_groups<R>(G);
+  c.pl_cl = !c.shared_solve && ngroup > 1 && pl_units<R>(G) <= 74 ? 4 : 1;
+  const int ncl = (ngroup + c.pl_cl - 1) / c.pl_cl;
+  if (!same_shape || c.pl_order_h.size() != (size_t)G.nPA * ncl) {
+    // clusters in wave order: column + cluster of the column
+    c.pl_order_h.clear();
+    for (int w = 0; w <= G.nPA + ncl - 2; ++w)
+      for (int pc = 0; pc < ncl; ++pc) {
         const int pa = w - pc;
-        if (pa >= 0 && pa < G.nPA) c.pl_order_h[k++] = pc * G.nPA + pa;
+        if (pa >= 0 && pa < G.nPA) c.pl_order_h.push_back(pc * G.nPA + pa);
       }
-    WCG_TRY(c.pl_order.ensure((size_t)G.npatch * sizeof(int)));
-    WCG_TRY(cudaMemcpyAsync(c.pl_order.p, c.pl_order_h.data(), G.npatch * sizeof(int),
+    WCG_TRY(c.pl_order.ensure(c.pl_order_h.size() * sizeof(int)));
+    WCG_TRY(cudaMemcpyAsync(c.pl_order.p, c.pl_order_h.data(), c.pl_order_h.size() * sizeof(int),
                             cudaMemcpyHostToDevice, c.stream));
   }
   // every array starts at zero (rows and lines outside the box stay zero)
@@ -1319,6 +1326,24 @@ static cudaError_t pl_setup(Context& c, const int* lo, const int* hi) {
   // the sweep ticket and the done counters of the SpMV and the sweeps
   WCG_TRY(cudaMemsetAsync(c.ticket.as<int>() + 1, 0, 3 * sizeof(int), c.stream));
   return cudaSuccess;
+}
+
+template <typename... P, typename... V>
+static cudaError_t launch_clusters(void (*kernel)(P...), unsigned grid, unsigned cluster,
+                                   unsigned threads, size_t smem, cudaStream_t st, V... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cluster;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 template <typename R>
@@ -1348,13 +1373,14 @@ static PencilSweepArgs<R> pl_args(Context& c) {
   return a;
 }
 
-template <typename R, int MODE, bool UPD>
-static cudaError_t pl_sweep(Context& c, PencilSweepArgs<R> a) {
+template <typename R, int MODE, bool UPD, int CL>
+static cudaError_t pl_sweep_cl(Context& c, PencilSweepArgs<R> a) {
   ProfScope prof(c, MODE == kFactor ? P_MICFACTOR : P_MICSWEEP);
   const PencilGeom& G = c.plg;
+  const int ncl = G.nPA * ((pl_groups<R>(G) + CL - 1) / CL);
   a.epoch = (unsigned)(++c.tile_epoch);
   a.ticket_base = c.pl_tickets;
-  c.pl_tickets += (int)G.npatch;
+  c.pl_tickets += ncl;
   constexpr size_t smem = sweep_dyn_smem<R>(MODE);
   // function attributes are per device: set once per instantiation and
   // device (the batch may step contexts of several devices from several
@@ -1362,12 +1388,19 @@ static cudaError_t pl_sweep(Context& c, PencilSweepArgs<R> a) {
   static std::atomic<unsigned long long> attr_set{0};
   const unsigned long long dbit = 1ull << (c.device & 63);
   if (!(attr_set.load(std::memory_order_acquire) & dbit)) {
-    WCG_TRY(cudaFuncSetAttribute(k_pencil_sweep<R, MODE, UPD>,
+    WCG_TRY(cudaFuncSetAttribute(k_pencil_sweep<R, MODE, UPD, CL>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set.fetch_or(dbit, std::memory_order_release);
   }
-  ++c.launches, k_pencil_sweep<R, MODE, UPD><<<(unsigned)G.npatch, kPencilThreads, smem, c.stream>>>(a);
-  return cudaGetLastError();
+  ++c.launches;
+  return launch_clusters(k_pencil_sweep<R, MODE, UPD, CL>, (unsigned)(ncl * CL), CL, sweep_threads<R>(),
+                         smem, c.stream, a);
+}
+
+template <typename R, int MODE, bool UPD>
+static cudaError_t pl_sweep(Context& c, PencilSweepArgs<R> a) {
+  if (c.pl_cl == 4) return pl_sweep_cl<R, MODE, UPD, 4>(c, a);
+  return pl_sweep_cl<R, MODE, UPD, 1>(c, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -1390,7 +1423,7 @@ struct SolveReq {
   PencilSweepArgs<float> fa32{}, ba32{};
   PlSpmvArgs<double> sa64{};
   PlSpmvArgs<float> sa32{};
-  int npatch = 0, nspmv = 0;
+  int nsweep = 0, nspmv = 0;  // CTAs of a sweep, blocks of the SpMV
   int launched = 0;  // iterations launched so far
   bool finished = false;
   cudaError_t cerr = cudaSuccess;
@@ -1474,7 +1507,7 @@ static cudaError_t ss_chunk(SharedSolve& S, const std::vector<SolveReq*>& L) {
     f1[i] = (int)n1;
     f2[i] = (int)n2;
     n1 += q.nspmv;
-    n2 += q.npatch;
+    n2 += q.nsweep;
     scs[i] = c.dscalars.as<double>();
   }
   if (n1 > INT_MAX || n2 > INT_MAX) return cudaErrorInvalidValue;
@@ -1493,18 +1526,18 @@ static cudaError_t ss_chunk(SharedSolve& S, const std::vector<SolveReq*>& L) {
   static std::atomic<unsigned long long> attr_set{0};
   const unsigned long long dbit = 1ull << (S.device & 63);
   if (!(attr_set.load(std::memory_order_acquire) & dbit)) {
-    WCG_TRY(cudaFuncSetAttribute(k_pencil_sweep_batch<R, kForward, true>,
+    WCG_TRY(cudaFuncSetAttribute(k_pencil_sweep_batch<R, kForward, true, 1>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smf));
-    WCG_TRY(cudaFuncSetAttribute(k_pencil_sweep_batch<R, kBackward, false>,
+    WCG_TRY(cudaFuncSetAttribute(k_pencil_sweep_batch<R, kBackward, false, 1>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb));
     attr_set.fetch_or(dbit, std::memory_order_release);
   }
   for (int b = 0; b < kSharedChunk; ++b) {
     k_pl_spmv_batch<R><<<(unsigned)n1, kRedThreads, 0, S.stream>>>(dsa, df1, n, b);
-    k_pencil_sweep_batch<R, kForward, true><<<(unsigned)n2, kPencilThreads, smf, S.stream>>>(
+    k_pencil_sweep_batch<R, kForward, true, 1><<<(unsigned)n2, sweep_threads<R>(), smf, S.stream>>>(
         dfa, df2, n, 2 * b);
-    k_pencil_sweep_batch<R, kBackward, false><<<(unsigned)n2, kPencilThreads, smb, S.stream>>>(
-        dba, df2, n, 2 * b + 1);
+    k_pencil_sweep_batch<R, kBackward, false, 1><<<(unsigned)n2, sweep_threads<R>(), smb,
+                                                   S.stream>>>(dba, df2, n, 2 * b + 1);
   }
   k_pl_batch_status<<<(unsigned)((6 * n + 255) / 256), 256, 0, S.stream>>>(dsc, n, dst);
   WCG_TRY(cudaGetLastError());
@@ -1516,7 +1549,7 @@ static cudaError_t ss_chunk(SharedSolve& S, const std::vector<SolveReq*>& L) {
     SolveReq& q = *L[(size_t)i];
     Context& c = *q.c;
     c.tile_epoch += 2 * kSharedChunk;
-    c.pl_tickets += 2 * kSharedChunk * q.npatch;
+    c.pl_tickets += 2 * kSharedChunk * q.nsweep;
     q.launched += kSharedChunk;
     std::memcpy(q.status, hst + 6 * i, sizeof(q.status));
   }
@@ -1628,9 +1661,8 @@ static cudaError_t pl_pcg(Context& c, R* r, R* x, double tol_abs, int maxiters, 
   R* q = pl_field<R>(c, PL_Q);
   R* y = pl_field<R>(c, PL_Y);
   double* sc = c.dscalars.as<double>();
-  double* part = c.scratch.as<double>();
   double* ppart = c.pl_part.as<double>();
-  const int np = (int)G.npatch;
+  const int np = pl_units<R>(G);
   *iters = 0;
   *conv = 0;
   *res = 0;
@@ -1666,44 +1698,32 @@ static cudaError_t pl_pcg(Context& c, R* r, R* x, double tol_abs, int maxiters, 
   fa.part = ppart;
   fa.done_ctr = done_ctr;
   fa.npart = np;
-  R* sold = s0;
-  R* snew = s1;
-  const R* AD = pl_field<R>(c, PL_AD);
-  const R* AS = pl_field<R>(c, PL_AS);
-  const R* AA = pl_field<R>(c, PL_AA);
-  const R* AC = pl_field<R>(c, PL_AC);
-  // the streamed SpMV: chunks of consecutive rows of one patch per block,
-  // about four blocks of resident capacity (kPlSpmvBlocks32) in all
-  const int nchunk = (int)std::min<long long>(
-      G.R, std::max<long long>(1, (4 * kPlSpmvBlocks32 + G.npatch - 1) / G.npatch));
-  const int rows_per_chunk = (G.R + nchunk - 1) / nchunk;
-  const int spmv_blocks = (int)(G.npatch * nchunk);
-  const int rows_blocks = pl_spmv_blocks(G);
-  WCG_TRY(ensure_scratch(c, (size_t)std::max(spmv_blocks, rows_blocks) * sizeof(double)));
-  part = c.scratch.as<double>();
-  if (c.shared_solve && c.spmv_rows && G.npatch <= c.shared_solve->max_patches.load()) {
+  const int spmv_blocks = pl_spmv_grid(G).blocks;
+  WCG_TRY(ensure_scratch(c, (size_t)spmv_blocks * sizeof(double)));
+  PlSpmvArgs<R> sa{};
+  sa.G = G;
+  sa.AD = pl_field<R>(c, PL_AD);
+  sa.AS = pl_field<R>(c, PL_AS);
+  sa.AA = pl_field<R>(c, PL_AA);
+  sa.AC = pl_field<R>(c, PL_AC);
+  sa.z = z;
+  sa.s0 = s0;
+  sa.s1 = s1;
+  sa.q = q;
+  sa.x = x;
+  sa.sc = sc;
+  sa.part = c.scratch.as<double>();
+  sa.done_ctr = c.ticket.as<int>() + 2;
+  if (c.shared_solve && G.npatch <= c.shared_solve->max_patches.load()) {
     // the iterations run in the batch's shared launches
     SolveReq req;
     req.c = &c;
     req.prec = c.prm.precision == 0 ? 0 : 1;
     ss_fa<R>(req) = fa;
     ss_ba<R>(req) = ba;
-    PlSpmvArgs<R>& sa = ss_sa<R>(req);
-    sa.G = G;
-    sa.AD = AD;
-    sa.AS = AS;
-    sa.AA = AA;
-    sa.AC = AC;
-    sa.z = z;
-    sa.s0 = s0;
-    sa.s1 = s1;
-    sa.q = q;
-    sa.x = x;
-    sa.sc = sc;
-    sa.part = part;
-    sa.done_ctr = c.ticket.as<int>() + 2;
-    req.npatch = (int)G.npatch;
-    req.nspmv = rows_blocks;
+    ss_sa<R>(req) = sa;
+    req.nsweep = pl_units<R>(G);
+    req.nspmv = spmv_blocks;
     WCG_TRY(cudaEventRecord(c.ev_ss_ready, c.stream));
     WCG_TRY(shared_solve_run(*c.shared_solve, req));
     WCG_TRY(cudaStreamWaitEvent(c.stream, c.ev_ss_done, 0));
@@ -1717,20 +1737,12 @@ static cudaError_t pl_pcg(Context& c, R* r, R* x, double tol_abs, int maxiters, 
     for (int b = 0; b < c.pcg_batch; ++b) {
       {
         ProfScope prof(c, P_PCGVEC);
-        if (c.spmv_rows) {  // its last block forms alpha
-          ++c.launches, k_pl_spmv_s<R><<<rows_blocks, kRedThreads, 0, c.stream>>>(
-              G, AD, AS, AA, AC, z, sold, snew, q, x, sc, part, c.ticket.as<int>() + 2);
-        } else {
-          ++c.launches, k_pl_spmv_stream<R><<<spmv_blocks, kRedThreads, 0, c.stream>>>(
-              G, rows_per_chunk, nchunk, AD, AS, AA, AC, z, sold, snew, q, x, sc, part);
-          ++c.launches, k_red_alpha<<<1, kRedThreads, 0, c.stream>>>(part, spmv_blocks, sc);
-        }
+        // its last block forms alpha
+        ++c.launches, k_pl_spmv_s<R><<<spmv_blocks, kRedThreads, 0, c.stream>>>(sa);
       }
       WCG_TRY((pl_sweep<R, kForward, true>(c, fa)));
       WCG_TRY((pl_sweep<R, kBackward, false>(c, ba)));
-      R* t = sold;
-      sold = snew;
-      snew = t;
+      sa.parity ^= 1;
     }
     WCG_TRY(fetch(c, sc + S_RES, 6, h));  // res, beta, tol, iter, maxit, done
     const int done = *(const int*)&h[5];
