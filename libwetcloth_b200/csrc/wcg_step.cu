@@ -554,16 +554,21 @@ __global__ void k_minmax(const R* __restrict__ P, long long pcap, long long n,
   }
 }
 
+// a warp per component (one thread over all partials took 160 us of a step)
 __global__ void k_minmax_final(const double* __restrict__ partial, int nb,
                                double* __restrict__ out) {
-  if (threadIdx.x != 0) return;
-  double r[6] = {1e20, 1e20, 1e20, -1e20, -1e20, -1e20};
-  for (int b = 0; b < nb; ++b)
-    for (int a = 0; a < 3; ++a) {
-      r[a] = partial[b * 6 + a] < r[a] ? partial[b * 6 + a] : r[a];
-      r[3 + a] = partial[b * 6 + 3 + a] > r[3 + a] ? partial[b * 6 + 3 + a] : r[3 + a];
-    }
-  for (int k = 0; k < 6; ++k) out[k] = r[k];
+  const int a = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (a >= 6) return;
+  double r = a < 3 ? 1e20 : -1e20;
+  for (int b = lane; b < nb; b += 32) {
+    const double v = partial[b * 6 + a];
+    r = a < 3 ? (v < r ? v : r) : (v > r ? v : r);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const double v = __shfl_down_sync(0xffffffffu, r, o);
+    r = a < 3 ? (v < r ? v : r) : (v > r ? v : r);
+  }
+  if (lane == 0) out[a] = r;
 }
 
 // max over particles of |v|^2 (TwoDScene::getMaxFluidVelocity :4180-4188)
@@ -603,7 +608,7 @@ static cudaError_t build_grid_t(Context& c) {
   if (ne > 0)
     ++c.launches, k_minmax<R><<<kRedBlocks, kRedThreads, 0, c.stream>>>(EP, c.ecap, ne,
                                                                       part + kRedBlocks * 6);
-  ++c.launches, k_minmax_final<<<1, 32, 0, c.stream>>>(part, ne > 0 ? 2 * kRedBlocks : kRedBlocks,
+  ++c.launches, k_minmax_final<<<1, 192, 0, c.stream>>>(part, ne > 0 ? 2 * kRedBlocks : kRedBlocks,
                                                         dsc);
   WCG_TRY(read_small(c, dsc, 6 * sizeof(double), c.hscalars));
   double bbmin[3] = {1e20, 1e20, 1e20}, bbmax[3] = {-1e20, -1e20, -1e20};
