@@ -183,6 +183,99 @@ __global__ void __launch_bounds__(kMgCoarseThreads) k_mg_coarsest(MgLevel<R> L, 
     }
 }
 
+// The same with x in shared memory and the cells of each colour listed there,
+// for levels whose box fits (mg_coarse_smem).  A thread holds the first
+// kMgHeld cells of each colour with their couplings in registers, so a colour
+// is six reads of x, a division and a barrier; further cells take their
+// couplings from global memory.  Bound by the latency of those 2 x iters
+// colours: 1550 us per V-cycle with everything in global memory (19 x 12 x 19
+// cells, FP64; 1225 us in FP32 at 18 x 10 x 18), most of it index arithmetic and
+// cache latency.
+template <typename R>
+constexpr int kMgHeld = sizeof(R) == 4 ? 2 : 1;
+template <typename R>
+__host__ __device__ constexpr size_t mg_coarse_smem(int n) {
+  return ((size_t)n * sizeof(R) + 15) / 16 * 16 + (size_t)n * sizeof(int);
+}
+constexpr size_t kMgCoarseSmemMax = 200 * 1024;
+
+template <typename R>
+__global__ void __launch_bounds__(kMgCoarseThreads) k_mg_coarsest_smem(MgLevel<R> L, int iters) {
+  extern __shared__ __align__(16) unsigned char dsm_mg[];
+  R* const x = reinterpret_cast<R*>(dsm_mg);
+  // cells with (i + j + k) odd from the front, even from the back
+  int* const list = reinterpret_cast<int*>(dsm_mg + ((size_t)L.n * sizeof(R) + 15) / 16 * 16);
+  __shared__ int s_cnt[2];
+  if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < L.n; idx += blockDim.x) {
+    x[idx] = L.x[idx];
+    if (!L.m[idx]) continue;
+    int i, j, k;
+    mg_ijk(idx, L.ni, L.nj, i, j, k);
+    // (cells of one colour do not touch: their order in the list is free)
+    if ((i + j + k) & 1) list[atomicAdd(&s_cnt[0], 1)] = idx;
+    else list[L.n - 1 - atomicAdd(&s_cnt[1], 1)] = idx;
+  }
+  __syncthreads();
+  const int cnt[2] = {s_cnt[0], s_cnt[1]};
+  const int sj = L.ni, sk = L.ni * L.nj;
+  // couplings in the order of mg_offdiag (-z -y -x +x +y +z), 0 beyond the box
+  struct Cell {
+    R c[6], d, b;
+    int idx, m;  // m: bit t set where neighbour t exists
+  };
+  auto take = [&](int idx) {
+    Cell e;
+    int i, j, k;
+    mg_ijk(idx, L.ni, L.nj, i, j, k);
+    e.idx = idx;
+    e.m = (k > 0) | (j > 0) << 1 | (i > 0) << 2 | (i + 1 < L.ni) << 3 | (j + 1 < L.nj) << 4 |
+          (k + 1 < L.nk) << 5;
+    e.c[0] = k > 0 ? L.az[idx - sk] : R(0);
+    e.c[1] = j > 0 ? L.ay[idx - sj] : R(0);
+    e.c[2] = i > 0 ? L.ax[idx - 1] : R(0);
+    e.c[3] = i + 1 < L.ni ? L.ax[idx] : R(0);
+    e.c[4] = j + 1 < L.nj ? L.ay[idx] : R(0);
+    e.c[5] = k + 1 < L.nk ? L.az[idx] : R(0);
+    e.d = L.d[idx];
+    e.b = L.b[idx];
+    return e;
+  };
+  auto relax = [&](const Cell& e) {
+    R s = R(0);
+    if (e.m & 1) s += e.c[0] * x[e.idx - sk];
+    if (e.m & 2) s += e.c[1] * x[e.idx - sj];
+    if (e.m & 4) s += e.c[2] * x[e.idx - 1];
+    if (e.m & 8) s += e.c[3] * x[e.idx + 1];
+    if (e.m & 16) s += e.c[4] * x[e.idx + sj];
+    if (e.m & 32) s += e.c[5] * x[e.idx + sk];
+    x[e.idx] = e.d != R(0) ? (e.b - s) / e.d : R(0);
+  };
+  auto cell_at = [&](int col, int t) { return col == 0 ? list[t] : list[L.n - 1 - t]; };
+  constexpr int H = kMgHeld<R>;
+  Cell held[2][H];
+#pragma unroll
+  for (int col = 0; col < 2; ++col)
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int t = threadIdx.x + h * kMgCoarseThreads;
+      if (t < cnt[col]) held[col][h] = take(cell_at(col, t));
+    }
+  for (int it = 0; it < iters; ++it)
+#pragma unroll
+    for (int col = 0; col < 2; ++col) {
+#pragma unroll
+      for (int h = 0; h < H; ++h)
+        if ((int)threadIdx.x + h * kMgCoarseThreads < cnt[col]) relax(held[col][h]);
+      for (int t = threadIdx.x + H * kMgCoarseThreads; t < cnt[col]; t += kMgCoarseThreads)
+        relax(take(cell_at(col, t)));
+      __syncthreads();
+    }
+  for (int idx = threadIdx.x; idx < L.n; idx += blockDim.x)
+    if (L.m[idx]) L.x[idx] = x[idx];
+}
+
 // b_c = R (b_f - A_f x_f) = 0.125 * (sum of the fine residuals of the DOF
 // children); x_c = 0.
 template <typename R>

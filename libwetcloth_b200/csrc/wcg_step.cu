@@ -1962,7 +1962,22 @@ static cudaError_t mg_vcycle(Context& c, R* z, R* r) {
     smooth(l, kMgPreSweeps);
     ++c.launches, k_mg_restrict<R><<<mg_blocks(L[l + 1].n), kMgThreads, 0, c.stream>>>(L[l], L[l + 1]);
   }
-  ++c.launches, k_mg_coarsest<R><<<1, kMgCoarseThreads, 0, c.stream>>>(L[nlev - 1], kMgCoarseSweeps);
+  const size_t cs = mg_coarse_smem<R>(L[nlev - 1].n);
+  if (cs <= kMgCoarseSmemMax) {
+    static std::atomic<unsigned long long> attr_set{0};  // once per device, as in pl_sweep
+    const unsigned long long dbit = 1ull << (c.device & 63);
+    if (!(attr_set.load(std::memory_order_acquire) & dbit)) {
+      WCG_TRY(cudaFuncSetAttribute(k_mg_coarsest_smem<R>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)kMgCoarseSmemMax));
+      attr_set.fetch_or(dbit, std::memory_order_release);
+    }
+    ++c.launches, k_mg_coarsest_smem<R><<<1, kMgCoarseThreads, cs, c.stream>>>(L[nlev - 1],
+                                                                              kMgCoarseSweeps);
+  } else {
+    ++c.launches, k_mg_coarsest<R><<<1, kMgCoarseThreads, 0, c.stream>>>(L[nlev - 1],
+                                                                         kMgCoarseSweeps);
+  }
   for (int l = nlev - 2; l >= 0; --l) {
     ++c.launches, k_mg_prolong<R><<<mg_blocks(L[l].n), kMgThreads, 0, c.stream>>>(L[l + 1], L[l]);
     smooth(l, kMgPreSweeps);
