@@ -418,132 +418,169 @@ __device__ inline int halo_face(int a, int x, int y, int z) {
 }
 __device__ inline int halo_centre(int x, int y, int z) { return (z * 6 + y) * 6 + x; }
 
-// Scatter: one warp per active bucket (WPB warps per block, each with its own
-// tile).  The bucket's particles (key cells in the bucket: one contiguous run
-// of the sorted arrays) are visited one at a time in sorted order; lane l < 27
-// is stencil slot (l % 3, l / 3 % 3, l / 9) of the visited particle, so the 27
-// lanes write 27 distinct nodes per node type and the warp adds into its tile
-// without atomics, every node receiving its contributions in sorted-particle
-// order: deterministic.  Lanes 0..17 evaluate the particle's 18 per-axis
-// weights (3 axes x offsets 0 and 1/2 x 3 nodes) once; the slot lanes take
-// theirs by shuffle.  Requires stencil offsets in {0, 1} (checked on the host).
-template <typename R, int WPB>
-__global__ void __launch_bounds__(32 * WPB)
-    k_p2g_scatter(GridDesc g, const int* __restrict__ active_list, long long n_active,
-                  const R* __restrict__ P, long long pcap, const int* __restrict__ start,
+// Scatter: one block of four warps per active bucket.  The bucket's particles
+// (key cells in the bucket: one contiguous run of the sorted arrays) are staged
+// in batches: their 18 per-axis weights and distances (3 axes x offsets 0 and
+// 1/2 x 3 nodes), evaluated once, and their attributes, as records in shared
+// memory.  Warps 0..2 take the x, y, z faces of every particle and warp 3 the
+// cell centres; lane l < 27 is stencil slot (l % 3, l / 3 % 3, l / 9), so the 27
+// lanes write 27 distinct nodes and a warp adds into the tile without atomics,
+// every node receiving its contributions in sorted-particle order: deterministic.
+// Requires stencil offsets in {0, 1} (checked on the host).
+//
+// Bound by instruction issue, and in small scenes by the chain of additions of
+// the fullest bucket.  One warp for all four node kinds, its particles' values
+// handed round by shuffles, took 212 warp instructions a particle and 1100
+// cycles each in turn: 4.96 ms at 256^3 (16.8M particles, FP32), 1.28 ms for 2.1M
+// in FP64, 309 us for a 16^3 dam break (512 particles a bucket).
+template <typename R>
+constexpr int kP2GBatch = sizeof(R) == 4 ? 32 : 16;  // particles staged at a time
+constexpr int kP2GRec = 52;  // a record: 3 axes x 3 nodes {w0, -d0, w5, -d5} (d = x_p - x_n),
+                             // 3 x {v_a, C_a}, {m, vol, r, -}
+template <typename R>
+struct Quad;
+template <>
+struct Quad<float> {
+  using T = float4;
+};
+template <>
+struct Quad<double> {
+  using T = double4;
+};
+
+template <typename R>
+__global__ void __launch_bounds__(128)
+    k_p2g_scatter(GridDesc g, const int* __restrict__ active_list, const R* __restrict__ P,
+                  long long pcap, const int* __restrict__ start,
                   const long long* __restrict__ key, const int* __restrict__ delta,
                   R* __restrict__ halo) {
-  __shared__ R tiles[WPB][kTileVals];
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const long long ai = (long long)blockIdx.x * WPB + wid;
-  if (ai >= n_active) return;
-  const int b = active_list[ai];
+  constexpr int NB = kP2GBatch<R>;
+  __shared__ R T[kTileVals];
+  __shared__ __align__(16) R rec[2][NB][kP2GRec];
+  __shared__ int first[2][NB][4];  // per warp: tile index of the stencil's first node
+  const int b = active_list[blockIdx.x];
   const long long n0 = (long long)b * 64;
   const int p0 = start[n0], p1 = start[n0 + 64];
   if (p1 <= p0) return;  // no particles: the merge skips this bucket
-  R* T = tiles[wid];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const R bs = (R)g.bs, dx = (R)g.dx;
   const R invh = R(1) / dx;
   const R rmin = dx * (R)kLiquidPhiRadius;
   const R three_bs = R(3) * bs;
-  for (int e = lane; e < kTileVals; e += 32) T[e] = e < 9 * kHaloF + kHaloC ? R(0) : three_bs;
-  __syncwarp();
+  for (int e = tid; e < kTileVals; e += 128) T[e] = e < 9 * kHaloF + kHaloC ? R(0) : three_bs;
   const int bk = b / (g.ni * g.nj);
   const int rem = b - bk * g.ni * g.nj;
   const int bj = rem / g.ni;
   const int bi = rem - bj * g.ni;
-  // weight lane (lane < 18): axis, offset (0 or 1/2), stencil node
-  const int wq = lane / 6, wo = (lane / 3) & 1, wn = lane % 3;
-  const R worg = wq == 0 ? (R)g.ox : (wq == 1 ? (R)g.oy : (R)g.oz);
-  const int wb4 = 4 * (wq == 0 ? bi : (wq == 1 ? bj : bk));
-  // slot lane (lane < 27)
-  const int si = lane % 3, sj = (lane / 3) % 3, sk = lane / 9;
-  const bool slot = lane < 27;
-  R* Tc = T + 9 * kHaloF;
-  R* Tphi = Tc + kHaloC;
-  for (int s0 = p0; s0 < p1; s0 += 32) {
-    const int s = s0 + lane;
-    R mine[kNumPCols];
-    int mdl = 0, mkl = 0;
-    if (s < p1) {
+  // staging: thread (particle, part): parts 0..2 an axis (weights, distances, the
+  // velocity and affine row), part 3 the rest
+  const int sp = tid % NB, part = tid / NB;
+  const R sorg = part == 0 ? (R)g.ox : (part == 1 ? (R)g.oy : (R)g.oz);
+  const int sb4 = 4 * (part == 0 ? bi : (part == 1 ? bj : bk));
+  R in[5];
+  int dl = 0, kl = 0;
+  auto load = [&](int s0) {
+    const int s = s0 + sp;
+    if (part < 4 && s < p1) {
+      dl = delta[s];
+      kl = (int)(key[s] & 63);
+      if (part < 3) {
+        in[0] = P[(PX + part) * pcap + s];
+        in[1] = P[(VX + part) * pcap + s];
 #pragma unroll
-      for (int c = 0; c < kNumPCols; ++c) mine[c] = P[c * pcap + s];
-      mdl = delta[s];
-      mkl = (int)(key[s] & 63);
+        for (int q = 0; q < 3; ++q) in[2 + q] = P[(C00 + 3 * part + q) * pcap + s];
+      } else {
+        in[0] = P[PM * pcap + s];
+        in[1] = P[PV * pcap + s];
+        in[2] = P[PR * pcap + s];
+      }
+    }
+  };
+  auto store = [&](int s0, int buf) {
+    if (part >= 4 || s0 + sp >= p1) return;
+    R* o = rec[buf][sp];
+    if (part < 3) {
+      const int cl = part == 0 ? (kl & 3) : (part == 1 ? ((kl >> 2) & 3) : (kl >> 4));
+      const int base = sb4 + cl - 1;
+      const int off0 = unpack_delta(dl, part);
+#pragma unroll
+      for (int n = 0; n < 3; ++n) {
+        const R d0 = in[0] - coord<R>(sorg, bs, dx, base + off0 + n, R(0));
+        const R d5 = in[0] - coord<R>(sorg, bs, dx, base + n, R(0.5));
+        R* q = o + (part * 3 + n) * 4;
+        q[0] = quad_kernel<R>(d0 * invh);
+        q[1] = -d0;
+        q[2] = quad_kernel<R>(d5 * invh);
+        q[3] = -d5;
+      }
+      R* q = o + 36 + part * 4;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) q[k] = in[1 + k];
+      // halo coordinates of the first node: (c - 1) - (4B - 1), one on along the
+      // face's own axis where the stencil offset says so
+      first[buf][sp][part] = halo_face(part, (kl & 3) + (part == 0 ? off0 : 0),
+                                       ((kl >> 2) & 3) + (part == 1 ? off0 : 0),
+                                       (kl >> 4) + (part == 2 ? off0 : 0));
     } else {
-#pragma unroll
-      for (int c = 0; c < kNumPCols; ++c) mine[c] = R(0);
+      R* q = o + 48;
+      q[0] = in[0];
+      q[1] = in[1];
+      q[2] = in[2];
+      first[buf][sp][3] = halo_centre(kl & 3, (kl >> 2) & 3, kl >> 4);
     }
-    const int cnt = min(32, p1 - s0);
-    for (int q = 0; q < cnt; ++q) {
-      R pc[kNumPCols];
-#pragma unroll
-      for (int c = 0; c < kNumPCols; ++c) pc[c] = __shfl_sync(full, mine[c], q);
-      const int dl = __shfl_sync(full, mdl, q);
-      const int kl = __shfl_sync(full, mkl, q);
-      const int cl0 = kl & 3, cl1 = (kl >> 2) & 3, cl2 = kl >> 4;  // key cell in the bucket
-      R wv = R(0), dv = R(0);
-      if (lane < 18) {
-        const int clq = wq == 0 ? cl0 : (wq == 1 ? cl1 : cl2);
-        const int node = wb4 + clq - 1 + (wo == 0 ? unpack_delta(dl, wq) : 0) + wn;
-        const R np = coord<R>(worg, bs, dx, node, wo ? R(0.5) : R(0));
-        dv = (wq == 0 ? pc[PX] : (wq == 1 ? pc[PY] : pc[PZ])) - np;
-        wv = quad_kernel<R>(dv * invh);
+  };
+  // slot lane: where its three per-axis weights sit in a record (offset 0 on a
+  // face's own axis, 1/2 elsewhere)
+  const int si = lane % 3, sj = (lane / 3) % 3, sk = lane < 27 ? lane / 9 : 0;
+  const int rx = si * 4 + (wid == 0 ? 0 : 2);
+  const int ry = (3 + sj) * 4 + (wid == 1 ? 0 : 2);
+  const int rz = (6 + sk) * 4 + (wid == 2 ? 0 : 2);
+  const bool slot = lane < 27;
+  const int nx = wid == 0 ? 7 : 6, ny = wid == 1 ? 7 : 6;  // extents of the warp's halo
+  const int sl = (sk * ny + sj) * nx + si;  // this slot's node after the first
+  R* const Tw = T + 3 * wid * kHaloF + sl;  // faces: mass, momentum, volume; centres: volume, phi
+  using Q4 = typename Quad<R>::T;
+  load(p0);
+  store(p0, 0);
+  __syncthreads();
+  int buf = 0;
+  for (int s0 = p0; s0 < p1; s0 += NB, buf ^= 1) {
+    load(s0 + NB);
+    const int cnt = min(NB, p1 - s0);
+    if (slot) {
+      for (int q = 0; q < cnt; ++q) {
+        const R* o = rec[buf][q];
+        R* const t = Tw + first[buf][q][wid];
+        const R wx = o[rx], dxx = o[rx + 1], wy = o[ry], dy = o[ry + 1], wz = o[rz],
+                dz = o[rz + 1];
+        const Q4 at = *reinterpret_cast<const Q4*>(o + 48);
+        const R w = (wx * wy) * wz;
+        if (wid < 3) {
+          const Q4 vc = *reinterpret_cast<const Q4*>(o + 36 + 4 * wid);
+          // (a zero weight adds +-0 to each sum, which leaves it unchanged: the
+          // same sums as k_p2g's skip of such weights)
+          const R vel = vc.x + (vc.y * dxx + vc.z * dy) + vc.w * dz;
+          t[0] += at.x * w;
+          t[kHaloF] += vel * at.x * w;
+          t[2 * kHaloF] += at.y * w;
+        } else {
+          // liquid level set over every particle of the 27 key cells around the
+          // node, liquid volume over the positive weights
+          const R r = at.z;
+          const R d = sqrt((dxx * dxx + dy * dy) + dz * dz) - (rmin > r ? rmin : r);
+          if (d < t[kHaloC]) t[kHaloC] = d;
+          t[0] += at.y * w;
+        }
+        // (the 27 lanes write 27 nodes, and a lane reads back only what it wrote
+        // or what another lane wrote a particle before)
+        __syncwarp(0x7ffffffu);
       }
-      const R w0x = __shfl_sync(full, wv, si), w5x = __shfl_sync(full, wv, 3 + si);
-      const R w0y = __shfl_sync(full, wv, 6 + sj), w5y = __shfl_sync(full, wv, 9 + sj);
-      const R w0z = __shfl_sync(full, wv, 12 + sk), w5z = __shfl_sync(full, wv, 15 + sk);
-      const R d0x = __shfl_sync(full, dv, si), d5x = __shfl_sync(full, dv, 3 + si);
-      const R d0y = __shfl_sync(full, dv, 6 + sj), d5y = __shfl_sync(full, dv, 9 + sj);
-      const R d0z = __shfl_sync(full, dv, 12 + sk), d5z = __shfl_sync(full, dv, 15 + sk);
-      if (slot) {
-        // halo coordinates of this slot's cell-centre node: (c - 1 + s) - (4B - 1)
-        const int hx = cl0 + si, hy = cl1 + sj, hz = cl2 + sk;
-        const R m = pc[PM], vol = pc[PV];
-        // faces: offset 0 on the face's own axis; x_n - x_p = -(x_p - x_n)
-        // (a zero weight adds +-0 to each sum, which leaves it unchanged:
-        // the same sums as k_p2g's skip of non-positive weights)
-        {
-          const R w = (w0x * w5y) * w5z;
-          const R vel = pc[VX] + (pc[C00] * (-d0x) + pc[C01] * (-d5y)) + pc[C02] * (-d5z);
-          const int t = halo_face(0, hx + unpack_delta(dl, 0), hy, hz);
-          T[t] += m * w;
-          T[kHaloF + t] += vel * m * w;
-          T[2 * kHaloF + t] += vol * w;
-        }
-        {
-          const R w = (w5x * w0y) * w5z;
-          const R vel = pc[VY] + (pc[C10] * (-d5x) + pc[C11] * (-d0y)) + pc[C12] * (-d5z);
-          const int t = halo_face(1, hx, hy + unpack_delta(dl, 1), hz);
-          T[3 * kHaloF + t] += m * w;
-          T[4 * kHaloF + t] += vel * m * w;
-          T[5 * kHaloF + t] += vol * w;
-        }
-        {
-          const R w = (w5x * w5y) * w0z;
-          const R vel = pc[VZ] + (pc[C20] * (-d5x) + pc[C21] * (-d5y)) + pc[C22] * (-d0z);
-          const int t = halo_face(2, hx, hy, hz + unpack_delta(dl, 2));
-          T[6 * kHaloF + t] += m * w;
-          T[7 * kHaloF + t] += vel * m * w;
-          T[8 * kHaloF + t] += vol * w;
-        }
-        // cell centre: liquid level set over every particle of the 27 key
-        // cells around the node, liquid volume over the positive weights
-        {
-          const int t = halo_centre(hx, hy, hz);
-          const R r = pc[PR];
-          const R d = sqrt((d5x * d5x + d5y * d5y) + d5z * d5z) - (rmin > r ? rmin : r);
-          if (d < Tphi[t]) Tphi[t] = d;
-          const R w = (w5x * w5y) * w5z;
-          Tc[t] += vol * w;
-        }
-      }
-      __syncwarp();
     }
+    store(s0 + NB, buf ^ 1);
+    __syncthreads();
   }
   R* H = halo + (long long)b * kTileVals;
-  for (int e = lane; e < kTileVals; e += 32) H[e] = T[e];
+  for (int e = tid; e < kTileVals; e += 128) H[e] = T[e];
 }
 
 // Merge: one block per active bucket, threads [0,64) u-faces, [64,128)

@@ -853,13 +853,11 @@ static cudaError_t map_particles_to_grid_t(Context& c) {
   const Walls w = make_walls(c);
   const bool elasto = c.ne > 0;
   if (tiled_transfers(c)) {
-    constexpr int wpb = sizeof(R) == 4 ? 4 : 2;  // warps (buckets) per block: 43 KB of tiles
     WCG_TRY(c.p2g_halo.ensure((size_t)c.g.nb * kTileVals * sizeof(R)));
-    ++c.launches, k_p2g_scatter<R, wpb><<<(unsigned)((c.n_active + wpb - 1) / wpb), 32 * wpb, 0,
-                                          c.stream>>>(
-        c.g, c.active_list.as<int>(), c.n_active, c.pbuf[c.cur].as<R>(), c.pcap,
-        c.cell_start.as<int>(), c.pkey.as<long long>() + c.cur * c.pcap,
-        c.pdelta.as<int>() + c.cur * c.pcap, c.p2g_halo.as<R>());
+    ++c.launches, k_p2g_scatter<R><<<(unsigned)c.n_active, 128, 0, c.stream>>>(
+        c.g, c.active_list.as<int>(), c.pbuf[c.cur].as<R>(), c.pcap, c.cell_start.as<int>(),
+        c.pkey.as<long long>() + c.cur * c.pcap, c.pdelta.as<int>() + c.cur * c.pcap,
+        c.p2g_halo.as<R>());
     // the merge writes the solid face weights too
     ++c.launches, k_p2g_merge<R><<<(unsigned)c.n_active, 256, 0, c.stream>>>(
         c.g, c.active_list.as<int>(), c.active.as<unsigned char>(), c.cell_start.as<int>(),
