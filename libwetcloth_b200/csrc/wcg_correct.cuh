@@ -162,8 +162,17 @@ __global__ void k_correct_project(GridDesc g, R* __restrict__ P, long long pcap,
   int KI, KJ, KK;
   node_ijk(g, kn, KI, KJ, KK);
   const int kp[3] = {KI - 1, KJ - 1, KK - 1};
+  // Far from the solid phi is positive and nothing moves: the stencil's nodes lie
+  // within sqrt(3) dx of its middle one and phi is a distance (3 dx in inactive
+  // buckets).  (1.03 ms with the 27 nodes summed for every eighth particle of
+  // the 256^3 half box.)
+  const int dls = delta[s];
+  const int M[3] = {KI + unpack_delta(dls, 0), KJ + unpack_delta(dls, 1), KK + unpack_delta(dls, 2)};
+  if (in_grid(g, M[0], M[1], M[2]) && active[bucket_of(g, M[0], M[1], M[2])] &&
+      F[G_SPHI * fstride + node_linear(g, M[0], M[1], M[2])] > R(2.5) * (R)g.dx)
+    return;
   R phi, gr[3];
-  solid_sample<R>(g, active, F, fstride, kp, delta[s], pos, pos, phi, gr);
+  solid_sample<R>(g, active, F, fstride, kp, dls, pos, pos, phi, gr);
   const R phi_now = phi + (gr[0] * R(0) + gr[1] * R(0) + gr[2] * R(0));
   if (phi_now < R(0))
     for (int a = 0; a < 3; ++a) P[(PX + a) * pcap + s] = pos[a] - phi_now * gr[a];

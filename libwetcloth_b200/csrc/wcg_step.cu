@@ -210,18 +210,37 @@ __global__ void k_load_particles(long long n, long long pcap, const double* x3,
 
 // scatter sorted state back to original particle order: x3 at out[0, 3n),
 // v3 at out[3n, 6n), C9 at out[6n, 15n), each in the caller's layout so the
-// copies out are contiguous
+// copies out are contiguous.  A block's particles go through shared memory, so
+// that consecutive lanes write consecutive values of a particle (and of its
+// neighbour where the original order follows the sorted one): with a thread
+// writing the 15 values of its own particle, each store touched 32 sectors
+// (1.69 ms for 16.8M particles).
+constexpr int kStoreThreads = 256;
 template <typename R>
-__global__ void k_store_particles(long long n, long long pcap, const R* P,
-                                  const int* pid, double* out) {
-  const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  const long long i = pid[s];
-  for (int a = 0; a < 3; ++a) {
-    out[i * 3 + a] = (double)P[(PX + a) * pcap + s];
-    out[3 * n + i * 3 + a] = (double)P[(VX + a) * pcap + s];
+__global__ void __launch_bounds__(kStoreThreads)
+    k_store_particles(long long n, long long pcap, const R* __restrict__ P,
+                      const int* __restrict__ pid, double* __restrict__ out) {
+  __shared__ R sv[15][kStoreThreads + 1];
+  __shared__ int sid[kStoreThreads];
+  const long long s0 = (long long)blockIdx.x * kStoreThreads;
+  const int m = (int)(n - s0 < kStoreThreads ? n - s0 : kStoreThreads);
+  if ((int)threadIdx.x < m) {
+    const long long s = s0 + threadIdx.x;
+    sid[threadIdx.x] = pid[s];
+#pragma unroll
+    for (int q = 0; q < 15; ++q) sv[q][threadIdx.x] = P[q * pcap + s];  // PX .. C22
   }
-  for (int q = 0; q < 9; ++q) out[6 * n + i * 9 + q] = (double)P[(C00 + q) * pcap + s];
+  __syncthreads();
+  for (int e = threadIdx.x; e < 3 * m; e += kStoreThreads) {
+    const int k = e / 3, a = e - 3 * k;
+    const long long i = sid[k];
+    out[i * 3 + a] = (double)sv[a][k];
+    out[3 * n + i * 3 + a] = (double)sv[3 + a][k];
+  }
+  for (int e = threadIdx.x; e < 9 * m; e += kStoreThreads) {
+    const int k = e / 9, a = e - 9 * k;
+    out[6 * n + (long long)sid[k] * 9 + a] = (double)sv[6 + a][k];
+  }
 }
 
 // positions in the reference's m_x layout (x, y, z, twist = 0 per particle) and
