@@ -170,6 +170,8 @@ int wcg_stage_liquid_async(wcg_ctx* ctx, long long n, const double* x3, const do
 int wcg_upload_staged(wcg_ctx* ctx);
 /* waits for every operation on the context, asynchronous copies included */
 int wcg_synchronize(wcg_ctx* ctx);
+/* the CUDA device the context lives on (-1: null context) */
+int wcg_device(const wcg_ctx* ctx);
 long long wcg_num_particles(const wcg_ctx* ctx);
 
 /* Elasto (cloth / yarn) particles, the reference's particles [0, n) ahead of
@@ -359,7 +361,7 @@ int wcg_num_substeps(wcg_ctx* ctx, double dt, int* n_out);
  * side).  With the particle correction on, the sub-step differentiated corrects the subset of the
  * correction stream's next call (wcg_set_correction_count).  Refused
  * (WCG_ERR_UNSUPPORTED) with elasto particles, the implicit viscosity, or the
- * particle split or merge on. */
+ * particle split or merge on.  The arrays are host or device memory. */
 int wcg_substep_vjp(wcg_ctx* ctx, double dt, const double* vbar3, const double* Cbar9,
                     const double* xbar3, double* vbar0, double* Cbar0, double* xbar0,
                     double* viscosity_bar);

@@ -173,6 +173,7 @@ SIGNATURES = {
                                        ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]),
     "wcg_download_liquid_async": (ctypes.c_int, [ctypes.c_void_p, _D, _D, _D]),
     "wcg_synchronize": (ctypes.c_int, [ctypes.c_void_p]),
+    "wcg_device": (ctypes.c_int, [ctypes.c_void_p]),
     "wcg_stage_liquid_async": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_longlong, _D, _D, _D, _D,
                                               _D, _D]),
     "wcg_upload_staged": (ctypes.c_int, [ctypes.c_void_p]),

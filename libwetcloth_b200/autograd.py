@@ -26,32 +26,76 @@ None, takes the scene's next call); sub-step k of a rollout takes call
 """
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import torch
+
+from . import _capi
 
 
 def _host(t):
     return t.detach().cpu().numpy().astype(np.float64)
 
 
+def _on_scene(scene, *tensors):
+    """Whether a sub-step can take these tensors where they are: all on the
+    scene's device, with as many rows as the scene has particles and finite
+    (anything else goes through the host arrays and their checks)."""
+    n = scene.num_particles
+    dev = int(scene.L.wcg_device(scene.h))
+    if not all(t.is_cuda and t.device.index == dev and t.shape[:1] == (n,) and
+               t.dtype.is_floating_point for t in tensors):
+        return False
+    return n > 0 and bool(torch.stack([torch.isfinite(t).all() for t in tensors]).all())
+
+
+def _snapshot(t, k):
+    """A float64 copy of t's values, k per particle, on t's device."""
+    return t.detach().to(torch.float64).reshape(-1, k).contiguous().clone()
+
+
+def _ptr(t):
+    return ctypes.cast(t.data_ptr(), _capi._D)
+
+
+def _load(scene, x, v, C):
+    """set_state from device tensors (masses, volumes and radii as uploaded)."""
+    if scene._attrs_dev is None or scene._attrs_dev[0].device != x.device:
+        scene._attrs_dev = tuple(torch.from_numpy(a).to(x.device) for a in scene._attrs)
+    # the library runs on the scene's own stream
+    torch.cuda.current_stream(x.device).synchronize()
+    scene.upload_device(x.shape[0], *[t.data_ptr() for t in (x, v, C, *scene._attrs_dev)])
+
+
 class _Substep(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, v, C, mu, scene, dt, substeps, call):
-        xs, vs, Cs = (_host(t) for t in (x, v, C))
         m = float(mu.detach().cpu().item()) if mu is not None else None
         if m is not None:
             scene.set_viscosity(m, substeps)
-        scene.set_state(xs, vs, Cs)
         k = scene.correction_count if call is None else int(call)
-        scene.set_correction_count(k)
-        scene.substep(dt)
         ctx.call = k
-        x1, v1, C1 = scene.download()
         ctx.scene = scene
         ctx.dt = dt
         ctx.mu = (m, substeps)
-        ctx.state = (xs, vs, Cs)
         dev = v.device
+        if _on_scene(scene, x, v, C):
+            # state already on the scene's device: the checkpoint and the results
+            # stay there (through the host, the copies were most of the call)
+            ctx.state = tuple(_snapshot(t, w) for t, w in ((x, 3), (v, 3), (C, 9)))
+            out = tuple(torch.empty_like(t) for t in ctx.state)
+            _load(scene, *ctx.state)
+            scene.set_correction_count(k)
+            scene.substep(dt)
+            _capi.check(scene.L.wcg_download_liquid_device(scene.h, *[t.data_ptr() for t in out]))
+            return out
+        xs, vs, Cs = (_host(t) for t in (x, v, C))
+        scene.set_state(xs, vs, Cs)
+        scene.set_correction_count(k)
+        scene.substep(dt)
+        x1, v1, C1 = scene.download()
+        ctx.state = (xs, vs, Cs)
         return (torch.from_numpy(x1).to(dev), torch.from_numpy(v1).to(dev),
                 torch.from_numpy(C1).to(dev))
 
@@ -67,6 +111,20 @@ class _Substep(torch.autograd.Function):
         m, substeps = ctx.mu
         if m is not None:
             scene.set_viscosity(m, substeps)
+        if isinstance(ctx.state[0], torch.Tensor):
+            where = ctx.state[0].device
+            cot = [torch.zeros((n, w), dtype=torch.float64, device=where) if g is None else
+                   g.detach().to(where, torch.float64).reshape(n, w).contiguous()
+                   for g, w in ((gv1, 3), (gC1, 9), (gx1, 3))]
+            bar = [torch.empty_like(t) for t in cot]
+            mub = ctypes.c_double(0.0)
+            _load(scene, *ctx.state)
+            scene.set_correction_count(ctx.call)
+            _capi.check(scene.L.wcg_substep_vjp(scene.h, ctx.dt, *[_ptr(t) for t in cot + bar],
+                                                ctypes.byref(mub)))
+            vb, Cb, xb = bar
+            gmu = None if m is None else torch.tensor(mub.value, dtype=torch.float64, device=dev)
+            return xb, vb, Cb, gmu, None, None, None, None
         scene.set_state(*ctx.state)
         scene.set_correction_count(ctx.call)
         vb, Cb, xb, mub = scene.substep_vjp(ctx.dt, host(gv1, 3), host(gC1, 9), host(gx1, 3),

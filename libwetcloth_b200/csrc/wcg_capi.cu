@@ -409,6 +409,8 @@ int wcg_upload_staged(wcg_ctx* ctx) {
   return WCG_OK;
 }
 
+int wcg_device(const wcg_ctx* ctx) { return ctx ? ctx->c.device : -1; }
+
 int wcg_synchronize(wcg_ctx* ctx) {
   WCG_CHECK_CTX(ctx);
   WCG_CALL(ctx, wcg::synchronize(ctx->c), "synchronize");
@@ -782,8 +784,9 @@ int wcg_substep_vjp(wcg_ctx* ctx, double dt, const double* vbar3, const double* 
            "substep_vjp");
   int st = device_status(ctx->c, "substep_vjp");
   if (st) return st;
-  if (ctx->c.adjoint_fixed_x)
-    for (long long i = 0; i < 3 * n; ++i) xbar0[i] = xbar3[i];
+  if (ctx->c.adjoint_fixed_x && n > 0 &&
+      cudaMemcpy(xbar0, xbar3, (size_t)3 * n * sizeof(double), cudaMemcpyDefault) != cudaSuccess)
+    return fail(WCG_ERR_CUDA, "substep_vjp: copy of the position cotangent");
   ctx->c.have_grid = true;
   if (!ctx->c.stats.converged)
     return fail(WCG_ERR_NOT_CONVERGED, "adjoint pressure solve did not converge");

@@ -2563,10 +2563,10 @@ static cudaError_t substep_vjp_t(Context& c, double dt, const double* vbar, cons
   WCG_TRY(c.adjp.ensure((size_t)15 * c.pcap * rb));  // B (12 columns), XB (3)
   WCG_TRY(c.adjstage.ensure((size_t)18 * np * sizeof(double)));
   double* st = c.adjstage.as<double>();
-  WCG_TRY(cudaMemcpyAsync(st, vbar, 3 * np * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-  WCG_TRY(cudaMemcpyAsync(st + 3 * np, Cbar, 9 * np * sizeof(double), cudaMemcpyHostToDevice,
+  WCG_TRY(cudaMemcpyAsync(st, vbar, 3 * np * sizeof(double), cudaMemcpyDefault, c.stream));
+  WCG_TRY(cudaMemcpyAsync(st + 3 * np, Cbar, 9 * np * sizeof(double), cudaMemcpyDefault,
                           c.stream));
-  WCG_TRY(cudaMemcpyAsync(st + 12 * np, xbar, 3 * np * sizeof(double), cudaMemcpyHostToDevice,
+  WCG_TRY(cudaMemcpyAsync(st + 12 * np, xbar, 3 * np * sizeof(double), cudaMemcpyDefault,
                           c.stream));
   R* F = c.gfield.as<R>();
   R* AG = c.adj.as<R>();
@@ -2664,12 +2664,12 @@ static cudaError_t substep_vjp_t(Context& c, double dt, const double* vbar, cons
       c.pkey.as<long long>() + c.cur * c.pcap, c.pdelta.as<int>() + c.cur * c.pcap, F, AG,
       c.gcap, st, st + 3 * np, XB, st + 15 * np, AM);
   WCG_TRY(cudaGetLastError());
-  WCG_TRY(cudaMemcpyAsync(vbar0, st, 3 * np * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-  WCG_TRY(cudaMemcpyAsync(Cbar0, st + 3 * np, 9 * np * sizeof(double), cudaMemcpyDeviceToHost,
+  WCG_TRY(cudaMemcpyAsync(vbar0, st, 3 * np * sizeof(double), cudaMemcpyDefault, c.stream));
+  WCG_TRY(cudaMemcpyAsync(Cbar0, st + 3 * np, 9 * np * sizeof(double), cudaMemcpyDefault,
                           c.stream));
   if (xbar0)
     WCG_TRY(cudaMemcpyAsync(xbar0, st + 15 * np, 3 * np * sizeof(double),
-                            cudaMemcpyDeviceToHost, c.stream));
+                            cudaMemcpyDefault, c.stream));
   return cudaStreamSynchronize(c.stream);
 }
 

@@ -93,6 +93,7 @@ class FluidScene:
         x, v, C, mass, vol, radius = map(arr, (x, v, C, mass, vol, radius))
         n = mass.shape[0]
         self._attrs = (mass, vol, radius)
+        self._attrs_dev = None  # their device copies, made by autograd when it needs them
         check(self.L.wcg_upload_liquid(self.h, n, _dp(x), _dp(v), _dp(C), _dp(mass),
                                        _dp(vol), _dp(radius)))
 

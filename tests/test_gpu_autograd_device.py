@@ -1,0 +1,62 @@
+"""autograd.substep on tensors that live on the scene's GPU against the same
+call on host tensors: the same kernels on the same values, so results and
+gradients are equal bit for bit."""
+import numpy as np
+import pytest
+
+from libwetcloth_b200 import _capi, scenes
+from libwetcloth_b200.solver import FluidScene
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _run(sc, where, precision, mu, fixed_x, dtype=torch.float64):
+    from libwetcloth_b200 import autograd
+    g = FluidScene(sc, precision=precision)
+    g.set_adjoint_positions(not fixed_x)
+    rng = np.random.default_rng(5)
+    n = sc.x.shape[0]
+    t = [torch.tensor(a, dtype=dtype, device=where, requires_grad=True)
+         for a in (sc.x, sc.v, rng.normal(0, 1, (n, 9)))]
+    m = torch.tensor(1e-3, dtype=torch.float64, device=where, requires_grad=True) if mu else None
+    cot = [torch.tensor(rng.normal(0, 1, (n, k)), device=where) for k in (3, 3, 9)]
+    out = autograd.substep(g, *t, 1e-3, viscosity=m, correction_call=2)
+    # the third output's cotangent is left out in one setting
+    used = 2 if fixed_x else 3
+    grads = torch.autograd.grad(out[:used], t + ([m] if mu else []), cot[:used])
+    res = [o.detach().cpu().numpy() for o in out] + [q.cpu().numpy() for q in grads]
+    assert all(o.device.type == where for o in out)
+    g.close()
+    return res
+
+
+@pytest.mark.parametrize("precision", [_capi.WCG_FP64, _capi.WCG_FP32_REFINE])
+@pytest.mark.parametrize("mu,fixed_x", [(False, False), (True, False), (False, True)])
+def test_device_tensors_equal_host_tensors(precision, mu, fixed_x, wcg):
+    sc = scenes.dam_break(16, 8, 0)
+    sc.v = np.random.default_rng(1).normal(0.0, 0.2, sc.x.shape)
+    a = _run(sc, "cpu", precision, mu, fixed_x)
+    b = _run(sc, "cuda", precision, mu, fixed_x)
+    assert len(a) == len(b)
+    for p, q in zip(a, b):
+        assert p.shape == q.shape and p.dtype == q.dtype and np.array_equal(p, q)
+
+
+def test_device_tensors_of_other_kinds(wcg):
+    """float32 leaves convert as on the host; non-finite input is refused with
+    the host path's error."""
+    from libwetcloth_b200 import autograd
+    sc = scenes.dam_break(16, 8, 0)
+    a = _run(sc, "cpu", _capi.WCG_FP64, False, False, torch.float32)
+    b = _run(sc, "cuda", _capi.WCG_FP64, False, False, torch.float32)
+    for p, q in zip(a, b):
+        assert np.array_equal(p, q)
+    g = FluidScene(sc)
+    x = torch.tensor(sc.x, device="cuda")
+    x[3, 1] = float("nan")
+    C = torch.zeros((x.shape[0], 9), device="cuda", dtype=torch.float64)
+    with pytest.raises(_capi.WcgError) as e:
+        autograd.substep(g, x, torch.zeros_like(x), C, 1e-3)
+    assert e.value.code == _capi.WCG_ERR_ARG
+    g.close()
