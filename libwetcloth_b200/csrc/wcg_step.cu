@@ -2738,7 +2738,7 @@ static cudaError_t correct_liquid_t(Context& c, double dt, int selector) {
   for (int t = 0; t < 2; ++t)
     for (int u = 0; u < 2; ++u)
       for (int r = 0; r < 2; ++r)
-        ++c.launches, k_correct<R><<<nblk(ncol, 128), 128, 0, c.stream>>>(
+        ++c.launches, k_correct<R><<<nblk(ncol * 32, 128), 128, 0, c.stream>>>(
             c.g, cg, r, u, t, P, c.pcap, pid, list, start,
             c.pkey.as<long long>() + c.cur * c.pcap, c.pdelta.as<int>() + c.cur * c.pcap,
             c.active.as<unsigned char>(), c.gfield.as<R>(), c.gcap, c.xw.as<R>(), selector, step,
