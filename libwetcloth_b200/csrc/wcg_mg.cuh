@@ -186,18 +186,27 @@ __global__ void __launch_bounds__(kMgCoarseThreads) k_mg_coarsest(MgLevel<R> L, 
 // The same with x in shared memory and the cells of each colour listed there,
 // for levels whose box fits (mg_coarse_smem).  A thread holds the first
 // kMgHeld cells of each colour with their couplings in registers, so a colour
-// is six reads of x, a division and a barrier; further cells take their
-// couplings from global memory.  Bound by the latency of those 2 x iters
-// colours: 1550 us per V-cycle with everything in global memory (19 x 12 x 19
-// cells, FP64; 1225 us in FP32 at 18 x 10 x 18), most of it index arithmetic and
-// cache latency.
+// is six reads of x, a division and a barrier; further cells have them in
+// shared memory as long as it lasts, the rest reads them from global memory.
+// Bound by the latency of those 2 x iters colours.  With everything in global
+// memory a V-cycle spent 1550 us here (19 x 12 x 19 cells, FP64; 1225 us in FP32
+// at 18 x 10 x 18), most of it index arithmetic and cache latency; with the
+// further cells alone there 570, now 490.
 template <typename R>
 constexpr int kMgHeld = sizeof(R) == 4 ? 2 : 1;
 template <typename R>
 __host__ __device__ constexpr size_t mg_coarse_smem(int n) {
   return ((size_t)n * sizeof(R) + 15) / 16 * 16 + (size_t)n * sizeof(int);
 }
-constexpr size_t kMgCoarseSmemMax = 200 * 1024;
+constexpr size_t kMgCoarseSmemMax = 220 * 1024;
+
+// Cells past the held ones that find a place in shared memory (8 values and an
+// index each).  FP64 alone: in FP32 twice as many cells are held, all there are
+// in a level of 4096 unless its colours differ much.
+template <typename R>
+__host__ __device__ constexpr int mg_coarse_places(int n) {
+  return sizeof(R) == 4 ? 0 : (int)((kMgCoarseSmemMax - 32 - mg_coarse_smem<R>(n)) / (8 * sizeof(R) + 2 * sizeof(int)));
+}
 
 template <typename R>
 __global__ void __launch_bounds__(kMgCoarseThreads) k_mg_coarsest_smem(MgLevel<R> L, int iters) {
@@ -254,6 +263,36 @@ __global__ void __launch_bounds__(kMgCoarseThreads) k_mg_coarsest_smem(MgLevel<R
   };
   auto cell_at = [&](int col, int t) { return col == 0 ? list[t] : list[L.n - 1 - t]; };
   constexpr int H = kMgHeld<R>;
+  // places: odd cells past the held ones, then even ones; 8 values each, strided
+  const int np = mg_coarse_places<R>(L.n);
+  R* const pv = reinterpret_cast<R*>(dsm_mg + (mg_coarse_smem<R>(L.n) + 15) / 16 * 16);
+  int* const pi = reinterpret_cast<int*>(pv + 8 * (size_t)np);  // index, existing neighbours
+  const int over0 = max(0, cnt[0] - H * kMgCoarseThreads);
+  auto put = [&](int at, const Cell& e) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) pv[k * np + at] = e.c[k];
+    pv[6 * np + at] = e.d;
+    pv[7 * np + at] = e.b;
+    pi[at] = e.idx;
+    pi[np + at] = e.m;
+  };
+  auto get = [&](int at) {
+    Cell e;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) e.c[k] = pv[k * np + at];
+    e.d = pv[6 * np + at];
+    e.b = pv[7 * np + at];
+    e.idx = pi[at];
+    e.m = pi[np + at];
+    return e;
+  };
+  constexpr bool kPlaces = sizeof(R) == 8;
+  if constexpr (kPlaces)
+    for (int col = 0; col < 2; ++col)
+      for (int t = threadIdx.x + H * kMgCoarseThreads; t < cnt[col]; t += kMgCoarseThreads) {
+        const int at = t - H * kMgCoarseThreads + (col ? over0 : 0);
+        if (at < np) put(at, take(cell_at(col, t)));
+      }
   Cell held[2][H];
 #pragma unroll
   for (int col = 0; col < 2; ++col)
@@ -268,8 +307,11 @@ __global__ void __launch_bounds__(kMgCoarseThreads) k_mg_coarsest_smem(MgLevel<R
 #pragma unroll
       for (int h = 0; h < H; ++h)
         if ((int)threadIdx.x + h * kMgCoarseThreads < cnt[col]) relax(held[col][h]);
-      for (int t = threadIdx.x + H * kMgCoarseThreads; t < cnt[col]; t += kMgCoarseThreads)
-        relax(take(cell_at(col, t)));
+      for (int t = threadIdx.x + H * kMgCoarseThreads; t < cnt[col]; t += kMgCoarseThreads) {
+        // (its own place: no barrier between put and get)
+        const int at = t - H * kMgCoarseThreads + (col ? over0 : 0);
+        relax(kPlaces && at < np ? get(at) : take(cell_at(col, t)));
+      }
       __syncthreads();
     }
   for (int idx = threadIdx.x; idx < L.n; idx += blockDim.x)

@@ -1980,7 +1980,8 @@ static cudaError_t mg_vcycle(Context& c, R* z, R* r) {
     ++c.launches, k_mg_restrict<R><<<mg_blocks(L[l + 1].n), kMgThreads, 0, c.stream>>>(L[l], L[l + 1]);
   }
   const size_t cs = mg_coarse_smem<R>(L[nlev - 1].n);
-  if (cs <= kMgCoarseSmemMax) {
+  if (cs + 64 <= kMgCoarseSmemMax) {
+    const size_t smem = mg_coarse_places<R>(L[nlev - 1].n) > 0 ? kMgCoarseSmemMax : cs;
     static std::atomic<unsigned long long> attr_set{0};  // once per device, as in pl_sweep
     const unsigned long long dbit = 1ull << (c.device & 63);
     if (!(attr_set.load(std::memory_order_acquire) & dbit)) {
@@ -1989,8 +1990,8 @@ static cudaError_t mg_vcycle(Context& c, R* z, R* r) {
                                    (int)kMgCoarseSmemMax));
       attr_set.fetch_or(dbit, std::memory_order_release);
     }
-    ++c.launches, k_mg_coarsest_smem<R><<<1, kMgCoarseThreads, cs, c.stream>>>(L[nlev - 1],
-                                                                              kMgCoarseSweeps);
+    ++c.launches, k_mg_coarsest_smem<R><<<1, kMgCoarseThreads, smem, c.stream>>>(
+        L[nlev - 1], kMgCoarseSweeps);
   } else {
     ++c.launches, k_mg_coarsest<R><<<1, kMgCoarseThreads, 0, c.stream>>>(L[nlev - 1],
                                                                          kMgCoarseSweeps);
