@@ -1,0 +1,64 @@
+"""The one-launch CSR factorisation and triangular solves at their edges.
+
+Rows are handed out in blocks of 256 and solved in order of their
+dependencies, four terms of a row at a time.  The matrices have one row fewer
+and one more than a block, rows of no, four and five and many lower entries, an
+empty row, and chains that cross every block.  The oracle's MIC(0)-PCG runs the
+same recurrences; its dot products sum in another order, so the iterates differ
+by rounding, and both stop at a residual of 1e-11 max|b|: they agree to that
+times the inverse's norm, at most 10 for diagonals that exceed the row's other
+entries by 0.1, here 1e-9 of the largest entry with a factor of ten to spare."""
+import numpy as np
+import pytest
+
+from libwetcloth_b200 import _capi
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-11
+
+
+def _matrix(n, kind, seed=0):
+    rng = np.random.default_rng(seed)
+    pairs = set()
+    if kind == "chain":  # every row waits for the one before
+        pairs |= {(i, i - 1) for i in range(1, n)}
+    elif kind == "wide":  # 0 to 8 lower entries a row
+        for i in range(n):
+            for j in rng.choice(i, min(i, i % 9), replace=False) if i else ():
+                pairs.add((i, int(j)))
+    else:  # "arrow": the last rows hold an entry of every fifth column
+        pairs |= {(i, i - 1) for i in range(1, n) if i % 3}
+        for i in range(max(1, n - 2), n):
+            pairs |= {(i, j) for j in range(0, i, 5)}
+    rows = [{} for _ in range(n)]
+    empty = n // 2 if n > 2 else -1
+    for i, j in pairs:
+        if empty not in (i, j):
+            rows[i][j] = rows[j][i] = -rng.uniform(0.2, 1.0)
+    start, col, val = [0], [], []
+    for i, r in enumerate(rows):
+        if i != empty:
+            r[i] = sum(abs(v) for v in r.values()) + rng.uniform(0.1, 1.0)
+        for j in sorted(r):
+            col.append(j)
+            val.append(r[j])
+        start.append(len(col))
+    b = rng.standard_normal(n)
+    if empty >= 0:
+        b[empty] = 0.0
+    return np.array(start, np.int64), np.array(col, np.int64), np.array(val), b
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 256, 257, 513, 1025])
+@pytest.mark.parametrize("kind", ["chain", "wide", "arrow"])
+def test_dataflow_edges_match_oracle(n, kind, wcg):
+    rs, col, val, b = _matrix(n, kind, n)
+    xg, resg, itg, st = _capi.pcg_solve_csr(rs, col, val, b, TOL, 500)
+    xo, ok, ito, _ = oracle.pcg_solve(rs, col, val, b, TOL, 500)
+    assert ok and st == _capi.WCG_OK and abs(itg - ito) <= 1
+    assert resg <= TOL * np.abs(b).max()
+    assert np.abs(xg - xo).max() <= 1e-9 * np.abs(xo).max()
+    # the same bits again, on fresh buffers
+    assert np.array_equal(xg, _capi.pcg_solve_csr(rs, col, val, b, TOL, 500)[0])

@@ -1,10 +1,10 @@
 """The strip-wise MIC(0) sweeps at the edges of their tiles.
 
-A patch is 16 x 16 lines, a strip 16 x 2, a staging ring 16 (FP32) or 8 (FP64)
-rows, a strip's inbox 16 and 32 rows.  The blocks below give DOF boxes of one
-line fewer and one more than those, boxes shorter than a ring, and one line
-across.  The tile wavefront (WCG_PCG_LAYOUT=tiles) solves the same system with
-the same recurrences; the pencil layout's three lower terms are subtracted in
+A patch is 16 x 16 lines, a strip 16 x 2; a lane takes two cells of its line per
+step and a strip stages chunks of two steps, three or four ahead.  The blocks
+below give DOF boxes of one line fewer and one more than those, of odd and even
+length, shorter than a ring, and one line across.  The tile wavefront
+(WCG_PCG_LAYOUT=tiles) solves the same system with the same recurrences; the pencil layout's three lower terms are subtracted in
 another order, so two solves to the criterion 1e-12 agree to 1e-10 of the
 largest pressure in FP64 (residual 1e-12 times a condition number below 1e2 at
 these sizes); in FP32 the coefficients are rounded to 6e-8 in both and the
