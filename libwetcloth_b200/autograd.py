@@ -68,6 +68,19 @@ def _load(scene, x, v, C):
     scene.upload_device(x.shape[0], *[t.data_ptr() for t in (x, v, C, *scene._attrs_dev)])
 
 
+def _read(scene, device):
+    """The scene's particle state as new tensors on its device.  The count is
+    the scene's after the sub-step: the split, the merge, a terminator and the
+    removal of particles without volume change it."""
+    n = scene.num_particles
+    out = tuple(torch.empty((n, w), dtype=torch.float64, device=device) for w in (3, 3, 9))
+    # memory that the allocator hands out again may have work pending on this
+    # stream; the library writes on its own
+    torch.cuda.current_stream(device).synchronize()
+    _capi.check(scene.L.wcg_download_liquid_device(scene.h, *[t.data_ptr() for t in out]))
+    return out
+
+
 class _Substep(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, v, C, mu, scene, dt, substeps, call):
@@ -84,12 +97,10 @@ class _Substep(torch.autograd.Function):
             # state already on the scene's device: the checkpoint and the results
             # stay there (through the host, the copies were most of the call)
             ctx.state = tuple(_snapshot(t, w) for t, w in ((x, 3), (v, 3), (C, 9)))
-            out = tuple(torch.empty_like(t) for t in ctx.state)
             _load(scene, *ctx.state)
             scene.set_correction_count(k)
             scene.substep(dt)
-            _capi.check(scene.L.wcg_download_liquid_device(scene.h, *[t.data_ptr() for t in out]))
-            return out
+            return _read(scene, x.device)
         xs, vs, Cs = (_host(t) for t in (x, v, C))
         scene.set_state(xs, vs, Cs)
         scene.set_correction_count(k)

@@ -60,3 +60,38 @@ def test_device_tensors_of_other_kinds(wcg):
         autograd.substep(g, x, torch.zeros_like(x), C, 1e-3)
     assert e.value.code == _capi.WCG_ERR_ARG
     g.close()
+
+
+@pytest.mark.parametrize("change", ["split", "merge", "terminator", "empty"])
+def test_particle_count_of_the_results(change, wcg):
+    """A sub-step that changes the number of particles returns as many rows as
+    the scene holds after it, on the device as on the host."""
+    from libwetcloth_b200 import autograd
+
+    def run(where):
+        sc = scenes.dam_break(16, 8, 0)
+        if change in ("split", "merge"):
+            scenes.mixed_volumes(sc, 3, mrel=(0.3, 0.7, 1.0, 2.5, 5.0))
+            sc.params.particle_split = change == "split"
+            sc.params.particle_merge = change == "merge"
+        if change == "empty":
+            sc.vol[5:50] = 0.0
+        g = FluidScene(sc)
+        if change == "terminator":
+            g.set_terminators([{"type": "sphere", "inside": True, "center": sc.x.mean(0),
+                                "param": (0.1,)}])
+        n = g.num_particles
+        if change == "merge":  # it works on the grid of a sub-step before
+            g.substep(1e-3)
+            g.set_state(sc.x, sc.v, np.zeros((n, 9)))
+        t = [torch.tensor(a, dtype=torch.float64, device=where)
+             for a in (sc.x, sc.v, np.zeros((n, 9)))]
+        out = [o.cpu().numpy() for o in autograd.substep(g, *t, 1e-3, correction_call=1)]
+        assert all(o.shape[0] == g.num_particles != n for o in out) and g.num_particles > 0
+        now = g.download()
+        g.close()
+        assert all(np.array_equal(o, a) for o, a in zip(out, now))
+        return out
+
+    for p, q in zip(run("cpu"), run("cuda")):
+        assert p.shape == q.shape and np.array_equal(p, q)
