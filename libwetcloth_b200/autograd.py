@@ -38,16 +38,21 @@ def _host(t):
     return t.detach().cpu().numpy().astype(np.float64)
 
 
-def _on_scene(scene, *tensors):
-    """Whether a sub-step can take these tensors where they are: all on the
-    scene's device, with as many rows as the scene has particles and finite
-    (anything else goes through the host arrays and their checks)."""
+def _on_scene(scene, x, v, C):
+    """Whether a sub-step can take these tensors where they are: on the scene's
+    device, 3, 3 and 9 finite values for every particle that the scene holds
+    and that has a mass, volume and radius from the last upload (anything else
+    goes through the host arrays and their checks)."""
     n = scene.num_particles
     dev = int(scene.L.wcg_device(scene.h))
-    if not all(t.is_cuda and t.device.index == dev and t.shape[:1] == (n,) and
-               t.dtype.is_floating_point for t in tensors):
+    attrs = scene._attrs
+    if n <= 0 or attrs is None or any(a is None or a.size != n for a in attrs):
         return False
-    return n > 0 and bool(torch.stack([torch.isfinite(t).all() for t in tensors]).all())
+    if not all(t.is_cuda and t.device.index == dev and t.shape[:1] == (n,) and
+               t.numel() == n * w and t.dtype.is_floating_point
+               for t, w in ((x, 3), (v, 3), (C, 9))):
+        return False
+    return bool(torch.stack([torch.isfinite(t).all() for t in (x, v, C)]).all())
 
 
 def _snapshot(t, k):
@@ -61,11 +66,14 @@ def _ptr(t):
 
 def _load(scene, x, v, C):
     """set_state from device tensors (masses, volumes and radii as uploaded)."""
+    n = x.shape[0]
+    if scene._attrs is None or any(a.size != n for a in scene._attrs):
+        raise ValueError(f"the scene's masses, volumes and radii are not those of {n} particles")
     if scene._attrs_dev is None or scene._attrs_dev[0].device != x.device:
         scene._attrs_dev = tuple(torch.from_numpy(a).to(x.device) for a in scene._attrs)
     # the library runs on the scene's own stream
     torch.cuda.current_stream(x.device).synchronize()
-    scene.upload_device(x.shape[0], *[t.data_ptr() for t in (x, v, C, *scene._attrs_dev)])
+    scene.upload_device(n, *[t.data_ptr() for t in (x, v, C, *scene._attrs_dev)])
 
 
 def _read(scene, device):

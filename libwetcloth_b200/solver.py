@@ -71,6 +71,8 @@ class FluidScene:
         check(self.L.wcg_create(ctypes.byref(prm), ctypes.byref(h)))
         self.h = h
         self.precision = prm.precision
+        self._attrs = None      # mass, volume and radius as last uploaded from the host
+        self._attrs_dev = None  # their device copies, made by autograd when it needs them
         if scene is not None:
             self.upload(scene.x, scene.v, scene.C, scene.mass, scene.vol, scene.radius)
             if getattr(scene, "elasto", None) is not None:
@@ -92,14 +94,20 @@ class FluidScene:
         arr = lambda a: None if a is None else np.ascontiguousarray(a, dtype=np.float64).reshape(-1)
         x, v, C, mass, vol, radius = map(arr, (x, v, C, mass, vol, radius))
         n = mass.shape[0]
+        for name, a, k in (("x", x, 3), ("v", v, 3), ("C", C, 9), ("vol", vol, 1),
+                           ("radius", radius, 1)):
+            if a is not None and a.size < n * k:
+                raise ValueError(f"{name}: {a.size} values for {n} particles")
         self._attrs = (mass, vol, radius)
-        self._attrs_dev = None  # their device copies, made by autograd when it needs them
+        self._attrs_dev = None
         check(self.L.wcg_upload_liquid(self.h, n, _dp(x), _dp(v), _dp(C), _dp(mass),
                                        _dp(vol), _dp(radius)))
 
     def set_state(self, x, v, C):
         """Replace the liquid particles' positions, velocities and affine
         matrices (mass, volume and radius as last uploaded)."""
+        if self._attrs is None:
+            raise ValueError("set_state: no masses, volumes and radii uploaded from the host")
         self.upload(x, v, C, *self._attrs)
 
     def substep_vjp(self, dt, vbar, Cbar, xbar, with_viscosity=False):

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from libwetcloth_b200 import _capi, scenes
-from libwetcloth_b200.solver import FluidScene
+from libwetcloth_b200.solver import FluidScene, make_params
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -95,3 +95,41 @@ def test_particle_count_of_the_results(change, wcg):
 
     for p, q in zip(run("cpu"), run("cuda")):
         assert p.shape == q.shape and np.array_equal(p, q)
+
+
+def test_widths_and_masses_are_checked(wcg):
+    """Tensors of another width, and a scene whose masses are of another
+    particle set, do not reach the device route: what the host arrays can take
+    gives the same as on the host, the rest is refused."""
+    from libwetcloth_b200 import autograd
+    sc = scenes.dam_break(16, 8, 0)
+    n = sc.x.shape[0]
+    wide = np.concatenate([sc.x, sc.v], 1)  # (n, 6): the first 3 n values are taken
+    wide.reshape(-1)[:3 * n] = sc.x.reshape(-1)
+    res = []
+    for where in ("cpu", "cuda"):
+        g = FluidScene(sc)
+        x, v, C = (torch.tensor(a, device=where) for a in (sc.x, sc.v, np.zeros((n, 9))))
+        res.append([o.cpu().numpy() for o in autograd.substep(
+            g, torch.tensor(wide, device=where), v, C, 1e-3, correction_call=0)])
+        for bad in ((x, v, C[:, :3]), (x, v[:, :1], C), (x[:-1], v, C)):
+            with pytest.raises(ValueError):
+                autograd.substep(g, *bad, 1e-3)
+        g.close()
+    assert all(p.shape == q.shape and np.array_equal(p, q) for p, q in zip(*res))
+    # more particles than masses, uploaded from the device
+    g = FluidScene(scenes.dam_break(12, 8, 0))
+    dev = [torch.tensor(a, device="cuda") for a in (sc.x, sc.v, np.zeros((n, 9)), sc.mass, sc.vol,
+                                                   sc.radius)]
+    g.upload_device(n, *[t.data_ptr() for t in dev])
+    m = g._attrs[0].size
+    assert m < n == g.num_particles
+    out = autograd.substep(g, *dev[:3], 1e-3, correction_call=0)
+    assert all(o.shape[0] == m for o in out)  # the host route: the particles with masses
+    g.close()
+    # masses never uploaded from the host
+    g = FluidScene(None, params=make_params(sc.params))
+    g.upload_device(n, *[t.data_ptr() for t in dev])
+    with pytest.raises(ValueError):
+        autograd.substep(g, *dev[:3], 1e-3)
+    g.close()

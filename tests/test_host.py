@@ -105,3 +105,42 @@ def test_replica_timing_reduction_gloo():
     for p in ps:
         p.join(timeout=60)
     assert sorted(res) == [(0, 20.0), (1, 20.0)]
+
+
+def test_device_substep_takes_whole_particles_only():
+    """autograd's device route hands raw pointers to the library: only tensors
+    of 3, 3 and 9 values for each particle of the scene, which has as many
+    masses, may take it."""
+    import types
+
+    import torch
+
+    from libwetcloth_b200 import autograd
+
+    class Tensor:  # what the rule looks at before it asks for the values
+        is_cuda, dtype, device = True, torch.float64, types.SimpleNamespace(index=0)
+
+        def __init__(self, *shape):
+            self.shape = torch.Size(shape)
+
+        def numel(self):
+            return self.shape.numel()
+
+    def scene(n, attrs):
+        L = types.SimpleNamespace(wcg_device=lambda h: 0)
+        return types.SimpleNamespace(num_particles=n, L=L, h=None, _attrs=attrs)
+
+    def ask(n, attrs, *shapes):
+        return autograd._on_scene(scene(n, attrs), *[Tensor(*s) for s in shapes])
+
+    ones = [np.ones(6)] * 3
+    good = ((6, 3), (6, 3), (6, 9))
+    for k, bad in ((0, (6, 6)), (1, (6, 1)), (2, (6, 3)), (0, (18,)), (0, (7, 3)), (2, (6,))):
+        assert not ask(6, ones, *good[:k], bad, *good[k + 1:])
+    assert not ask(6, None, *good)                      # masses never uploaded
+    assert not ask(6, [np.ones(5)] * 3, *good)          # masses of another set
+    assert not ask(6, [np.ones(6), None, np.ones(6)], *good)
+    assert not ask(0, [np.ones(0)] * 3, (0, 3), (0, 3), (0, 9))
+    # the state of a checkpoint against masses uploaded since
+    with pytest.raises(ValueError):
+        autograd._load(scene(6, [np.ones(5)] * 3), Tensor(6, 3), None, None)
