@@ -23,7 +23,8 @@
 // Rows are handed out to blocks by an atomic ticket in the order of the
 // dependencies (ascending, or descending for the backward solve), so whatever
 // a row waits for belongs to a block that started earlier or to its own.  Every
-// wait is bounded.
+// wait is bounded: it ends when no row of the launch has got on for some millions
+// of rounds (Patience), however long the chain of rows before it is.
 // Products and sums are rounded separately (_rn intrinsics), as the
 // reference's compiled code evaluates them.  Dot products are deterministic
 // block reductions; their summation order is not Eigen's, so the iterates
@@ -165,8 +166,51 @@ __device__ inline int ld_acquire(const int* p) {
 __device__ inline void st_release(int* p, int v) {
   asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-// rounds without progress before a wait gives up (well over a second)
-constexpr long long kMaxRounds = 1ll << 22;
+__device__ inline int ld_relaxed(const int* p) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// How long a warp waits.  The last rows of a long chain are resident from the
+// start and idle until the chain reaches them (a band of 24 over 60 000 rows:
+// seconds), so a wait does not end after a number of its own rounds but once the
+// whole launch has stood still for that long: every elimination of the
+// factorisation and every finished row of a solve adds to `progress`, and a warp
+// that idles looks there every kLook rounds.  What may pass between two additions
+// is the walk over one row's entries (two rows' in an elimination), at a few
+// rounds each: the limit has room for the longest.  A warp that gives up sets
+// `err`, and all others follow.  (The additions cost 0.5 of 34 ms on a 40^3 grid;
+// a clock read in every round that got on, to add less often, 1.5.)
+constexpr long long kMaxRounds = 1ll << 22;  // a third of a second at the least
+constexpr int kLook = 1024;
+
+struct Patience {
+  int* progress;
+  int* err;
+  long long limit;
+  long long idle = 0;
+  int round = 0, seen = 0;
+  __device__ Patience(int* progress_, int* err_, int longest_row)
+      : progress(progress_), err(err_), limit(kMaxRounds + 16ll * longest_row) {}
+  // a round without progress of the warp's own (all its lanes call): true once
+  // the wait is over
+  __device__ bool over() {
+    if (++round & (kLook - 1)) return false;
+    int p = 0, e = 0;
+    if ((threadIdx.x & 31) == 0) {
+      p = ld_relaxed(progress);
+      e = ld_relaxed(err);
+    }
+    p = __shfl_sync(0xffffffffu, p, 0);
+    if (__shfl_sync(0xffffffffu, e, 0)) return true;
+    idle = p == seen ? idle + kLook : 0;
+    seen = p;
+    if (idle <= limit) return false;
+    if ((threadIdx.x & 31) == 0) atomicExch(err, 1);
+    return true;
+  }
+};
 
 // The eliminations of column k (finished) in column j: mult is the entry of
 // row j in column k, d the running pivot of column j.
@@ -229,7 +273,7 @@ __global__ void __launch_bounds__(kThreads)
                  const int* __restrict__ urow, double* uval, const int* __restrict__ tstart,
                  const int* __restrict__ tk, const int* __restrict__ tp,
                  const double* __restrict__ adiag, double* __restrict__ invdiag, int* ready,
-                 int* err) {
+                 int* progress, int* err, int longest_row) {
   __shared__ int s_block;
   if (threadIdx.x == 0) s_block = atomicAdd(ticket, 1);
   __syncthreads();
@@ -238,7 +282,7 @@ __global__ void __launch_bounds__(kThreads)
   int q = fin ? 0 : tstart[j];
   const int eq = fin ? 0 : tstart[j + 1];
   double d = fin ? 0.0 : adiag[j];
-  long long idle = 0;
+  Patience wait(progress, err, longest_row);
   // lanes of a warp may depend on one another: every round lets each lane do
   // what it can, so the lanes that are ready go on
   while (__any_sync(0xffffffffu, !fin)) {
@@ -251,6 +295,7 @@ __global__ void __launch_bounds__(kThreads)
           moved = true;
         } else if (ld_acquire(ready + k)) {
           d = eliminate(j, k, __ldcg(uval + tp[q]), d, rowstart, col, ustart, urow, uval);
+          atomicAdd(progress, 1);
           ++q;
           moved = true;
         }
@@ -268,16 +313,12 @@ __global__ void __launch_bounds__(kThreads)
         moved = true;
       }
     }
-    if (__any_sync(0xffffffffu, moved)) {
-      idle = 0;
-    } else if (++idle > kMaxRounds) {
-      atomicExch(err, 1);
-      fin = true;
-    }
+    if (!__any_sync(0xffffffffu, moved) && wait.over()) fin = true;
   }
 }
 
-// scalar slots (doubles); SC_DONE holds an int: 1 converged, 2 iteration limit
+// scalar slots (doubles); SC_DONE holds an int: 1 converged, 2 iteration limit,
+// 3 a wait gave up
 enum : int { SC_RHO = 0, SC_RES, SC_ITER, SC_DONE, SC_ALPHA, SC_BETA, SC_TOL, SC_MAXIT, kNumSc };
 
 // solve_lower (PCGSolver.h:211-222, LOWER) or solve_lower_transpose_in_place
@@ -295,7 +336,8 @@ __global__ void __launch_bounds__(kTriThreads, 1)
     k_csr_tri(int n, int* ticket, int ticket_base, unsigned tag, const int* __restrict__ start,
               const int* __restrict__ dep, const int* __restrict__ pos,
               const double* __restrict__ uval, const double* __restrict__ invdiag,
-              const double* in, double* out, u64* words, const double* __restrict__ sc, int* err) {
+              const double* in, double* out, u64* words, const double* __restrict__ sc,
+              int* progress, int* err, int longest_row) {
   __shared__ u64 sw[2 * kTriThreads];
   __shared__ int s_block;
   constexpr unsigned full = 0xffffffffu;
@@ -334,7 +376,7 @@ __global__ void __launch_bounds__(kTriThreads, 1)
     }
   };
   if (!fin) next_terms();
-  long long idle = 0;
+  Patience wait(progress, err, longest_row);
   while (!__all_sync(full, fin)) {
     bool moved = false;
     // terms from other blocks, all loads in flight at once
@@ -385,6 +427,7 @@ __global__ void __launch_bounds__(kTriThreads, 1)
             st_word(words + 2ll * row, w0);
             st_word(words + 2ll * row + 1, w1);
             out[row] = y;
+            atomicAdd(progress, 1);
             fin = true;
           }
         }
@@ -392,12 +435,7 @@ __global__ void __launch_bounds__(kTriThreads, 1)
       again = __any_sync(full, step);
       moved = moved || again;
     } while (again);
-    if (__any_sync(full, moved)) {
-      idle = 0;
-    } else if (++idle > kMaxRounds) {
-      if (!fin) atomicExch(err, 1);
-      fin = true;
-    }
+    if (!__any_sync(full, moved) && wait.over()) fin = true;
   }
 }
 
@@ -495,10 +533,12 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// the last block: rho_new = z.r, beta = rho_new / rho (init: rho alone)
+// the last block: rho_new = z.r, beta = rho_new / rho (init: rho alone), and the
+// end of the solve where a wait of the factorisation or of a triangular solve
+// before it gave up
 __global__ void __launch_bounds__(kThreads)
     k_csr_dot(int n, const double* __restrict__ z, const double* __restrict__ r, double* sc,
-              double* part, int* ctr, int init) {
+              double* part, int* ctr, const int* __restrict__ err, int init) {
   __shared__ double sm[kThreads];
   if (*(const int*)(sc + SC_DONE)) return;
   double acc = 0.0;
@@ -508,6 +548,7 @@ __global__ void __launch_bounds__(kThreads)
   if (grid_reduce(acc, part, ctr, sm, false, &rho) && threadIdx.x == 0) {
     if (!init) sc[SC_BETA] = __ddiv_rn(rho, sc[SC_RHO]);
     sc[SC_RHO] = rho;
+    if (*err) *(int*)(sc + SC_DONE) = 3;
   }
 }
 
@@ -529,16 +570,19 @@ struct Solver {
   u64* words;
   unsigned tag = 0;   // of the last triangular solve
   int tickets = 0;    // handed out by the triangular solves so far
+  int longest = 0;    // entries of the longest row
 
   // ctl: 0 malformed matrix, 1 wait given up, 2 reduction count, 3 ticket of
-  // the triangular solves, 4 ticket of the factorisation
+  // the triangular solves, 4 ticket of the factorisation, 5 progress of the rows
   void precondition(const double* in, double* out) {
     const int nb = (n + kTriThreads - 1) / kTriThreads;
     k_csr_tri<true><<<nb, kTriThreads, 0, st>>>(n, ctl + 3, tickets, ++tag, tstart, tk, tp, uval,
-                                                invdiag, in, out, words, sc, ctl + 1);
+                                                invdiag, in, out, words, sc, ctl + 5, ctl + 1,
+                                                longest);
     tickets += nb;
     k_csr_tri<false><<<nb, kTriThreads, 0, st>>>(n, ctl + 3, tickets, ++tag, ustart, urow, nullptr,
-                                                 uval, invdiag, out, out, words, sc, ctl + 1);
+                                                 uval, invdiag, out, out, words, sc, ctl + 5,
+                                                 ctl + 1, longest);
     tickets += nb;
   }
   unsigned grid() const { return std::min(nblocks(n), (unsigned)kDotBlocks); }
@@ -614,6 +658,7 @@ cudaError_t csr_solve(const int* h_rowstart, const int* h_col, const double* h_v
   std::vector<int> rs(h_rowstart, h_rowstart + n + 1);
   const int base = rs[0];
   for (int& v : rs) v -= base;
+  for (int i = 0; i < n; ++i) S.longest = std::max(S.longest, rs[i + 1] - rs[i]);
   CSR_TRY(cudaMemcpyAsync(S.rowstart, rs.data(), ib, cudaMemcpyHostToDevice, st));
   CSR_TRY(cudaMemcpyAsync(S.col, h_col + base, nnz * sizeof(int), cudaMemcpyHostToDevice, st));
   CSR_TRY(cudaMemcpyAsync(S.val, h_val + base, nnz * sizeof(double), cudaMemcpyHostToDevice, st));
@@ -653,13 +698,16 @@ cudaError_t csr_solve(const int* h_rowstart, const int* h_col, const double* h_v
     CSR_TRY(cudaMemcpyAsync(S.sc + SC_TOL, lim, sizeof(lim), cudaMemcpyHostToDevice, st));
     k_csr_factor<<<nblocks(n), kThreads, 0, st>>>(n, S.ctl + 4, S.rowstart, S.col, S.ustart, S.urow,
                                                   S.uval, S.tstart, S.tk, S.tp, S.adiag, S.invdiag,
-                                                  ready, S.ctl + 1);
+                                                  ready, S.ctl + 5, S.ctl + 1, S.longest);
     S.precondition(S.r, S.z);
-    k_csr_dot<<<S.grid(), kThreads, 0, st>>>(n, S.z, S.r, S.sc, S.part, S.ctl + 2, 1);
+    k_csr_dot<<<S.grid(), kThreads, 0, st>>>(n, S.z, S.r, S.sc, S.part, S.ctl + 2, S.ctl + 1, 1);
     CSR_TRY(cudaGetLastError());
-    double rho = 0.0;
-    CSR_TRY(S.read(&rho, SC_RHO, 1));
-    if (!(rho == 0.0 || rho != rho) && maxiter > 0) {
+    double h0[4];
+    CSR_TRY(S.read(h0, SC_RHO, 4));  // rho, residual, iterations, done
+    const double rho = h0[0];
+    int done0;
+    std::memcpy(&done0, &h0[3], sizeof(done0));
+    if (!done0 && !(rho == 0.0 || rho != rho) && maxiter > 0) {
       CSR_TRY(cudaMemcpyAsync(S.s, S.z, vb, cudaMemcpyDeviceToDevice, st));
       for (;;) {
         for (int k = 0; k < kCheck; ++k) {
@@ -668,7 +716,8 @@ cudaError_t csr_solve(const int* h_rowstart, const int* h_col, const double* h_v
           k_csr_update_xr<<<S.grid(), kThreads, 0, st>>>(n, S.s, S.z, S.x, S.r, S.sc, S.part,
                                                          S.ctl + 2);
           S.precondition(S.r, S.z);
-          k_csr_dot<<<S.grid(), kThreads, 0, st>>>(n, S.z, S.r, S.sc, S.part, S.ctl + 2, 0);
+          k_csr_dot<<<S.grid(), kThreads, 0, st>>>(n, S.z, S.r, S.sc, S.part, S.ctl + 2, S.ctl + 1,
+                                                   0);
           k_csr_direction<<<S.grid(), kThreads, 0, st>>>(n, S.z, S.s, S.sc);
         }
         CSR_TRY(cudaGetLastError());

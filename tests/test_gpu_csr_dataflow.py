@@ -1,9 +1,10 @@
 """The one-launch CSR factorisation and triangular solves at their edges.
 
-Rows are handed out in blocks of 256 and solved in order of their
-dependencies, four terms of a row at a time.  The matrices have one row fewer
-and one more than a block, rows of no, four and five and many lower entries, an
-empty row, and chains that cross every block.  The oracle's MIC(0)-PCG runs the
+Rows are handed out in blocks (256 of them in the factorisation, 1024 in the
+triangular solves) and solved in order of their dependencies, four terms of a
+row at a time.  The matrices have one row fewer and one more than a block of
+either kind, rows of no, four and five and many lower entries, an empty row,
+and chains that cross every block.  The oracle's MIC(0)-PCG runs the
 same recurrences; its dot products sum in another order, so the iterates differ
 by rounding, and both stop at a residual of 1e-11 max|b|: they agree to that
 times the inverse's norm, at most 10 for diagonals that exceed the row's other
@@ -51,7 +52,7 @@ def _matrix(n, kind, seed=0):
     return np.array(start, np.int64), np.array(col, np.int64), np.array(val), b
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 256, 257, 513, 1025])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 256, 257, 513, 1023, 1024, 1025, 2049, 5000])
 @pytest.mark.parametrize("kind", ["chain", "wide", "arrow"])
 def test_dataflow_edges_match_oracle(n, kind, wcg):
     rs, col, val, b = _matrix(n, kind, n)
@@ -62,3 +63,32 @@ def test_dataflow_edges_match_oracle(n, kind, wcg):
     assert np.abs(xg - xo).max() <= 1e-9 * np.abs(xo).max()
     # the same bits again, on fresh buffers
     assert np.array_equal(xg, _capi.pcg_solve_csr(rs, col, val, b, TOL, 500)[0])
+
+
+def _band(n, w):
+    """Symmetric, diagonally dominant, every row coupled to its w neighbours on
+    either side."""
+    rng = np.random.default_rng(n + w)
+    off = np.zeros((n, 2 * w + 1))
+    on = np.zeros(off.shape, bool)
+    for d in range(1, w + 1):
+        u = -rng.uniform(0.2, 1.0, n - d)
+        off[d:, w - d], off[:n - d, w + d] = u, u
+        on[d:, w - d] = on[:n - d, w + d] = True
+    off[:, w] = np.abs(off).sum(1) + rng.uniform(0.1, 1.0, n)
+    on[:, w] = True
+    col = (np.arange(n)[:, None] + np.arange(-w, w + 1))[on]
+    return np.concatenate([[0], np.cumsum(on.sum(1))]), col, off[on], rng.standard_normal(n)
+
+
+def test_long_chain_of_wide_rows(wcg):
+    """A band of 24 over 60 000 rows: every column waits for the one before, and
+    the last ones, resident from the start, wait for seconds.  The band has no
+    dropped entries, so the factor is the Cholesky factor: one iteration, as
+    the oracle takes."""
+    rs, col, val, b = _band(60000, 24)
+    xg, resg, itg, st = _capi.pcg_solve_csr(rs, col, val, b, TOL, 20)
+    xo, ok, ito, _ = oracle.pcg_solve(rs, col, val, b, TOL, 20)
+    assert ok and st == _capi.WCG_OK and itg == ito
+    assert resg <= TOL * np.abs(b).max()
+    assert np.abs(xg - xo).max() <= 1e-9 * np.abs(xo).max()
