@@ -69,20 +69,15 @@ struct Mem {
     if (e_ != cudaSuccess) return e_;    \
   } while (0)
 
-// rows must list strictly ascending columns in [0, n); counts the upper
-// entries of each row (the factor's column) and takes the diagonal
+// rows (whose bounds the host has checked) must list strictly ascending columns in
+// [0, n); counts the upper entries of each row (the factor's column) and takes the
+// diagonal
 __global__ void k_csr_rows(int n, const int* __restrict__ rowstart, const int* __restrict__ col,
                            const double* __restrict__ val, int* __restrict__ ucount,
                            double* __restrict__ adiag, int* bad) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int s = rowstart[i], e = rowstart[i + 1];
-  if (e < s) {
-    atomicExch(bad, 1);
-    ucount[i] = 0;
-    adiag[i] = 0.0;
-    return;
-  }
   int prev = -1, cnt = 0;
   double d = 0.0;
   for (int p = s; p < e; ++p) {
@@ -760,8 +755,10 @@ extern "C" int wcg_pcg_solve_csr(const int* rowstart, const int* col, const doub
   *residual_out = 0.0;
   *iterations_out = 0;
   if (n == 0) return WCG_OK;
-  if (rowstart[n] < rowstart[0])
-    return wcg::set_last_error(WCG_ERR_ARG, "wcg_pcg_solve_csr: rowstart decreases");
+  // no row may reach outside [rowstart[0], rowstart[n]): the kernels read what it names
+  for (int i = 0; i < n; ++i)
+    if (rowstart[i + 1] < rowstart[i])
+      return wcg::set_last_error(WCG_ERR_ARG, "wcg_pcg_solve_csr: rowstart decreases");
   int outcome = 0;
   const cudaError_t e = wcg::csr_solve(rowstart, col, val, n, rhs, x, tolerance_factor,
                                        max_iterations, residual_out, iterations_out, &outcome);
@@ -771,7 +768,7 @@ extern "C" int wcg_pcg_solve_csr(const int* rowstart, const int* col, const doub
   if (outcome == 2)
     return wcg::set_last_error(WCG_ERR_ARG,
                                "wcg_pcg_solve_csr: rows must hold strictly ascending columns "
-                               "in [0, n) and rowstart must not decrease");
+                               "in [0, n)");
   if (outcome == 3)
     return wcg::set_last_error(WCG_ERR_DEVICE,
                                "wcg_pcg_solve_csr: a row reached its wait limit");

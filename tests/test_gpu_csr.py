@@ -186,6 +186,17 @@ def test_pcg_solve_csr_rejects_malformed(wcg):
     assert it.value == 0
 
 
+def test_pcg_solve_csr_rejects_rows_out_of_range(wcg):
+    """A rowstart that decreases anywhere, so that a row before it reaches past
+    the arrays, is refused before any device work."""
+    col = np.array([0, 1, 1], np.int32)
+    val = np.array([4.0, -1.0, 4.0])
+    for rs in ([0, 1 << 28, 3], [0, 4, 3], [2, 0, 3], [0, -5, 3]):
+        with pytest.raises(_capi.WcgError) as e:
+            _capi.pcg_solve_csr(np.array(rs, np.int32), col, val, np.ones(2), 1e-8, 10)
+        assert e.value.code == _capi.WCG_ERR_ARG
+
+
 @pytest.mark.gpu
 def test_pcg_solve_csr_rejects_unsorted_rows(wcg):
     rs = np.array([0, 2, 4], np.int32)
