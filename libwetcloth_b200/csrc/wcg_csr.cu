@@ -50,6 +50,7 @@ constexpr double kMinRatio = 0.25;  // min_diagonal_ratio (:101)
 constexpr int kThreads = 256;
 constexpr int kDotBlocks = 296;     // 2 per SM of a B200
 constexpr int kCheck = 8;           // iterations per look at the stop test
+constexpr long long kOneAlloc = 8 << 20;  // entries up to which a solve allocates once
 
 inline unsigned nblocks(long long n) { return (unsigned)((n + kThreads - 1) / kThreads); }
 
@@ -601,39 +602,48 @@ cudaError_t csr_solve(const int* h_rowstart, const int* h_col, const double* h_v
   } guard{S.st};
   cudaStream_t st = S.st;
   const long long nnz = (long long)h_rowstart[n] - h_rowstart[0];
-  // one allocation for everything (the factor has at most nnz entries)
+  // One allocation, or two for more than kOneAlloc entries: the factor's columns
+  // hold the entries right of the diagonal, whose number comes from the device.  (A
+  // second allocation, its release and the wait cost 0.7 of 35 ms at 0.45M entries;
+  // the room for all entries at most 160 MB.)
   const size_t vb = (size_t)n * sizeof(double), ib = (size_t)(n + 1) * sizeof(int);
   const size_t scan_b = (size_t)((n + 1 + kScanTile - 1) / kScanTile + 1) * sizeof(int);
-  Mem mem;
+  Mem mem, factor;
   size_t total = 0;
   auto place = [&](size_t bytes) {
     const size_t at = total;
     total += (bytes + 255) & ~(size_t)255;
     return at;
   };
-  const size_t o_rs = place(ib), o_col = place(nnz * sizeof(int)), o_val = place(nnz * sizeof(double));
-  const size_t o_us = place(ib), o_ur = place(nnz * sizeof(int)), o_uv = place(nnz * sizeof(double));
-  const size_t o_ts = place(ib), o_tk = place(nnz * sizeof(int)), o_tp = place(nnz * sizeof(int));
+  const size_t o_rs = place(ib), o_col = place(nnz * sizeof(int)),
+               o_val = place(nnz * sizeof(double));
+  const size_t o_us = place(ib), o_ts = place(ib);
   const size_t o_ad = place(vb), o_id = place(vb);
   const size_t o_x = place(vb), o_r = place(vb), o_z = place(vb), o_s = place(vb);
   const size_t o_part = place(kDotBlocks * sizeof(double)), o_tmp = place(scan_b);
-  // zeroed: counters, the transpose counts and cursors, the ready flags, the
-  // words of the triangular solves, the scalars
+  struct FactorPlace {
+    size_t uval, urow, tk, tp;
+  };
+  auto place_factor = [&](size_t k) {
+    return FactorPlace{place(k * sizeof(double)), place(k * sizeof(int)), place(k * sizeof(int)),
+                       place(k * sizeof(int))};
+  };
+  FactorPlace fp{};
+  if (nnz <= kOneAlloc) fp = place_factor(nnz);
+  // zeroed: counters, the ready flags, the scalars, and the words of the
+  // triangular solves (16 bytes a row), whose place the transpose counts and cursors
+  // have first (4 (n + 1) bytes each)
+  const size_t wb = 2 * (size_t)n * sizeof(u64);
   const size_t o_zero = total;
-  const size_t o_ctl = place(8 * sizeof(int)), o_tc = place(ib), o_tcur = place(ib);
-  const size_t o_rdy = place(ib), o_w = place(2 * (size_t)n * sizeof(u64));
-  const size_t o_sc = place(kNumSc * sizeof(double));
+  const size_t o_ctl = place(8 * sizeof(int)), o_rdy = place(ib);
+  const size_t o_sc = place(kNumSc * sizeof(double)), o_w = place(wb);
   CSR_TRY(mem.alloc(total));
   unsigned char* const m = mem.as<unsigned char>();
   S.rowstart = (int*)(m + o_rs);
   S.col = (int*)(m + o_col);
   S.val = (double*)(m + o_val);
   S.ustart = (int*)(m + o_us);
-  S.urow = (int*)(m + o_ur);
-  S.uval = (double*)(m + o_uv);
   S.tstart = (int*)(m + o_ts);
-  S.tk = (int*)(m + o_tk);
-  S.tp = (int*)(m + o_tp);
   S.adiag = (double*)(m + o_ad);
   S.invdiag = (double*)(m + o_id);
   S.x = (double*)(m + o_x);
@@ -645,8 +655,8 @@ cudaError_t csr_solve(const int* h_rowstart, const int* h_col, const double* h_v
   S.words = (u64*)(m + o_w);
   S.sc = (double*)(m + o_sc);
   int* const tmp = (int*)(m + o_tmp);
-  int* const tcount = (int*)(m + o_tc);
-  int* const tcur = (int*)(m + o_tcur);
+  int* const tcount = (int*)(m + o_w);
+  int* const tcur = tcount + n + 1;
   int* const ready = (int*)(m + o_rdy);
   CSR_TRY(cudaMemsetAsync(m + o_zero, 0, total - o_zero, st));
   // rowstart relative to its first entry
@@ -660,20 +670,35 @@ cudaError_t csr_solve(const int* h_rowstart, const int* h_col, const double* h_v
   // the upper counts of the rows go to tstart's place until they are scanned
   int* const ucount = S.tstart;
   k_csr_rows<<<nblocks(n), kThreads, 0, st>>>(n, S.rowstart, S.col, S.val, ucount, S.adiag, S.ctl);
-  int hctl[2] = {0, 0};
+  // factor columns: the upper parts of the rows
+  exclusive_scan<int, int>(ucount, n, S.ustart, tmp, S.ustart + n, st);
+  int hctl[2] = {0, 0}, nu = 0;
   CSR_TRY(cudaMemcpyAsync(hctl, S.ctl, sizeof(int), cudaMemcpyDeviceToHost, st));
+  if (nnz > kOneAlloc)
+    CSR_TRY(cudaMemcpyAsync(&nu, S.ustart + n, sizeof(int), cudaMemcpyDeviceToHost, st));
   CSR_TRY(cudaStreamSynchronize(st));
   if (hctl[0]) {
     *outcome = 2;
     return cudaSuccess;
   }
-  // factor columns (upper parts of the rows) and their transpose
-  exclusive_scan<int, int>(ucount, n, S.ustart, tmp, S.ustart + n, st);
+  unsigned char* f = m;
+  if (nnz > kOneAlloc) {
+    total = 0;
+    fp = place_factor(nu);
+    CSR_TRY(factor.alloc(total));
+    f = factor.as<unsigned char>();
+  }
+  S.uval = (double*)(f + fp.uval);
+  S.urow = (int*)(f + fp.urow);
+  S.tk = (int*)(f + fp.tk);
+  S.tp = (int*)(f + fp.tp);
+  // their entries and their transpose
   k_csr_upper<<<nblocks(n), kThreads, 0, st>>>(n, S.rowstart, S.col, S.val, S.ustart, S.urow,
                                                S.uval, tcount);
   exclusive_scan<int, int>(tcount, n, S.tstart, tmp, S.tstart + n, st);
   k_csr_transpose<<<nblocks(n), kThreads, 0, st>>>(n, S.ustart, S.urow, S.tstart, tcur, S.tk, S.tp);
   k_csr_sort_transpose<<<nblocks(n), kThreads, 0, st>>>(n, S.tstart, S.tk, S.tp);
+  CSR_TRY(cudaMemsetAsync(S.words, 0, wb, st));
   CSR_TRY(cudaGetLastError());
 
   // PCG

@@ -92,3 +92,44 @@ def test_long_chain_of_wide_rows(wcg):
     assert ok and st == _capi.WCG_OK and itg == ito
     assert resg <= TOL * np.abs(b).max()
     assert np.abs(xg - xo).max() <= 1e-9 * np.abs(xo).max()
+
+
+def test_device_memory_of_a_solve(wcg):
+    """The factor and its transpose take the entries right of the diagonal, not
+    all: per entry of the matrix 12 bytes, per entry of the factor 20, per row
+    80 and a little (a pollster sees the least free memory while the solve
+    runs; 10 % for granularity)."""
+    torch = pytest.importorskip("torch")
+    import threading
+    import time
+    blocks, w = 6000, 80  # dense blocks: chains of 80 rows
+    n = blocks * w
+    rng = np.random.default_rng(0)
+    B = -rng.uniform(0.2, 1.0, (w, w))
+    B = B + B.T
+    np.fill_diagonal(B, np.abs(B).sum(1) + 1.0)
+    val = np.tile(B.reshape(-1), blocks)
+    col = (np.arange(blocks, dtype=np.int32)[:, None, None] * w +
+           np.arange(w, dtype=np.int32)[None, None] + np.zeros((1, w, 1), np.int32)).reshape(-1)
+    rs = np.arange(n + 1, dtype=np.int32) * w
+    b = rng.standard_normal(n)
+    _capi.pcg_solve_csr(rs[:w + 1], col[:w * w], val[:w * w], b[:w], TOL, 20)  # the context
+    free, _ = torch.cuda.mem_get_info()
+    least, done = [free], threading.Event()
+
+    def watch():
+        while not done.is_set():
+            least[0] = min(least[0], torch.cuda.mem_get_info()[0])
+            time.sleep(5e-4)
+
+    t = threading.Thread(target=watch)
+    t.start()
+    try:
+        x, res, it, st = _capi.pcg_solve_csr(rs, col, val, b, TOL, 20)
+    finally:
+        done.set()
+        t.join()
+    assert st == _capi.WCG_OK and res <= TOL * np.abs(b).max()
+    nnz, nu = n * w, blocks * w * (w - 1) // 2
+    used = free - least[0]
+    assert 0.9 * (12 * nnz + 20 * nu) <= used <= 1.1 * (12 * nnz + 20 * nu + 84 * n)
