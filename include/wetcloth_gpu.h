@@ -374,10 +374,11 @@ int wcg_set_viscosity(wcg_ctx* ctx, double viscosity, int substeps);
 
 /* Failure handling of the MIC(0) wavefront (no reference counterpart; the
  * reference's triangular solves are serial and never wait).  Each poll of a
- * wavefront edge word is bounded by spin_limit polls (default 2^20); a wait
- * that reaches it records a device error, the sweep finishes with zeros in
- * place of the missing values, and the call returns WCG_ERR_DEVICE -- the
- * context stays usable.  stale_patch >= 0 makes that patch of the pencil
+ * wavefront edge word is bounded by spin_limit polls (default 2^20), and each
+ * wait inside a block for such a word by 64 spin_limit polls of shared memory (at
+ * least 2^24, at most 2^31 - 1); a wait that reaches its limit records a device
+ * error, the sweep finishes with zeros in place of the missing values, and the
+ * call returns WCG_ERR_DEVICE -- the context stays usable.  stale_patch >= 0 makes that patch of the pencil
  * layout (indices past the last patch mean the last one) wait for a tag that
  * no producer writes, so a test can run the limit out on purpose; -1 turns
  * it off. */

@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -158,6 +159,15 @@ struct PencilGeom {
   long long npatch;      // nPA * nPC
   long long len;         // elements per array (npatch * R * 2 * lines per patch)
 };
+
+// Polls of a word or a count in shared memory before a strip or a receiver of the
+// sweeps gives up: longer than the waits in front of it, which follow spin_limit
+// (a poll of L2 takes about 20 times one of shared memory), so that no one gives
+// up on a wait that may still end; at most 2^31 - 1, a minute or more.
+constexpr int inbox_polls(long long spin_limit) {
+  const long long polls = spin_limit < (1ll << 18) ? 1ll << 24 : 64 * spin_limit;
+  return (int)(polls < INT_MAX ? polls : INT_MAX);
+}
 
 // Arrays of the pencil layout (Reals, len each; PL64_* are doubles).
 // PL_COEF spans four arrays: the MIC(0) factor, per step of a strip four rows

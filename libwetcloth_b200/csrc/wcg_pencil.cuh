@@ -179,6 +179,7 @@ struct PencilSweepArgs {
   int red_init;          // backward: the first z.r of a solve (beta = 0)
   int npart;             // partials (groups)
   long long spin_limit;  // polls of an edge word before the wait gives up
+  int box_polls;         // and of a word or a count in shared memory (inbox_polls)
   int stale_patch;       // failure-path test: this patch waits for a tag nothing
                          // writes (-1: none)
 };
@@ -230,7 +231,6 @@ __host__ __device__ constexpr int sweep_inc() {
   return sizeof(R) == 4 ? 16 : 8;
 }
 constexpr int kRecv = 4;   // steps a receiver lane polls at once
-constexpr long long kInboxPolls = 1ll << 24;  // bound of a wait in shared memory
 
 // chunks of a strip in flight or in use (one CTA per SM: 96 KB of FP32 or 144 KB
 // of FP64 cells, enough for the latency of HBM at its full rate)
@@ -512,7 +512,7 @@ __device__ __forceinline__ void pencil_sweep_run(const PencilSweepArgs<R>& A, in
               record_error(A.err, kErrWaitTimeout);
               gave_up = true;
             }
-          } else if (v < rows && ++idle > kInboxPolls) {
+          } else if (v < rows && ++idle > A.box_polls) {
             // the strip no longer takes words (its own wait gave up)
             record_error(A.err, kErrWaitTimeout);
             v = rows;
@@ -643,11 +643,11 @@ __device__ __forceinline__ void pencil_sweep_run(const PencilSweepArgs<R>& A, in
         const unsigned tag = (unsigned)(v + 1);
         unsigned off = (words_off<EW>(wc, tag) & mc) | (words_off<EW>(wa, tag) & ma);
         if (__any_sync(full, off != 0)) {
-          long long it = 0;
+          int it = 0;
           do {
             load_words(v);
             off = (words_off<EW>(wc, tag) & mc) | (words_off<EW>(wa, tag) & ma);
-            if (++it > kInboxPolls) {
+            if (++it > A.box_polls) {
               if (lane == 0) record_error(A.err, kErrWaitTimeout);
               gave_up = true;
             }
@@ -770,9 +770,9 @@ __device__ __forceinline__ void pencil_sweep_run(const PencilSweepArgs<R>& A, in
         load_step(slot, 1, f1);
         if (to_box && v0 >= taken + kInC && !gave_up) {
           // the next strip has to take its steps first
-          long long it = 0;
+          int it = 0;
           while (v0 >= (taken = look()) + kInC) {
-            if (++it > kInboxPolls) {
+            if (++it > A.box_polls) {
               if (lane == 0) record_error(A.err, kErrWaitTimeout);
               gave_up = true;
               break;

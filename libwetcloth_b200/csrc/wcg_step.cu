@@ -1390,6 +1390,7 @@ static PencilSweepArgs<R> pl_args(Context& c) {
   a.min_ratio = (R)0.25;
   a.err = c.derr.as<int>();
   a.spin_limit = c.spin_limit;
+  a.box_polls = inbox_polls(c.spin_limit);
   a.stale_patch = c.stale_patch < 0 ? -1 : (int)std::min<long long>(c.stale_patch,
                                                                      c.plg.npatch - 1);
   return a;

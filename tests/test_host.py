@@ -144,3 +144,27 @@ def test_device_substep_takes_whole_particles_only():
     # the state of a checkpoint against masses uploaded since
     with pytest.raises(ValueError):
         autograd._load(scene(6, [np.ones(5)] * 3), Tensor(6, 3), None, None)
+
+
+def test_inner_waits_outlast_the_wait_limit(tmp_path):
+    """A strip of the sweeps waits in shared memory for words that a receiver
+    brings, and the receiver's own wait follows the limit of
+    wcg_set_wait_limit (polls of L2, some 20 times as long as one of shared
+    memory): the strip's limit is longer, up to the 2^31 - 1 polls that it ends
+    at."""
+    from libwetcloth_b200 import build
+    nvcc = build.nvcc()
+    if not os.path.exists(nvcc):
+        pytest.skip("no nvcc")
+    limits = [1, 200, (1 << 18) - 1, 1 << 18, 1 << 20, 1 << 30, 1 << 40]
+    src = tmp_path / "polls.cu"
+    src.write_text('#include "%s/wcg_context.h"\n#include <cstdio>\nint main() {\n%s}\n' % (
+        build.CSRC, "".join(f'  std::printf("%lld\\n", (long long)wcg::inbox_polls({v}ll));\n' for v in limits)))
+    exe = tmp_path / "polls"
+    subprocess.run([nvcc, "-std=c++17", "-arch=sm_100a", "-o", str(exe), str(src)], check=True,
+                   timeout=300)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
+    polls = [int(v) for v in out]
+    assert polls == sorted(polls)
+    for v, p in zip(limits, polls):
+        assert 1 << 24 <= p < 1 << 31 and p >= min(32 * v, (1 << 31) - 1)
