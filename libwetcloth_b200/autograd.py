@@ -10,7 +10,9 @@ and the advection), the liquid phi behind the ghost-fluid fractions and the
 solid projection of the particle correction; the grid's discrete structure
 (activation, DOFs, valid faces) is held at the checkpoint's values.  The
 scene's particle state after backward is the checkpoint of the last node
-differentiated.
+differentiated.  Tensors on the scene's device stay there, and so does their
+checkpoint while half of the device's memory is free; every other
+checkpoint is held on the host.
 
 ``rollout(scene, x, v, C, dt, steps, viscosity, checkpoint_every)`` runs
 ``steps`` sub-steps as one node that keeps only every ``checkpoint_every``-th
@@ -38,11 +40,34 @@ def _host(t):
     return t.detach().cpu().numpy().astype(np.float64)
 
 
+_ASK = 256 << 20  # bytes of checkpoints that a scene makes between two looks at the memory
+
+
+def _room(scene, device, nbytes):
+    """Whether a checkpoint of nbytes may stay on the device: half of its memory
+    is left to everything else, so a chain of any length still fits (its later
+    nodes keep their checkpoints on the host).  The driver is asked once for
+    every _ASK bytes of a scene's checkpoints (asking takes 70 us and up to
+    1 ms, a sub-step and its reverse of 110 000 particles 11 ms)."""
+    scene._checkpoint_bytes += nbytes
+    if scene._checkpoint_bytes < _ASK:
+        return True
+    free, total = torch.cuda.mem_get_info(device)
+    if free - nbytes < total // 2:  # blocks that the allocator holds unused are room too
+        free += torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
+    if free - nbytes < total // 2:
+        scene._checkpoint_bytes = _ASK  # the next one asks again
+        return False
+    scene._checkpoint_bytes = nbytes
+    return True
+
+
 def _on_scene(scene, x, v, C):
     """Whether a sub-step can take these tensors where they are: on the scene's
     device, 3, 3 and 9 finite values for every particle that the scene holds
-    and that has a mass, volume and radius from the last upload (anything else
-    goes through the host arrays and their checks)."""
+    and that has a mass, volume and radius from the last upload, and room for
+    the checkpoint (anything else goes through the host arrays and their
+    checks)."""
     n = scene.num_particles
     dev = int(scene.L.wcg_device(scene.h))
     attrs = scene._attrs
@@ -51,6 +76,8 @@ def _on_scene(scene, x, v, C):
     if not all(t.is_cuda and t.device.index == dev and t.shape[:1] == (n,) and
                t.numel() == n * w and t.dtype.is_floating_point
                for t, w in ((x, 3), (v, 3), (C, 9))):
+        return False
+    if not _room(scene, x.device, 15 * 8 * n):
         return False
     return bool(torch.stack([torch.isfinite(t).all() for t in (x, v, C)]).all())
 

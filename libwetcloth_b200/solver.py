@@ -73,6 +73,7 @@ class FluidScene:
         self.precision = prm.precision
         self._attrs = None      # mass, volume and radius as last uploaded from the host
         self._attrs_dev = None  # their device copies, made by autograd when it needs them
+        self._checkpoint_bytes = float("inf")  # of autograd since its last look at the memory
         if scene is not None:
             self.upload(scene.x, scene.v, scene.C, scene.mass, scene.vol, scene.radius)
             if getattr(scene, "elasto", None) is not None:

@@ -133,3 +133,28 @@ def test_widths_and_masses_are_checked(wcg):
     with pytest.raises(ValueError):
         autograd.substep(g, *dev[:3], 1e-3)
     g.close()
+
+
+def test_checkpoint_leaves_half_of_the_memory(wcg, monkeypatch):
+    """A node's checkpoint is on the device while half of its memory stays free,
+    else on the host; results and gradients are the same bits."""
+    from libwetcloth_b200 import autograd
+    sc = scenes.dam_break(16, 8, 0)
+    n = sc.x.shape[0]
+    total = torch.cuda.mem_get_info()[1]
+    res = []
+    for room in (True, False):
+        free = total // 2 + 120 * n - (0 if room else 1)
+        monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d=None: (free, total))
+        monkeypatch.setattr(torch.cuda, "memory_reserved", lambda d=None: 0)
+        monkeypatch.setattr(torch.cuda, "memory_allocated", lambda d=None: 0)
+        g = FluidScene(sc)
+        t = [torch.tensor(a, device="cuda", requires_grad=True)
+             for a in (sc.x, sc.v, np.zeros((n, 9)))]
+        out = autograd.substep(g, *t, 1e-3, correction_call=0)
+        assert isinstance(out[0].grad_fn.state[0], torch.Tensor) == room
+        grads = torch.autograd.grad(out[1].square().sum(), t)
+        assert all(o.is_cuda for o in (*out, *grads))
+        res.append([o.detach().cpu().numpy() for o in (*out, *grads)])
+        g.close()
+    assert all(np.array_equal(p, q) for p, q in zip(*res))

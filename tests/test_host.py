@@ -107,7 +107,7 @@ def test_replica_timing_reduction_gloo():
     assert sorted(res) == [(0, 20.0), (1, 20.0)]
 
 
-def test_device_substep_takes_whole_particles_only():
+def test_device_substep_takes_whole_particles_only(monkeypatch):
     """autograd's device route hands raw pointers to the library: only tensors
     of 3, 3 and 9 values for each particle of the scene, which has as many
     masses, may take it."""
@@ -128,7 +128,10 @@ def test_device_substep_takes_whole_particles_only():
 
     def scene(n, attrs):
         L = types.SimpleNamespace(wcg_device=lambda h: 0)
-        return types.SimpleNamespace(num_particles=n, L=L, h=None, _attrs=attrs)
+        return types.SimpleNamespace(num_particles=n, L=L, h=None, _attrs=attrs,
+                                     _checkpoint_bytes=0)
+
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: (1 << 30, 1 << 30))
 
     def ask(n, attrs, *shapes):
         return autograd._on_scene(scene(n, attrs), *[Tensor(*s) for s in shapes])
@@ -144,6 +147,38 @@ def test_device_substep_takes_whole_particles_only():
     # the state of a checkpoint against masses uploaded since
     with pytest.raises(ValueError):
         autograd._load(scene(6, [np.ones(5)] * 3), Tensor(6, 3), None, None)
+
+
+def test_checkpoint_room(monkeypatch):
+    """A checkpoint stays on the device while half of its memory is left, blocks
+    that the allocator holds unused counted in."""
+    import types
+
+    import torch
+
+    from libwetcloth_b200 import autograd
+    state = {"free": 0, "reserved": 0, "used": 0}
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: (state["free"], 1000))
+    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda d: state["reserved"])
+    monkeypatch.setattr(torch.cuda, "memory_allocated", lambda d: state["used"])
+    for free, reserved, used, nbytes, fits in (
+            (1000, 0, 0, 500, True), (1000, 0, 0, 501, False), (600, 0, 0, 100, True),
+            (600, 0, 0, 101, False), (400, 300, 100, 100, True), (400, 300, 100, 101, False),
+            (400, 300, 300, 0, False)):
+        state.update(free=free, reserved=reserved, used=used)
+        scene = types.SimpleNamespace(_checkpoint_bytes=float("inf"))
+        assert autograd._room(scene, "cuda:0", nbytes) == fits
+    # asked once for every _ASK bytes, and each time once the answer was no
+    scene = types.SimpleNamespace(_checkpoint_bytes=float("inf"))
+    monkeypatch.setattr(autograd, "_ASK", 100)
+    state.update(free=1000, reserved=0, used=0)
+    assert autograd._room(scene, "cuda:0", 40)
+    state.update(free=0)
+    assert autograd._room(scene, "cuda:0", 40)      # 80 since the last look
+    assert not autograd._room(scene, "cuda:0", 40)  # 120
+    assert not autograd._room(scene, "cuda:0", 1)
+    state.update(free=1000)
+    assert autograd._room(scene, "cuda:0", 1)
 
 
 def test_inner_waits_outlast_the_wait_limit(tmp_path):
