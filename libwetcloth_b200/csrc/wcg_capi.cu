@@ -784,9 +784,14 @@ int wcg_substep_vjp(wcg_ctx* ctx, double dt, const double* vbar3, const double* 
            "substep_vjp");
   int st = device_status(ctx->c, "substep_vjp");
   if (st) return st;
-  if (ctx->c.adjoint_fixed_x && n > 0 &&
-      cudaMemcpy(xbar0, xbar3, (size_t)3 * n * sizeof(double), cudaMemcpyDefault) != cudaSuccess)
-    return fail(WCG_ERR_CUDA, "substep_vjp: copy of the position cotangent");
+  if (ctx->c.adjoint_fixed_x && n > 0) {
+    // on the context's stream and waited for: cudaMemcpy between two device arrays
+    // returns before the copy is done
+    WCG_CALL(ctx, cudaMemcpyAsync(xbar0, xbar3, (size_t)3 * n * sizeof(double), cudaMemcpyDefault,
+                                  ctx->c.stream),
+             "substep_vjp");
+    WCG_CALL(ctx, cudaStreamSynchronize(ctx->c.stream), "substep_vjp");
+  }
   ctx->c.have_grid = true;
   if (!ctx->c.stats.converged)
     return fail(WCG_ERR_NOT_CONVERGED, "adjoint pressure solve did not converge");

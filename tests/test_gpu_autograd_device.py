@@ -43,6 +43,18 @@ def test_device_tensors_equal_host_tensors(precision, mu, fixed_x, wcg):
         assert p.shape == q.shape and p.dtype == q.dtype and np.array_equal(p, q)
 
 
+@pytest.mark.parametrize("fixed_x", [False, True])
+def test_on_a_side_stream(fixed_x, wcg):
+    """The same under a stream of the caller's, which nothing orders with the
+    default stream: what the call returns is finished when it returns."""
+    sc = scenes.dam_break(32, 8, 0)
+    a = _run(sc, "cuda", _capi.WCG_FP64, False, fixed_x)
+    for _ in range(3):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            b = _run(sc, "cuda", _capi.WCG_FP64, False, fixed_x)
+        assert all(np.array_equal(p, q) for p, q in zip(a, b))
+
+
 def test_device_tensors_of_other_kinds(wcg):
     """float32 leaves convert as on the host; non-finite input is refused with
     the host path's error."""
