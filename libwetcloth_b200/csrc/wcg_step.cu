@@ -2554,11 +2554,16 @@ static cudaError_t substep_vjp_t(Context& c, double dt, const double* vbar, cons
   }
   WCG_TRY(project_fine(c, dt));
   WCG_TRY(apply_pressure_and_extrapolate(c, dt));
-  if (np == 0 || c.n_active == 0) {
-    std::fill(vbar0, vbar0 + 3 * np, 0.0);
-    std::fill(Cbar0, Cbar0 + 9 * np, 0.0);
-    if (xbar0) std::copy(xbar, xbar + 3 * np, xbar0);
-    return cudaSuccess;
+  if (np == 0) return cudaSuccess;
+  if (c.n_active == 0) {  // (the caller's arrays may be device memory)
+    WCG_TRY(c.adjstage.ensure((size_t)9 * np * sizeof(double)));
+    const double* zero = c.adjstage.as<double>();
+    WCG_TRY(cudaMemsetAsync(c.adjstage.p, 0, (size_t)9 * np * sizeof(double), c.stream));
+    WCG_TRY(cudaMemcpyAsync(vbar0, zero, 3 * np * sizeof(double), cudaMemcpyDefault, c.stream));
+    WCG_TRY(cudaMemcpyAsync(Cbar0, zero, 9 * np * sizeof(double), cudaMemcpyDefault, c.stream));
+    if (xbar0)
+      WCG_TRY(cudaMemcpyAsync(xbar0, xbar, 3 * np * sizeof(double), cudaMemcpyDefault, c.stream));
+    return cudaStreamSynchronize(c.stream);
   }
   WCG_TRY(c.adj.ensure((size_t)kNumAdjFields * c.gcap * rb));
   WCG_TRY(c.adjmask.ensure((size_t)3 * c.gcap));
