@@ -298,6 +298,9 @@ int wcg_create(const wcg_params* params, wcg_ctx** out) {
   if (const char* v = getenv("WCG_PCG_LAYOUT")) ctx->c.pcg_layout = !strcmp(v, "tiles") ? 1 : 0;
   // transfer formulation: bucket tiles (default) or the global gathers
   if (const char* v = getenv("WCG_TRANSFERS")) ctx->c.xfer_mode = !strcmp(v, "gather") ? 1 : 0;
+  // groups per cluster of the MIC(0) sweeps, 1 or 4, whatever the box (for the
+  // tests; both compute identical results)
+  if (const char* v = getenv("WCG_SWEEP_CL")) ctx->c.pl_cl_given = !strcmp(v, "4") ? 4 : 1;
   // cluster extents of the launch schedule (wcg_schedule): held for
   // wcg_get_schedule, without effect on the sweeps
   ctx->c.sweep_cluster = 0;

@@ -264,6 +264,7 @@ struct Context {
   DevBuf pl_edge;                // tagged edge words
   DevBuf pl_order;               // clusters of the sweeps in wave order (int32)
   int pl_cl = 4;                 // groups per cluster in this solve's sweeps
+  int pl_cl_given = 0;           // 1 or 4: that many in every solve (0: by the box)
   // cluster extents of the launch schedule, kept for wcg_get_schedule (the
   // sweeps choose their clusters whatever they say)
   int sweep_cluster = 1;

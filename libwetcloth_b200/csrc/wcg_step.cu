@@ -1328,7 +1328,9 @@ static cudaError_t pl_setup(Context& c, const int* lo, const int* hi) {
   // the shape made no difference (256^3 FP32: 669 / 661 / 666 us an iteration in
   // clusters of 2, 4 and 8).
   const int ngroup = pl_groups<R>(G);
-  c.pl_cl = !c.shared_solve && ngroup > 1 && pl_units<R>(G) <= 74 ? 4 : 1;
+  c.pl_cl = ngroup > 1 && pl_units<R>(G) <= 74 ? 4 : 1;
+  if (c.pl_cl_given) c.pl_cl = c.pl_cl_given;
+  if (c.shared_solve) c.pl_cl = 1;  // its launches over several solves run without
   const int ncl = (ngroup + c.pl_cl - 1) / c.pl_cl;
   if (!same_shape || c.pl_order_h.size() != (size_t)G.nPA * ncl) {
     // clusters in wave order: column + cluster of the column

@@ -27,14 +27,15 @@ def _scene(kind):
         return scenes.dam_break(48, 2, 4, block_hi=(0.5, 0.3, 0.95))
     if kind == "curl48":
         return scenes.half_box(48, 2, 5, amplitude=0.5, sigma_cells=2.0)
-    if kind == "curl96":  # 6 patches along c: several cluster columns
-        return scenes.half_box(96, 2, 6, amplitude=0.5, sigma_cells=3.0)
     raise ValueError(kind)
 
 
-def _solve(sc, layout, precision, cluster=1):
-    cc, ca = (str(cluster).split("x") + ["1"])[:2] if "x" in str(cluster) else (str(cluster), "1")
-    env = {"WCG_PCG_LAYOUT": layout, "WCG_SWEEP_CLUSTER": cc, "WCG_SWEEP_CLUSTER_A": ca}
+def _solve(sc, layout, precision, groups=None):
+    """The pressure and the solver's figures; groups: the groups per cluster of
+    the sweeps (None: chosen by the box)."""
+    env = {"WCG_PCG_LAYOUT": layout}
+    if groups is not None:
+        env["WCG_SWEEP_CL"] = str(groups)
     old = {k: os.environ.get(k) for k in env}
     os.environ.update(env)
     try:
@@ -51,6 +52,13 @@ def _solve(sc, layout, precision, cluster=1):
     g.project_fine(DT)
     p = g.field("pressure")
     st = g.stats()
+    # extents of the DOF box (fields are bucket-major, 4 x 4 x 4 nodes a bucket)
+    dims, _, _ = g.grid_info()
+    dof = np.flatnonzero(g.ifield("dof_index") >= 0)
+    b, n = dof // 64, dof % 64
+    xyz = [4 * (b % dims[0]) + n % 4, 4 * (b // dims[0] % dims[1]) + n // 4 % 4,
+           4 * (b // (dims[0] * dims[1])) + n // 16]
+    st["box"] = [int(k.max() - k.min()) + 1 for k in xyz]
     g.close()
     return p, st
 
@@ -112,23 +120,45 @@ def test_pencil_deterministic_256_patches(precision, wcg):
         assert np.array_equal(p, res[0][0])
 
 
-@pytest.mark.parametrize("cluster", [2, 4, 8, 16, "1x4", "2x4", "4x4", "1x8", "2x8"])
-@pytest.mark.parametrize("kind,precision", [("curl48", _capi.WCG_FP64),
-                                            ("slab64_x", _capi.WCG_FP64),
-                                            ("curl96", _capi.WCG_FP64),
-                                            ("curl48", _capi.WCG_FP32_REFINE)])
-def test_pencil_cluster_sweeps_bit_identical(kind, precision, cluster, wcg):
-    """Clusters only change how edge values travel (shared memory of the
-    neighbouring CTA instead of a global round trip): c-faces with clusters
-    along c ("8"), both faces with 2-D clusters ("CCxCA": CC c-patches by CA
-    a-patches).  The arithmetic is the same, so pressures and iteration
-    counts are bit-identical, also when the patch counts are not multiples
-    of the cluster extents."""
-    sc = _scene(kind)
+def _groups(box, precision):
+    """(groups in a column of patches, groups in all) of a DOF box: 16 x 16 lines
+    a patch across its longest axis, one group a patch in FP32 and two in FP64."""
+    s = box.index(max(box))
+    a, c = [k for k in range(3) if k != s]
+    col = -(-box[c] // 16) * (1 if precision == _capi.WCG_FP32_REFINE else 2)
+    return col, col * -(-box[a] // 16)
+
+
+# blocks of liquid (cells) whose boxes have 1, 2, 3, 5 and more groups in a column
+# (multiples of 4 and not), and 74 groups at most or more in all
+@pytest.mark.parametrize("cells,precision,column,many", [
+    ((20, 40, 2), _capi.WCG_FP32_REFINE, 1, False),
+    ((20, 40, 10), _capi.WCG_FP32_REFINE, 2, False),
+    ((24, 60, 24), _capi.WCG_FP32_REFINE, 3, False),
+    ((30, 70, 58), _capi.WCG_FP32_REFINE, 5, False),
+    ((100, 130, 118), _capi.WCG_FP32_REFINE, 9, False),
+    ((130, 140, 118), _capi.WCG_FP32_REFINE, 9, True),
+    ((20, 40, 2), _capi.WCG_FP64, 2, False),
+    ((20, 60, 24), _capi.WCG_FP64, 6, False),
+    ((30, 70, 58), _capi.WCG_FP64, 10, False),
+    ((78, 100, 74), _capi.WCG_FP64, 12, False),
+    ((90, 100, 74), _capi.WCG_FP64, 12, True),
+])
+def test_sweeps_in_clusters_and_without_bit_identical(cells, precision, column, many, wcg):
+    """Clusters only change how the c-face values of a group travel (shared memory
+    of the next CTA in place of a global round trip): the sweeps in clusters of 4
+    groups, those without and the form that the box's size chooses give the same
+    pressures and iteration counts bit for bit, also where the groups of a column
+    are not a multiple of 4."""
+    n = 160
+    sc = scenes.dam_break(n, 2, 9, block_hi=tuple(c / n for c in cells))
+    sc.v = np.random.default_rng(3).normal(0.0, 0.2, sc.x.shape)
     a, sa = _solve(sc, "pencil", precision, 1)
-    b, sb = _solve(sc, "pencil", precision, cluster)
-    assert sb["converged"] == 1
-    assert sa["pcg_iters"] == sb["pcg_iters"] and sa["refinements"] == sb["refinements"]
+    col, groups = _groups(sa["box"], precision)
+    assert col == column and (groups > 74) == many, (sa["box"], col, groups)
+    assert sa["converged"] == 1
     m = ~np.isnan(a)
-    assert np.array_equal(m, ~np.isnan(b))
-    assert np.array_equal(a[m], b[m])
+    for g in (4, None):
+        b, sb = _solve(sc, "pencil", precision, g)
+        assert sa["pcg_iters"] == sb["pcg_iters"] and sa["refinements"] == sb["refinements"]
+        assert np.array_equal(m, ~np.isnan(b)) and np.array_equal(a[m], b[m])
