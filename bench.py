@@ -553,7 +553,7 @@ def run_batch(args, steps=3):
         g.close()
     hist = {}
     for k in chosen:
-        key = "x".join(str(v) for v in cands[k])
+        key = str(cands[k][2])
         hist[key] = hist.get(key, 0) + 1
 
     # sequential: one scene after another, each its own steps
@@ -603,7 +603,7 @@ def run_batch(args, steps=3):
             "batched_tuned_particle_steps_per_s": round(total_p * steps / sched_s, 1),
             "speedup_tuned": round(seq_s / sched_s, 3),
             "schedules_chosen": hist,
-            "schedule_key": "sweep_cluster x sweep_cluster_a x pcg_batch",
+            "schedule_key": "PCG iterations per host check",
             "batched_shared_solve_particle_steps_per_s": round(total_p * steps / shared_s, 1),
             "speedup_shared_solve": round(seq_s / shared_s, 3),
             "shared_solve_launches_per_pass": shared_launches,

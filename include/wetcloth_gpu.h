@@ -469,9 +469,9 @@ int wcg_batch_autotune(wcg_batch* b, const double* dt, const int* candidates, in
  *   sweep_cluster    0 (the default), 1, 2, 3, 4, 8, 9 or 16, and
  *   sweep_cluster_a  1, 4 (with sweep_cluster 1..4) or 8 (with sweep_cluster
  *                    1..2): the extents of the thread-block clusters that
- *                    the MIC(0) sweeps once ran in.  Accepted and returned;
- *                    the sweeps run one CTA per patch, which is faster than
- *                    every cluster shape was, whatever they say;
+ *                    the MIC(0) sweeps once ran in.  Accepted and returned,
+ *                    without effect: the sweeps choose clusters of 4 CTAs or
+ *                    none by the size of the box;
  *   pcg_batch        PCG iterations launched per convergence check on the
  *                    host (1..64; default 8). */
 typedef struct wcg_schedule {

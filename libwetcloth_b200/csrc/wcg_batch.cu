@@ -6,8 +6,9 @@
 // scenes leave most SMs idle and their launches are short, so running several
 // at once fills the machine.  The thread count is chosen by
 // wcg_batch_autotune, which times one batch step per candidate, and each
-// scene's launch schedule (the PCG iterations per host check) by wcg_batch_autotune_schedules, from the device time of each
-// scene's step under each candidate.  With the shared solve on
+// scene's launch schedule (the PCG iterations per host check) by
+// wcg_batch_autotune_schedules, from the device time of each scene's step under
+// each candidate.  With the shared solve on
 // (wcg_batch_set_shared_solve), the PCG iterations of all scenes waiting in
 // their pressure solve run as one launch per kernel from a coordinator
 // thread (wcg_step.cu), in place of one launch per scene.  Results are those

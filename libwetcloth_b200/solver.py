@@ -281,8 +281,8 @@ class FluidScene:
     def schedule(self):
         """The pressure solve's launch schedule (sweep_cluster,
         sweep_cluster_a, pcg_batch); performance only, results unchanged.
-        The cluster shape is kept for the caller but has no effect: the sweeps
-        choose their own."""
+        The cluster extents are kept for the caller but have no effect: the
+        sweeps choose their own."""
         s = _capi.WcgSchedule()
         check(self.L.wcg_get_schedule(self.h, ctypes.byref(s)))
         return (s.sweep_cluster, s.sweep_cluster_a, s.pcg_batch)
@@ -388,9 +388,9 @@ class FluidScene:
 
 
 
-# launch schedules the batch autotuner tries by default; what differs in time
-# is 4 or 8 PCG iterations per host check (the cluster shapes have no effect)
-DEFAULT_SCHEDULES = ((0, 1, 8), (1, 1, 8), (2, 1, 8), (4, 1, 8), (1, 1, 4), (2, 1, 4))
+# launch schedules the batch autotuner tries by default: 8 or 4 PCG iterations per
+# host check (the cluster extents have no effect)
+DEFAULT_SCHEDULES = ((0, 1, 8), (0, 1, 4))
 
 
 class FluidBatch:
