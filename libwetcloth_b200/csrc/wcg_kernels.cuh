@@ -434,11 +434,14 @@ __device__ inline int halo_centre(int x, int y, int z) { return (z * 6 + y) * 6 
 // every node receiving its contributions in sorted-particle order: deterministic.
 // Requires stencil offsets in {0, 1} (checked on the host).
 //
-// Bound by instruction issue, and in small scenes by the chain of additions of
-// the fullest bucket.  One warp for all four node kinds, its particles' values
-// handed round by shuffles, took 212 warp instructions a particle and 1100
-// cycles each in turn: 4.96 ms at 256^3 (16.8M particles, FP32), 1.28 ms for 2.1M
-// in FP64, 309 us for a 16^3 dam break (512 particles a bucket).
+// Bound by the wavefronts of shared memory (99 % of the pipe at 192^3 in FP32, the
+// issue slots at 58 %), and in small scenes by the chain of additions of the fullest
+// bucket.  One warp for all four node kinds, its particles' values handed round by
+// shuffles, took 212 warp instructions a particle and 1100 cycles each in turn.
+// That form and this, ms with the merge: a 16^3 dam break (512 particles a bucket)
+// 0.32 and 0.10, at 64^3 0.40 and 0.28, the half box at 128^3 in FP64 (2.1M
+// particles) 1.58 and 1.48, and at 256^3 in FP32 (16.8M) 6.5 and 6.7: the one size
+// where it costs, 0.2 of a step's 28 or 118 (the launch alone 4.96 and 5.19).
 template <typename R>
 constexpr int kP2GBatch = sizeof(R) == 4 ? 32 : 16;  // particles staged at a time
 constexpr int kP2GRec = 52;  // a record: 3 axes x 3 nodes {w0, -d0, w5, -d5} (d = x_p - x_n),

@@ -152,8 +152,9 @@ __global__ void __launch_bounds__(kMgThreads)
 // One colour of a red-black Gauss-Seidel sweep: parity 1 = cells with
 // (i + j + k) odd (RBGS_with_pattern's first pass), 0 = even.  A thread takes the
 // cell of its colour in a pair along x, so every lane has one, and asks for the
-// mask of its next cell before it waits for the values of this one.  Memory
-// bound, every sector of 7 values and the mask once per colour.  A thread per
+// mask of its next cell before it waits for the values of this one.  Bound by
+// loads, every sector of 7 values and the mask once per colour (192^3 in FP32: DRAM
+// at 47 %, of 30 cycles an instruction of a warp 22 wait for one).  A thread per
 // cell, with half the lanes idle: V-cycles of the half box at 256^3 in FP32 12.4
 // ms a step (79 us a colour of the finest level), this 10.5; at 128^3 in FP64 6.84
 // and 6.55.  (Both colours in one pass, tiles of 30 x 14 columns walking planes
@@ -210,14 +211,20 @@ __global__ void __launch_bounds__(kMgCoarseThreads) k_mg_coarsest(MgLevel<R> L, 
 }
 
 // The same with x in shared memory and the cells of each colour listed there,
-// for levels whose box fits (mg_coarse_smem).  A thread holds the first
-// kMgHeld cells of each colour with their couplings in registers, so a colour
-// is six reads of x, a division and a barrier; further cells have them in
-// shared memory as long as it lasts, the rest reads them from global memory.
-// Bound by the latency of those 2 x iters colours.  With everything in global
-// memory a V-cycle spent 1550 us here (19 x 12 x 19 cells, FP64; 1225 us in FP32
-// at 18 x 10 x 18), most of it index arithmetic and cache latency; with the
-// further cells alone there 570, now 490.
+// for levels whose box fits (mg_coarse_smem): 18 700 cells in FP64, 28 100 in FP32.
+// The box, not the unknowns in it, decides, and level 0 spans the whole grid with
+// its padding of 24 cells an axis: half boxes from 16 cells a side on and dam breaks
+// from 24 on fit, but not smaller ones, whose coarsest level is the grid itself
+// (41 000 cells and more), nor most sheet scenes, a few unknowns in a wide box
+// (51 000 to 125 000 cells up to 28 a side, 54 000 to 131 000 from 64 to 120).  Those run the kernel above.
+// A thread holds the first kMgHeld cells of each colour with their couplings in
+// registers, so a colour is six reads of x, a division and a barrier; further cells
+// have them in shared memory as long as it lasts, the rest reads them from global
+// memory.  Bound by the latency of those 2 x iters colours (of 26 cycles an
+// instruction of a warp 7 wait for shared memory, 7 for global or spilled values, 6
+// at the barrier).  With everything in global memory a V-cycle spent 1550 us here
+// (19 x 12 x 19 cells, FP64; 1225 us in FP32 at 18 x 10 x 18), most of it index
+// arithmetic and cache latency; with the further cells alone there 570, now 490.
 template <typename R>
 constexpr int kMgHeld = sizeof(R) == 4 ? 2 : 1;
 template <typename R>

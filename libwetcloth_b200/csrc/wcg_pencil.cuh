@@ -17,15 +17,18 @@
 //   (s, a-1, c): step v-1 of lane - 1 (step v+15 of lane + 15 of the patch below)
 //   (s, a, c-1): step v-1 of lane - 16, or step v+1 of lane + 16 of the strip
 //                before (of the last strip of the patch before along c)
-// so a CTA takes a patch, one warp per strip, and every strip reads and writes
-// one contiguous run of memory.  The factor lies step by step too, four rows of
-// 64 per step: 1/sqrt(d'), S_s, S_a, S_c.
-// Values crossing a patch edge go through a global buffer of tagged 64-bit
-// words, (epoch << 32 | 32 data bits), one word per 32 bits of payload: the
-// consumer re-reads its word until the tag equals the launch's epoch, so no
-// fence or flag is needed and a patch waits only for the rows it reads.
-// Patches are handed out by an atomic ticket in wave order (PAi + PCi), so a
-// patch's upstream patches always started before it.
+// so a warp takes a strip, a CTA a group of consecutive strips along c (a patch in
+// FP32, half of one in FP64), and every strip reads and writes one contiguous run
+// of memory.  The factor lies step by step too, four rows of 64 per step:
+// 1/sqrt(d'), S_s, S_a, S_c.
+// Values crossing a patch edge along a, or along c the edge of a group that is not
+// in the same cluster, go through a global buffer of tagged 64-bit words,
+// (epoch << 32 | 32 data bits), one word per 32 bits of payload: the consumer
+// re-reads its word until the tag equals the launch's epoch, so no fence or flag is
+// needed and a strip waits only for the words of its next step.
+// Groups, or clusters of them, are handed out by an atomic ticket in wave order
+// (column along a + cluster along c), so whatever is upstream of one always
+// started before it.
 //
 // The arithmetic is that of the tile sweeps in wcg_pcg.cuh (restating
 // robertbridson's factor_modified_incomplete_cholesky0 / solve_lower /
@@ -214,8 +217,11 @@ struct PencilSweepArgs {
 //
 // Bound: the chain of Ls / 2 + NA + NC steps that the last cell waits for, then
 // the bytes of a step (forward 8, backward 7 values per cell).  A step takes
-// about 500 cycles of a warp in FP32 and 900 in FP64, so it is kept to two cells
-// per lane: with single cells a row took 320-400 and 450-500 and a hop between
+// about 500 cycles of a warp in FP32 and 900 in FP64, some 85 and 155 instructions
+// of one warp at 6.1 and 5.7 cycles each: the fixed latency of dependent
+// instructions takes 1.9 of those, branches 1.2 and 0.9, loads of either memory 0.9
+// and 1.3 (counters at 192^3 and 128^3; DRAM at 12 and 10 %).  So a step is kept to
+// two cells per lane: with single cells a row took 320-400 and 450-500 and a hop between
 // strips 1500.  Per launch (the events around it included), one CTA barrier per
 // row and every face lane polling L2 / one-cell strips / this: 256^3 half box in
 // FP32 426 / 270 / 213 us; FP64 half box at 128^3 287 / 161 / 138, dam break at
@@ -232,8 +238,8 @@ __host__ __device__ constexpr int sweep_inc() {
 }
 constexpr int kRecv = 4;   // steps a receiver lane polls at once
 
-// chunks of a strip in flight or in use (one CTA per SM: 96 KB of FP32 or 144 KB
-// of FP64 cells, enough for the latency of HBM at its full rate)
+// chunks of a strip in flight or in use (96 KB a CTA in FP32, one CTA per SM; 72 KB
+// in FP64, two)
 template <typename R>
 struct SweepSlots {
   static constexpr int N = sizeof(R) == 4 ? 4 : 3;
