@@ -40,6 +40,7 @@ def _host(t):
     return t.detach().cpu().numpy().astype(np.float64)
 
 
+_DTYPES = (torch.float64, torch.float32, torch.float16)  # those that numpy has too
 _ASK = 256 << 20  # bytes of checkpoints that a scene makes between two looks at the memory
 
 
@@ -74,7 +75,7 @@ def _on_scene(scene, x, v, C):
     if n <= 0 or attrs is None or any(a is None or a.size != n for a in attrs):
         return False
     if not all(t.is_cuda and t.device.index == dev and t.shape[:1] == (n,) and
-               t.numel() == n * w and t.dtype.is_floating_point
+               t.numel() == n * w and t.dtype in _DTYPES
                for t, w in ((x, 3), (v, 3), (C, 9))):
         return False
     if not _room(scene, x.device, 15 * 8 * n):
@@ -160,7 +161,7 @@ class _Substep(torch.autograd.Function):
         if isinstance(ctx.state[0], torch.Tensor):
             where = ctx.state[0].device
             cot = [torch.zeros((n, w), dtype=torch.float64, device=where) if g is None else
-                   g.detach().to(where, torch.float64).reshape(n, w).contiguous()
+                   g.detach().resolve_neg().to(where, torch.float64).reshape(n, w).contiguous()
                    for g, w in ((gv1, 3), (gC1, 9), (gx1, 3))]
             bar = [torch.empty_like(t) for t in cot]
             mub = ctypes.c_double(0.0)

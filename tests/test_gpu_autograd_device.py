@@ -170,3 +170,23 @@ def test_checkpoint_leaves_half_of_the_memory(wcg, monkeypatch):
         res.append([o.detach().cpu().numpy() for o in (*out, *grads)])
         g.close()
     assert all(np.array_equal(p, q) for p, q in zip(*res))
+
+
+def test_cotangents_with_the_negative_bit(wcg):
+    """A cotangent that torch holds as a lazily negated view arrives negated, and
+    bfloat16 tensors, which have no host array, stay refused."""
+    from libwetcloth_b200 import autograd
+    sc = scenes.dam_break(16, 8, 0)
+    n = sc.x.shape[0]
+    g = FluidScene(sc)
+    t = [torch.tensor(a, device="cuda", requires_grad=True)
+         for a in (sc.x, sc.v, np.zeros((n, 9)))]
+    c = torch.randn((n, 3), device="cuda", dtype=torch.float64)
+    res = []
+    for cot in (-c, torch._neg_view(c)):
+        out = autograd.substep(g, *t, 1e-3, correction_call=0)
+        res.append([q.cpu().numpy() for q in torch.autograd.grad(out[1], t, cot)])
+    assert all(np.array_equal(p, q) for p, q in zip(*res))
+    with pytest.raises(TypeError):
+        autograd.substep(g, t[0].detach().bfloat16(), t[1], t[2], 1e-3)
+    g.close()

@@ -140,6 +140,10 @@ def test_device_substep_takes_whole_particles_only(monkeypatch):
     good = ((6, 3), (6, 3), (6, 9))
     for k, bad in ((0, (6, 6)), (1, (6, 1)), (2, (6, 3)), (0, (18,)), (0, (7, 3)), (2, (6,))):
         assert not ask(6, ones, *good[:k], bad, *good[k + 1:])
+    monkeypatch.setattr(Tensor, "dtype", torch.bfloat16)  # which the host arrays refuse
+    assert not ask(6, ones, *good)
+    monkeypatch.undo()
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: (1 << 30, 1 << 30))
     assert not ask(6, None, *good)                      # masses never uploaded
     assert not ask(6, [np.ones(5)] * 3, *good)          # masses of another set
     assert not ask(6, [np.ones(6), None, np.ones(6)], *good)
