@@ -92,6 +92,13 @@ class FluidScene:
 
     # ---- particles ----
     def upload(self, x, v, C, mass, vol, radius):
+        mass, vol, radius = self._upload(x, v, C, mass, vol, radius)
+        # copies: set_state takes them as they were uploaded, whatever the caller
+        # does to its arrays
+        self._attrs = tuple(None if a is None else a.copy() for a in (mass, vol, radius))
+        self._attrs_dev = None
+
+    def _upload(self, x, v, C, mass, vol, radius):
         arr = lambda a: None if a is None else np.ascontiguousarray(a, dtype=np.float64).reshape(-1)
         x, v, C, mass, vol, radius = map(arr, (x, v, C, mass, vol, radius))
         n = mass.shape[0]
@@ -99,17 +106,16 @@ class FluidScene:
                            ("radius", radius, 1)):
             if a is not None and a.size < n * k:
                 raise ValueError(f"{name}: {a.size} values for {n} particles")
-        self._attrs = (mass, vol, radius)
-        self._attrs_dev = None
         check(self.L.wcg_upload_liquid(self.h, n, _dp(x), _dp(v), _dp(C), _dp(mass),
                                        _dp(vol), _dp(radius)))
+        return mass, vol, radius
 
     def set_state(self, x, v, C):
         """Replace the liquid particles' positions, velocities and affine
         matrices (mass, volume and radius as last uploaded)."""
         if self._attrs is None:
             raise ValueError("set_state: no masses, volumes and radii uploaded from the host")
-        self.upload(x, v, C, *self._attrs)
+        self._upload(x, v, C, *self._attrs)
 
     def substep_vjp(self, dt, vbar, Cbar, xbar, with_viscosity=False):
         """Reverse mode of substep(dt) at the current (pre-step) state:

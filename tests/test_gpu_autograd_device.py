@@ -190,3 +190,23 @@ def test_cotangents_with_the_negative_bit(wcg):
     with pytest.raises(TypeError):
         autograd.substep(g, t[0].detach().bfloat16(), t[1], t[2], 1e-3)
     g.close()
+
+
+def test_masses_are_those_uploaded(wcg):
+    """The masses, volumes and radii are those of the upload on either route, also
+    after the caller has changed its arrays in place."""
+    from libwetcloth_b200 import autograd
+    res = []
+    for where in ("cpu", "cuda"):
+        sc = scenes.dam_break(16, 8, 0)
+        g = FluidScene(sc)
+        t = [torch.tensor(a, device=where)
+             for a in (sc.x, sc.v, np.zeros((sc.x.shape[0], 9)))]
+        a = autograd.substep(g, *t, 1e-3, correction_call=0)
+        sc.mass *= 2.0
+        sc.radius *= 0.5
+        b = autograd.substep(g, *t, 1e-3, correction_call=0)
+        res += [[o.cpu().numpy() for o in q] for q in (a, b)]
+        g.close()
+    for r in res[1:]:
+        assert all(np.array_equal(p, q) for p, q in zip(res[0], r))
